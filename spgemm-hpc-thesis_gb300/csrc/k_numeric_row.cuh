@@ -4,13 +4,12 @@
 //   1. enumerates the products in reference order (spg_enum.cuh): product t gets
 //      its column, sequence number t and value __dmul_rn(a, b) (one rounding, as
 //      `const double product = aValue * b` in spgemm_exchange.cpp:287);
-//   2. sorts the products by column with a stable LSD radix sort (8-bit digits
-//      over the bits of max(col) - min(col) only; ranks from ballot-matched
-//      lane groups and per-warp digit counters), so that equal columns stay in
-//      product order.
-//      When the column range and the sequence number fit in 32 bits together,
-//      the sort moves one packed word (column - min) << s | seq per product;
-//      otherwise it moves the column and a 16-bit sequence number side by side;
+//   2. sorts the products by column so that equal columns stay in product
+//      order.  When the column range and the sequence number fit in 32 bits
+//      together, the sort moves one packed word (column - min) << s | seq per
+//      product -- a warp row sorts these words in registers (warp_sort), a CTA
+//      row by the bucket sort below -- otherwise the column and a 16-bit
+//      sequence number side by side (a warp row by a stable LSD radix sort);
 //   3. sums each run of equal columns sequentially in product order with
 //      __dadd_rn, starting from its first product (the `emplace` then `+=` of
 //      spgemm_exchange.cpp:288-293), and keeps the sums that are != 0.0
@@ -32,6 +31,7 @@
 #include <type_traits>
 
 #include "spg_enum.cuh"
+#include "spg_warp_sort.cuh"
 
 namespace spg {
 namespace {
@@ -104,18 +104,16 @@ constexpr int rank_group(int items) {
         if (items % g == 0) return g;
     return 1;
 }
-// Which rows take the bucket sort: CTA rows, and warp rows of 8-16 products per
-// lane (32 coarse buckets, no extra fine bit, so that a warp's counters stay
-// small).  On the power-law product, with the bins on three streams, K4 took
-// 12.64 -> 12.10 ms, uniform 0.204 -> 0.199 ms; on one stream the 512-product
-// bin alone is slower (0.77 -> 0.94 ms: a warp row's passes need no barrier,
-// so the radix sort's extra instructions cost little while the bin runs
-// alone), but beside the CTA bins the fewer instructions win.  Warp rows of 6
-// products per lane measured the same either way; fewer keep the radix sort.
-constexpr int kWarpBucketMinItems = 8;
-constexpr int kWarpBucketMaxItems = 16;
+// Which rows take the bucket sort: CTA rows.  A warp row sorts its packed keys
+// in registers (spg_warp_sort.cuh).  Against the radix sort of rows of <= 192
+// products and the bucket sort of 193-512 (power-law product, one bin at a
+// time): <= 512 products 0.95 -> 0.49 ms, <= 384 0.79 -> 0.50, <= 256 0.35 ->
+// 0.23, <= 192 0.37 -> 0.25, <= 128 0.145 -> 0.094; 65,536 rows of 256: 0.190 ->
+// 0.147 ms.  Issue slots bound these kernels, and the network takes about half
+// the instructions of either sort (about 90 a key), none of them waiting on
+// shared memory.
 template <int W, int ITEMS>
-constexpr bool kBucketRows = W > 1 || (ITEMS >= kWarpBucketMinItems && ITEMS <= kWarpBucketMaxItems);
+constexpr bool kBucketRows = W > 1;
 // A fine bucket holding more products than this (a column repeated many times)
 // sends the row to the radix sort: ranking inside a bucket is quadratic.
 constexpr uint32_t kMaxFine = 64;
@@ -662,9 +660,22 @@ __device__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, dou
                            int nbits, int lane, int warp, int tid) {
     using Sm = RowSmem<W, ITEMS, SV>;
     constexpr int kSeqBits = Sm::kSeqBits;
-    // 2. sort by column: the bucket sort for CTA rows, the radix sort for warp
-    //    rows and where the bucket sort declines
-    if constexpr (!kBucketRows<W, ITEMS>) {
+    // 2. sort by column: warp rows in registers (the padding words above P sort
+    //    last: a real word is all ones only when P is the row's capacity), CTA
+    //    rows by the bucket sort, and by the radix sort where that declines
+    if constexpr (W == 1 && PACKED) {
+        uint32_t k[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const int pos = i * 32 + lane;
+            k[i] = pos < P ? ((sm.keys[pos] - cmin) << kSeqBits) | static_cast<uint32_t>(pos) : 0xffffffffu;
+        }
+        warp_sort<ITEMS>(k, lane);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) sm.keys[lane * ITEMS + i] = k[i];
+        __syncwarp();
+    } else if constexpr (W == 1) {
         radix_sort_row<W, ITEMS, SV, PACKED, true>(sm, P, cmin, nbits, lane, warp, tid);
     } else {
         if (nbits == 0 || !bucket_sort<W, ITEMS, SV, PACKED>(sm, P, cmin, nbits, lane, warp, tid))
@@ -849,10 +860,10 @@ __device__ uint32_t numeric_row(const Job& J, int row, RowSmem<W, ITEMS, SV>& sm
 constexpr int kWarpKernelThreads = 256;
 
 // Resident CTAs per SM the warp-row kernels are compiled for (caps registers
-// at 80 and 64 per thread).  Measured on power-law rows, one bin at a time:
-// the 12- and 16-item kernels 0.92 / 0.85 -> 0.79 / 0.80 ms against 2 CTAs
-// (128 registers), the 6- and 8-item ones 0.39 -> 0.35 ms against 3.
-constexpr int warp_kernel_min_blocks(int items) { return items >= 12 ? 3 : 4; }
+// at 128, 80 and 64 per thread).  Measured on power-law rows, one bin at a
+// time, against one CTA more: 8 items 0.256 -> 0.228 ms, 6 items 0.263 ->
+// 0.252, 12 and 16 items 0.49 -> 0.50 (but the concurrent phase 4% shorter).
+constexpr int warp_kernel_min_blocks(int items) { return items >= 12 ? 2 : (items >= 6 ? 3 : 4); }
 
 // The row kernels are persistent: a launch has at most a few waves of CTAs
 // that loop over the bin's rows.  A warp-row kernel takes its rows by a fixed
