@@ -430,23 +430,24 @@ constexpr int64_t slab_cap(int bin) { return bin == 17 ? 16 * 32 * 24 : 16 * 32 
 
 // Team shapes of the bins of 769-1536 and 2049-8192 products: warps, products
 // per thread, CTAs per SM, product values in shared memory (else in a per-CTA
-// global slab at the end of the scratch).  With the values in slabs, shared
-// memory stops limiting the resident CTAs, and more CTAs per SM hide each
-// other's barriers.  Measured on the power-law workload, one bin at a time:
-//   1024: 2x16, 8 CTAs/SM, shared values    1.48 ms -> 2x16, 12 CTAs/SM, slab 1.34 ms
-//         (9 CTAs/SM with shared values 1.56 ms, 10 with a slab 1.46 ms)
-//   1536: 8x6, 4 CTAs/SM, shared values     1.99 ms -> 4x12, 8 CTAs/SM, slab 1.90 ms
-//         (8x6 at 5 CTAs/SM with a slab 2.02 ms)
-//   3072: 12x8, 2 CTAs/SM, shared values    1.99 ms -> 8x12, 4 CTAs/SM, slab 1.67 ms
-//   4096: 8x16, 2 CTAs/SM, shared values    1.12 ms -> 8x16, 3 CTAs/SM, slab 1.00 ms
-//         (8x16 at 4 CTAs/SM with a slab 0.97 ms, 16x8 at 2 1.02 ms)
-//   6144: 16x12, 1 CTA/SM, shared values    1.55 ms -> 16x12, 2 CTAs/SM, slab 1.34 ms
-//         (8x24 at 3 CTAs/SM 1.42 ms, 12x16 at 2 1.33 ms against 1.28)
-//   8192: 16x16, 1 CTA/SM, shared values    0.73 ms (2 CTAs/SM with a slab: the same)
+// global slab at the end of the scratch).  The warps hide each other's latency
+// and barriers, so a shape pays where it keeps 32 warps per SM in 64 registers
+// each; shared memory limits the resident CTAs less with the values in slabs.
+// Measured (kernel times in ms: power-law product of 1,048,576 rows beside the
+// other bins / 16 uneven uniform products):
+//    768: 4x6, 8 CTAs 1.07 / 0.100, 2x12, 12 CTAs 1.01 / 0.099, 3x8, 10 CTAs 1.01 / 0.092
+//   1024: 2x16, 12 CTAs, slab 0.88 / 0.147, 4x8, 10 CTAs, slab 0.88 / 0.126, 4x8, 8 CTAs 0.80 / 0.119
+//   1536: 4x12, slab: 6 CTAs 1.30 / 0.392, 8 CTAs 1.15 / 0.353, 10 CTAs 1.35 / 0.401;
+//         6x8, 5 CTAs 1.34 / 0.375, 8x6, 4 CTAs, slab 1.72 / 0.538
+//   2048: 8x8: 3 CTAs 0.97 / 0.557, 4 CTAs 0.82 / 0.494, 5 CTAs 0.98 / 0.551; 4x16, 6 CTAs 0.94 / 0.522
+//   3072: 8x12, slab: 3 CTAs 1.15 / 0.221, 4 CTAs 1.06 / 0.209, 5 CTAs 1.23 / 0.228; 12x8, 2 CTAs 1.61 / 0.264
+//   4096: 8x16, 3 CTAs, slab 0.65, 4 CTAs 0.74; 16x8, 2 CTAs 0.81
+//   6144: 16x12, 2 CTAs, slab 0.74, 3 CTAs 0.76; 8x24, 3 CTAs 0.86
+//   8192: 16x16, 1 CTA 0.41, 2 CTAs with a slab 0.43
 // The slabs of these bins share one region: the bins run one after the other
 // on one stream.
-constexpr int kB10W = 2, kB10I = 16, kB10MinB = 12;
-constexpr bool kB10SV = false;
+constexpr int kB10W = 4, kB10I = 8, kB10MinB = 8;
+constexpr bool kB10SV = true;
 constexpr int kB11W = 4, kB11I = 12, kB11MinB = 8;
 constexpr bool kB11SV = false;
 constexpr int kB13W = 8, kB13I = 12, kB13MinB = 4;
@@ -561,7 +562,7 @@ void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t 
     double* slab = static_cast<double*>(d_scratch);
     unsigned long long* const tk = &d_stats->ticket[bin];  // the bin's row queue
     switch (bin) {
-        case 9: run_block<4, 6, 8>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk); break;     // <= 768
+        case 9: run_block<3, 8, 10>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk); break;     // <= 768
         case 10:  // <= 1024
             run_block<kB10W, kB10I, kB10MinB, kB10SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
                                                      tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(10, count, num_sms)));

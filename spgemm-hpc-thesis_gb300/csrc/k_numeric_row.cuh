@@ -5,11 +5,13 @@
 //      its column, sequence number t and value __dmul_rn(a, b) (one rounding, as
 //      `const double product = aValue * b` in spgemm_exchange.cpp:287);
 //   2. sorts the products by column so that equal columns stay in product
-//      order.  When the column range and the sequence number fit in 32 bits
-//      together, the sort moves one packed word (column - min) << s | seq per
-//      product -- a warp row sorts these words in registers (warp_sort), a CTA
-//      row by the bucket sort below -- otherwise the column and a 16-bit
-//      sequence number side by side (a warp row by a stable LSD radix sort);
+//      order.  A warp row sorts one packed word (column - min) << s | sequence
+//      number per product in registers (warp_sort); a CTA row distributes its
+//      products over fine buckets (bucket_order), then every warp settles the
+//      order inside the buckets of its share in registers (settle), again on
+//      packed words.  Where the column range and the sequence number do not fit
+//      32 bits: a stable LSD radix sort (warp rows), 64-bit words (CTA rows);
+//      a CTA row that repeats a column often takes the radix sort too;
 //   3. sums each run of equal columns sequentially in product order with
 //      __dadd_rn, starting from its first product (the `emplace` then `+=` of
 //      spgemm_exchange.cpp:288-293), and keeps the sums that are != 0.0
@@ -57,53 +59,26 @@ __device__ __forceinline__ int hidx(int d, int w) {
     return W == 1 ? d : d * kHistStride<W> + w;
 }
 
-// Bucket sort (bucket_sort below): 2^kCoarseBits<W> coarse buckets (256 for a
-// CTA row, 32 for a warp row), whose 16-bit counters take kBkCoarseWords<W>
-// words and whose table (first fine bucket, fine bits) kBkInfoWords<W>; then
-// the fine counters.  (7 coarse bits for CTA rows measured 0.25 ms slower on
-// the power-law product.)
+// Buckets of a CTA row (bucket_order below): coarse buckets (their table of two
+// words each, then their counters) and at most one fine bucket per product (and
+// one word past the last).
 template <int W>
-constexpr int kCoarseBits = W == 1 ? 5 : 8;
+constexpr int kCoarseBits = W <= 4 ? 7 : 8;
 template <int W>
-constexpr int kBkCoarseWords = (1 << kCoarseBits<W>) / 2;
-template <int W>
-constexpr int kBkInfoWords = 1 << kCoarseBits<W>;
-// Fine bits of a coarse bucket of n products: floor(log2 n) + fine_extra(cap)
-// (at most the bucket's column bits), so P products take at most
-// P << fine_extra(cap) fine counters, plus one past the last; fine bucket
-// numbers stay below 2^16 (they are stored in 16-bit words).  On the power-law
-// product one extra bit for CTA rows measured 1.1% faster than none (buckets
-// of 0.5-1 products on average instead of 1-2: shorter rank loops), two 5%
-// slower; for warp rows one extra bit measured 4% slower than none.
-constexpr int kFineExtraBits = 1;
-constexpr int kWarpFineExtraBits = 0;
-constexpr int fine_extra(int cap, int w = 2) {
-    int e = w == 1 ? kWarpFineExtraBits : kFineExtraBits;
-    while (e > 0 && (cap << e) >= 65536) --e;
-    return e;
-}
+constexpr int kCoarse = 1 << kCoarseBits<W>;
 template <int W, int ITEMS>
-constexpr int kBkWords = kBkCoarseWords<W> + kBkInfoWords<W> + ((W * 32 * ITEMS) << fine_extra(W * 32 * ITEMS, W)) / 2 + 1;
-
-// In the packed layout the scatter also stores every product's fine bucket
-// beside it (in the sequence-number array, which that layout leaves unused),
-// so that ranking a position reads its bucket instead of recomputing it from
-// the coarse table (0.29 ms of K4 on the power-law product).
-constexpr bool kStoreFine = true;
-// The fine histogram keeps every product's arrival index in its bucket (the
-// counter's old value), so the scatter places products at bucket start plus
-// arrival with no second round of atomics.
-constexpr bool kArrivalScatter = true;
-// Products ranked together in the bucket sort's rank step (see bucket_sort):
-// the largest divisor of ITEMS not above kRankGroup.  On the power-law product:
-// one at a time 13.96 ms of K4, two 13.75, four 13.91, six 13.87 (register
-// pressure grows with the group).
-constexpr int kRankGroup = 2;
-constexpr int rank_group(int items) {
-    for (int g = kRankGroup; g > 1; --g)
-        if (items % g == 0) return g;
-    return 1;
-}
+constexpr int kBucketWords = W == 1 ? 4 : 3 * kCoarse<W> + W * 32 * ITEMS + 4;
+// A warp finishes the sort of its share of a CTA row's positions, rounded to
+// whole buckets, in registers: kShareItems per lane.  A fine bucket larger than
+// the rounding allows sends the row to the radix sort.
+// Against ranking every product inside its bucket by a loop over the bucket in
+// shared memory, then moving it (65-75% of the sort's instructions, waiting on
+// shared memory): rows of 1,025-1,536 products 0.44 -> 0.35 ms (16 uneven
+// uniform products), of which settling the order takes 0.02 ms; power-law
+// product, all bins 11.6 -> 9.3 ms with the other changes of this file.
+template <int ITEMS>
+constexpr int kShareItems = ITEMS + 2;
+constexpr uint32_t kMaxFine = 32;
 // Which rows take the bucket sort: CTA rows.  A warp row sorts its packed keys
 // in registers (spg_warp_sort.cuh).  Against the radix sort of rows of <= 192
 // products and the bucket sort of 193-512 (power-law product, one bin at a
@@ -112,17 +87,6 @@ constexpr int rank_group(int items) {
 // 0.147 ms.  Issue slots bound these kernels, and the network takes about half
 // the instructions of either sort (about 90 a key), none of them waiting on
 // shared memory.
-template <int W, int ITEMS>
-constexpr bool kBucketRows = W > 1;
-// A fine bucket holding more products than this (a column repeated many times)
-// sends the row to the radix sort: ranking inside a bucket is quadratic.
-constexpr uint32_t kMaxFine = 64;
-
-// Digit-counter sets of CTA rows.  CTA rows take the radix sort only where the
-// bucket sort declines, so one set (an extra barrier per pass) leaves them more
-// shared memory.
-constexpr int kHistSets = 1;
-
 // SV: product values in shared memory (else in a per-CTA global slab).
 template <int W, int ITEMS, bool SV = true>
 struct RowSmem {
@@ -133,13 +97,8 @@ struct RowSmem {
     int64_t warp_tmp[W + 1];    // block scans
     uint32_t keys[kCap];        // columns (unpacked) or packed (column, sequence) words
     union {
-        // digit counters of the radix sort at hidx<W>(digit, warp); with two
-        // sets (kHistSets) CTA rows alternate them so that clearing the next
-        // pass's set needs no barrier of its own
-        alignas(16) uint32_t hist[W == 1 ? 1 : kHistSets][kHistWords<W>];
-        // bucket sort of CTA rows: coarse counters, coarse bucket table, fine
-        // counters (16-bit counters, two per word)
-        alignas(16) uint32_t bk[kBucketRows<W, ITEMS> ? kBkWords<W, ITEMS> : 1];
+        alignas(16) uint32_t hist[kHistWords<W>];  // digit counters of the radix sort at hidx<W>(digit, warp)
+        alignas(16) uint32_t bk[kBucketWords<W, ITEMS>];  // bucket counters, then bucket starts (CTA rows)
     };
     uint32_t cnt[W * ITEMS];    // kept entries per (warp, item)
     uint16_t seqs[kCap];        // sequence numbers of the unpacked path
@@ -260,31 +219,6 @@ struct RowOut {
     int32_t nz_add;     // a piece of a split row: add to *nz instead of storing it
 };
 
-// 16-bit counter i of an array of packed pairs (low half: even i).
-__device__ __forceinline__ uint32_t half16(const uint32_t* a, uint32_t i) {
-    return (a[i >> 1] >> ((i & 1u) << 4)) & 0xffffu;
-}
-// Adds one to 16-bit counter i and returns its previous value.
-__device__ __forceinline__ uint32_t bump16(uint32_t* a, uint32_t i) {
-    const uint32_t sh = (i & 1u) << 4;
-    return (atomicAdd(&a[i >> 1], 1u << sh) >> sh) & 0xffffu;
-}
-// bump16 for every valid lane of a warp (all 32 lanes call it), one atomic per
-// run of consecutive lanes with the same counter: consecutive products of one
-// B row mostly fall into the same coarse bucket, and a shared atomic that many
-// lanes aim at one word is serialised.  Valid lanes are a prefix of the warp.
-__device__ __forceinline__ void bump16_runs(uint32_t* a, uint32_t i, bool valid, int lane) {
-    const uint32_t prev = __shfl_up_sync(0xffffffffu, i, 1);
-    const bool head = valid && (lane == 0 || prev != i);
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-    if (head) {
-        const unsigned later = heads & ~((2u << lane) - 1u);  // heads after this lane (lane 31: none)
-        const int next = later ? __ffs(later) - 1 : __popc(vmask);
-        atomicAdd(&a[i >> 1], static_cast<uint32_t>(next - lane) << ((i & 1u) << 4));
-    }
-}
-
 // Exclusive scan of v over the W*32 threads of a row's team in thread order,
 // with the total and the team-wide maximum of m (red: 2*W words; one barrier
 // for a CTA, none for a warp).  red is next written after later barriers of
@@ -317,294 +251,239 @@ __device__ inline uint32_t block_excl_scan_max(uint32_t v, uint32_t m, int32_t* 
     return base + incl - v;
 }
 
-// Zeroes the bucket sort's coarse counters and the fine counters of a row of P
-// products, which the sort expects to find cleared.  Called before the row's
-// enumeration, whose barriers order it before the sort's first atomics; the
-// previous row's sort ended with barriers, so no warp still reads them.
+// Zeroes the counters of a CTA row of P products, which bucket_order expects to
+// find cleared: after the row's enumeration, before the barrier of its column
+// range.
 template <int W, int ITEMS, bool SV>
 __device__ __forceinline__ void clear_buckets(RowSmem<W, ITEMS, SV>& sm, int P, int tid) {
-    constexpr int kExtra = fine_extra(RowSmem<W, ITEMS, SV>::kCap, W);
-    static_assert((RowSmem<W, ITEMS, SV>::kCap << kExtra) < 65536, "fine bucket numbers are 16-bit");
-    uint32_t* fc = sm.bk + kBkCoarseWords<W> + kBkInfoWords<W>;
-    const int fwords = ((P << kExtra) + 2) >> 1;
-    for (int i = tid; i < kBkCoarseWords<W>; i += W * 32) sm.bk[i] = 0u;
-    for (int i = tid; i < fwords; i += W * 32) fc[i] = 0u;
+    uint4* b4 = reinterpret_cast<uint4*>(sm.bk + 2 * kCoarse<W>);  // coarse counters, fine counters 0 .. P
+    const int n4 = (kCoarse<W> + P + 4) / 4;
+    for (int i = tid; i < n4; i += W * 32) b4[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Step 2 of a CTA row without digit passes: the products (columns at
-// keys[0..P), offsets k = column - cmin of nbits >= 1 bits, sequence number =
-// position) are bucketed, then ranked inside their bucket.
-//   * coarse buckets: the top min(nbits, 8) bits of k (16-bit counters);
+// Orders a CTA row's products (columns at keys[0..P), sequence number =
+// position, offsets k = column - cmin of nbits >= 1 bits) by fine bucket, in any
+// order inside a bucket: seqs then holds their sequence numbers (the columns stay
+// where they are), the fine counters hold the bucket starts.
+//   * coarse buckets: the top bits of k;
 //   * coarse bucket c of n_c products gets 2^fb_c fine buckets over its column
-//     span, fb_c = min(span bits, floor(log2 n_c)), so that dense parts of the
-//     row (the diagonal band of a banded product) get finer buckets than sparse
-//     ones and no more fine buckets than products exist;
-//   * the products are scattered into their fine buckets in any order (shared
-//     atomics), then every product finds its place in its bucket by counting
-//     the bucket's products with a smaller (column, sequence) pair: the pair is
-//     unique, so the result is the order of a stable sort by column, the
-//     reference's order of every column's products.
+//     span, fb_c = min(span bits, floor(log2 n_c)), so that dense parts of the row
+//     (the diagonal band of a banded product) get finer buckets than sparse ones:
+//     one or two products per bucket on average;
+//   * the fine histogram's atomics give every product its arrival index in its
+//     bucket, so that it is placed without a second round of atomics.
 // Instruction cost per product does not grow with the column range, unlike a
-// digit pass.  Returns false, leaving keys untouched, when a fine bucket would
-// hold more than kMaxFine products (a column repeated that often); the row then
-// takes the radix sort.  On success keys (and seqs when !PACKED) hold the sorted
-// products in the layout finish_row reads: packed (column - cmin, sequence)
-// words, or columns and 16-bit sequence numbers side by side.
-template <int W, int ITEMS, bool SV, bool PACKED>
-__device__ bool bucket_sort(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits, int lane, int warp,
-                            int tid) {
-    using Sm = RowSmem<W, ITEMS, SV>;
+// digit pass.  Returns the largest bucket's size; above kMaxFine seqs is not
+// written.
+template <int W, int ITEMS, bool SV>
+__device__ __forceinline__ uint32_t bucket_order(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits, int lane,
+                                                 int warp, int tid, int& nfine) {
     constexpr int NT = W * 32;
-    constexpr int kSeqBits = Sm::kSeqBits;
-    static_assert(kBucketRows<W, ITEMS>, "rows of this shape have no bucket counters");
-    uint32_t* cc = sm.bk;                                     // coarse counters
-    uint32_t* info = sm.bk + kBkCoarseWords<W>;                  // first fine bucket | fine bits << 16
-    uint32_t* fc = sm.bk + kBkCoarseWords<W> + kBkInfoWords<W>;     // fine counters, then starts, then ends
-    const int cbits = nbits < kCoarseBits<W> ? nbits : kCoarseBits<W>;
-    const int sc = nbits - cbits;                             // column bits inside a coarse bucket
-    const uint32_t scmask = (1u << sc) - 1u;
-    // 0. the coarse counters and the fine counters of P products are zero on
-    //    entry (clear_buckets, before the row's enumeration)
-    constexpr int kExtra = fine_extra(Sm::kCap, W);
-    const int fwords = ((P << kExtra) + 2) >> 1;  // one counter past the last fine bucket
-    // 1. coarse histogram
-    uint32_t k[ITEMS], f[ITEMS];
+    uint2* info = reinterpret_cast<uint2*>(sm.bk);  // fine bucket of k = x + (k >> y)
+    uint32_t* cc = sm.bk + 2 * kCoarse<W>;          // coarse counters
+    uint32_t* fc = sm.bk + 3 * kCoarse<W>;          // fine counters, then starts
+    const int sc = max(nbits - kCoarseBits<W>, 0);  // column bits inside a coarse bucket
+    uint32_t f[ITEMS];
+    // Position i * NT + tid: whole steps past P are skipped, and no warp is left
+    // with less than its share when P is below the capacity.
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
-        const int pos = (warp * ITEMS + i) * 32 + lane;
-        k[i] = pos < P ? sm.keys[pos] - cmin : 0u;
-        bump16_runs(cc, k[i] >> sc, pos < P, lane);
+        if (i * NT >= P) break;
+        const int pos = i * NT + tid;
+        if (pos < P) atomicAdd(&cc[(sm.keys[pos] - cmin) >> sc], 1u);
     }
-    row_sync<W>();
-    // 2. fine buckets of every coarse bucket, numbered in coarse order: every
-    //    warp computes the whole table and stores it (the same words with the
-    //    same values), so that only a warp-level barrier precedes its use
+    __syncthreads();
+    // every warp computes the whole table and stores it (the same words with the
+    // same values), so that only a warp-level barrier precedes its use
     {
-        constexpr int kPer = (1 << kCoarseBits<W>) / 32;  // coarse buckets per lane
-        uint32_t fcount[kPer], fbits[kPer], sum = 0;
+        constexpr int kPer = kCoarse<W> / 32;
+        uint32_t n[kPer], bits[kPer], sum = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; j += 4) *reinterpret_cast<uint4*>(n + j) = *reinterpret_cast<const uint4*>(cc + lane * kPer + j);
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const uint32_t n = half16(cc, static_cast<uint32_t>(lane * kPer + j));  // zero beyond 2^cbits
-            const int lg = n ? 31 - __clz(n) + kExtra : 0;
-            fbits[j] = static_cast<uint32_t>(lg < sc ? lg : sc);
-            fcount[j] = n ? (1u << fbits[j]) : 0u;
-            sum += fcount[j];
+            bits[j] = min(31u - __clz(n[j] | 1u), static_cast<uint32_t>(sc));
+            n[j] = n[j] ? 1u << bits[j] : 0u;
+            sum += n[j];
         }
-        uint32_t base = warp_incl_scan(sum, lane) - sum;
+        const uint32_t incl = warp_incl_scan(sum, lane);
+        nfine = static_cast<int>(__shfl_sync(0xffffffffu, incl, 31));
+        uint32_t base = incl - sum;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            info[lane * kPer + j] = base | (fbits[j] << 16);
-            base += fcount[j];
+            info[lane * kPer + j] = make_uint2(base - (static_cast<uint32_t>(lane * kPer + j) << bits[j]),
+                                               static_cast<uint32_t>(sc) - bits[j]);
+            base += n[j];
         }
     }
     __syncwarp();
-    // 3. fine histogram
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
-        const int pos = (warp * ITEMS + i) * 32 + lane;
-        f[i] = 0u;
-        if (pos < P) {
-            const uint32_t in = info[k[i] >> sc];
-            f[i] = (in & 0xffffu) + ((k[i] & scmask) >> (sc - static_cast<int>(in >> 16)));
-            if constexpr (kArrivalScatter) f[i] |= bump16(fc, f[i]) << 16;  // arrival in the high half
-            else bump16(fc, f[i]);
+        if (i * NT >= P) break;
+        if (i * NT + tid < P) {
+            const uint32_t k = sm.keys[i * NT + tid] - cmin;
+            const uint2 in = info[k >> sc];
+            f[i] = in.x + (k >> in.y);
+            f[i] |= atomicAdd(&fc[f[i]], 1u) << 16;  // arrival in the high half
         }
     }
-    row_sync<W>();
-    // 4. exclusive scan of the fine counters (at most P of them; contiguous
-    //    words per thread), and the largest fine bucket
+    __syncthreads();
+    // exclusive scan of the fine counters, ITEMS consecutive ones per thread
+    uint32_t gmax;
     {
-        const int per = (fwords + NT - 1) / NT;
-        const int w0 = tid * per;
-        const int w1 = min(w0 + per, fwords);
-        uint32_t sum = 0, mx = 0;
-        for (int w = w0; w < w1; ++w) {
-            const uint32_t x = fc[w];
-            const uint32_t lo = x & 0xffffu, hi = x >> 16;
-            sum += lo + hi;
-            mx = max(mx, max(lo, hi));
+        const int w0 = tid * ITEMS;
+        const bool act = w0 <= nfine;  // the bucket past the last included: its start is P
+        uint32_t x[ITEMS], sum = 0, mx = 0;
+        constexpr int V = ITEMS % 4 == 0 ? 4 : (ITEMS % 2 == 0 ? 2 : 1);
+        using Vec = std::conditional_t<V == 4, uint4, std::conditional_t<V == 2, uint2, uint32_t>>;
+        if (act) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; j += V) *reinterpret_cast<Vec*>(x + j) = *reinterpret_cast<const Vec*>(fc + w0 + j);
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                if (w0 + j >= nfine) x[j] = 0u;  // not cleared past P
+                sum += x[j];
+                mx = max(mx, x[j]);
+            }
         }
-        uint32_t total, gmax;
+        uint32_t total;
         uint32_t base = block_excl_scan_max<W>(sum, mx, sm.red, lane, warp, total, gmax);
-        if (gmax > kMaxFine) return false;  // uniform: every thread saw the same maximum
-        for (int w = w0; w < w1; ++w) {
-            const uint32_t x = fc[w];
-            const uint32_t lo = x & 0xffffu;
-            fc[w] = base | ((base + lo) << 16);
-            base += lo + (x >> 16);
+        if (gmax > kMaxFine) return gmax;  // uniform: every thread saw the same maximum
+        if (act) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                const uint32_t n = x[j];
+                x[j] = base;
+                base += n;
+            }
+#pragma unroll
+            for (int j = 0; j < ITEMS; j += V) *reinterpret_cast<Vec*>(fc + w0 + j) = *reinterpret_cast<const Vec*>(x + j);
         }
+        if (tid == 0 && nfine == W * 32 * ITEMS) fc[nfine] = static_cast<uint32_t>(P);
     }
-    row_sync<W>();
-    // 5. scatter into the fine buckets (any order inside a bucket)
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
-        const int pos = (warp * ITEMS + i) * 32 + lane;
+        if (i * NT >= P) break;
+        const int pos = i * NT + tid;
         if (pos < P) {
-            const uint32_t fi = f[i] & 0xffffu;
-            const uint32_t at = kArrivalScatter ? half16(fc, fi) + (f[i] >> 16) : bump16(fc, fi);
-            if constexpr (PACKED) {
-                sm.keys[at] = (k[i] << kSeqBits) | static_cast<uint32_t>(pos);
-                if constexpr (kStoreFine) sm.seqs[at] = static_cast<uint16_t>(fi);
-            } else {
-                sm.keys[at] = k[i] + cmin;  // the unpacked layout keeps columns
-                sm.seqs[at] = static_cast<uint16_t>(pos);
-            }
+            sm.seqs[fc[f[i] & 0xffffu] + (f[i] >> 16)] = static_cast<uint16_t>(pos);
         }
     }
-    row_sync<W>();
-    // 6. every sorted position takes its product's place inside the product's
-    //    bucket: the number of the bucket's products with a smaller (column,
-    //    sequence) pair.  Positions run in lane order, so the lanes of a warp
-    //    mostly share buckets (same loop bounds, broadcast loads).  The counters
-    //    hold every bucket's start (arrival scatter; the one past the last bucket
-    //    holds P) or its end.
-    uint32_t* const dst = f;  // the fine indices are no longer needed
-    uint32_t* const key = k;  // nor the column offsets
-    uint32_t sqv[PACKED ? 1 : ITEMS];  // sequence numbers of the unpacked layout
-    // Positions are ranked kRankGroup at a time in lock-step: their buckets'
-    // bounds are loaded together, then one loop over the longest of their
-    // buckets issues independent loads for all of them.
-    constexpr int G = rank_group(ITEMS);
-#pragma unroll
-    for (int i0 = 0; i0 < ITEMS; i0 += G) {
-        uint32_t beg[G], len[G], r[G], maxlen = 0;
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const int i = i0 + g;
-            const int p = (warp * ITEMS + i) * 32 + lane;
-            key[i] = 0u;
-            beg[g] = 0u;
-            len[g] = 0u;
-            r[g] = 0u;
-            if (p < P) {
-                key[i] = sm.keys[p];
-                uint32_t fb;
-                if constexpr (PACKED && kStoreFine) {
-                    fb = sm.seqs[p];
-                } else {
-                    const uint32_t kk = PACKED ? key[i] >> kSeqBits : key[i] - cmin;
-                    const uint32_t in = info[kk >> sc];
-                    fb = (in & 0xffffu) + ((kk & scmask) >> (sc - static_cast<int>(in >> 16)));
-                }
-                if constexpr (!PACKED) sqv[i] = sm.seqs[p];
-                // counters hold bucket starts (arrival scatter) or ends
-                const uint32_t end = kArrivalScatter ? half16(fc, fb + 1u) : half16(fc, fb);
-                beg[g] = kArrivalScatter ? half16(fc, fb) : (fb ? half16(fc, fb - 1u) : 0u);
-                len[g] = end - beg[g];
-                maxlen = max(maxlen, len[g]);
-            }
-        }
-        for (uint32_t q = 0; q < maxlen; ++q) {
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const int i = i0 + g;
-                if (q < len[g]) {
-                    const uint32_t kq = sm.keys[beg[g] + q];
-                    if constexpr (PACKED) {
-                        r[g] += kq < key[i] ? 1u : 0u;
-                    } else {
-                        r[g] += (kq < key[i] || (kq == key[i] && sm.seqs[beg[g] + q] < sqv[i])) ? 1u : 0u;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) dst[i0 + g] = beg[g] + r[g];
-    }
-    row_sync<W>();
-    // 7. products at their sorted positions
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int p = (warp * ITEMS + i) * 32 + lane;
-        if (p < P) {
-            sm.keys[dst[i]] = key[i];
-            if constexpr (!PACKED) sm.seqs[dst[i]] = static_cast<uint16_t>(sqv[i]);
-        }
-    }
-    row_sync<W>();
-    return true;
+    __syncthreads();
+    return gmax;
 }
 
+// The warp's share of the positions [0, P): from the bucket that holds position
+// warp * ceil(P / W) to the one that holds the next warp's first.  Bucket starts
+// are monotone: each half of the warp narrows its bound 16-fold per step.
+template <int W, int ITEMS, bool SV>
+__device__ __forceinline__ void warp_share(const RowSmem<W, ITEMS, SV>& sm, int P, int nfine, int lane, int warp, int& x0,
+                                           int& x1) {
+    const uint32_t* fc = sm.bk + 3 * kCoarse<W>;
+    const int share = (P + W - 1) / W;
+    const int half = lane >> 4, l = lane & 15;
+    const int m = (warp + half) * share;
+    int lo = 0, n = 1;
+    uint32_t v = 0;
+    for (int range = nfine + 1; range > 1;) {
+        const int stride = (range + 15) >> 4;
+        const int i = lo + l * stride;
+        v = i <= nfine ? fc[i] : 0xffffu;
+        const unsigned below = __ballot_sync(0xffffffffu, static_cast<int>(v) <= m);
+        n = __popc((below >> (half * 16)) & 0xffffu);
+        lo += (n - 1) * stride;
+        range = stride;
+    }
+    v = __shfl_sync(0xffffffffu, v, half * 16 + n - 1);
+    const int x = m >= P ? P : static_cast<int>(v);
+    x0 = __shfl_sync(0xffffffffu, x, 0);
+    x1 = __shfl_sync(0xffffffffu, x, 16);
+}
+
+// Odd-even transposition of a warp's 32 * N keys (lane l holds keys l * N ... of
+// the sequence, N even): `rounds` rounds sort a sequence whose keys are out of
+// order only inside runs of at most `rounds` positions.
+template <int N, typename K>
+__device__ __forceinline__ void settle(K (&k)[N], int rounds, int lane) {
+    static_assert(N % 2 == 0, "pairs keep their parity from lane to lane");
+    for (int r = 0; r < rounds; r += 2) {
+#pragma unroll
+        for (int i = 0; i + 1 < N; i += 2) compare_exchange(k, i, i + 1);
+        const K up = __shfl_down_sync(0xffffffffu, k[0], 1), down = __shfl_up_sync(0xffffffffu, k[N - 1], 1);
+#pragma unroll
+        for (int i = 1; i + 1 < N; i += 2) compare_exchange(k, i, i + 1);
+        if (lane < 31) k[N - 1] = min(k[N - 1], up);
+        if (lane > 0) k[0] = max(k[0], down);
+    }
+}
+
+// Sorts a share whose (column, sequence) pairs do not fit 32 bits, at keys /
+// seqs [0, n) in bucket order, as 64-bit keys.
+template <int N>
+__device__ __noinline__ void settle_wide(uint32_t* keys, uint16_t* seqs, int n, int rounds, int lane) {
+    unsigned long long k[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int p = lane * N + i;
+        k[i] = p < n ? (static_cast<unsigned long long>(keys[p]) << 16) | seqs[p] : ~0ull;
+    }
+    settle(k, rounds, lane);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int p = lane * N + i;
+        if (p < n) {
+            keys[p] = static_cast<uint32_t>(k[i] >> 16);
+            seqs[p] = static_cast<uint16_t>(k[i]);
+        }
+    }
+    __syncwarp();
+}
+
+// True unless v is +0.0 or -0.0 (NaN included), without the FP64 pipe, which
+// takes 16 cycles for a warp's instruction.
+__device__ __forceinline__ bool nonzero(double v) {
+    return (static_cast<unsigned long long>(__double_as_longlong(v)) << 1) != 0ull;
+}
 
 // The stable LSD radix sort of a row's products by column: 8-bit digits over
 // the bits of max(col) - min(col), and with kNarrow a last pass of at most 4
-// bits (four votes, 16 counters per warp) when no more remain.  Leaves keys
-// (and seqs when !PACKED) in the layout finish_row reads.
-template <int W, int ITEMS, bool SV, bool PACKED, bool kNarrow>
+// bits (four votes, 16 counters per warp) when no more remain.  Leaves columns
+// in keys and sequence numbers in seqs.
+template <int W, int ITEMS, bool SV, bool kNarrow>
 __device__ __forceinline__ void radix_sort_row(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits, int lane,
                                                int warp, int tid) {
-    constexpr int kSeqBits = RowSmem<W, ITEMS, SV>::kSeqBits;
-    int hb = 0;  // counter set of this pass
     auto digits_from = [&](int shift) { return (kNarrow && nbits - shift <= 4) ? 16 : 256; };
-    if constexpr (PACKED) {
-        if (nbits == 0) {  // one column: already in sequence order; just pack
-#pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const int pos = (warp * ITEMS + i) * 32 + lane;
-                if (pos < P) sm.keys[pos] = ((sm.keys[pos] - cmin) << kSeqBits) | static_cast<uint32_t>(pos);
-            }
-        }
-    } else {
-        for (int i = tid; i < P; i += W * 32) sm.seqs[i] = static_cast<uint16_t>(i);
-    }
-    if (nbits > 0) clear_counters<W>(sm.hist[0], digits_from(0), tid);
+    for (int i = tid; i < P; i += W * 32) sm.seqs[i] = static_cast<uint16_t>(i);
+    if (nbits > 0) clear_counters<W>(sm.hist, digits_from(0), tid);
     row_sync<W>();
     // One pass over the digit of NB bits at `shift` (NB = 8, or 4 for the last).
     auto pass = [&](auto nb, int shift) {
         constexpr int NB = decltype(nb)::value;
         constexpr uint32_t kMask = (1u << NB) - 1u;
-        uint32_t* hist = sm.hist[hb];
+        uint32_t* hist = sm.hist;
         uint32_t k[ITEMS], rk[ITEMS];
-        if constexpr (PACKED) {
-            // Packed words (col - cmin) << kSeqBits | seq; the first pass packs.
+        uint16_t sq[ITEMS];
 #pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const int pos = (warp * ITEMS + i) * 32 + lane;
-                uint32_t d = kMask;
-                k[i] = 0xffffffffu;
-                if (pos < P) {
-                    const uint32_t raw = sm.keys[pos];
-                    k[i] = shift == 0 ? ((raw - cmin) << kSeqBits) | static_cast<uint32_t>(pos) : raw;
-                    d = (k[i] >> (kSeqBits + shift)) & kMask;
-                }
-                rk[i] = rank_item<NB>(d, &hist[hidx<W>(d, warp)], lane);
-            }
-            row_sync<W>();
-            scan_counters<W, (1 << NB)>(hist, sm.warp_tmp);
-            row_sync<W>();
+        for (int i = 0; i < ITEMS; ++i) {
+            const int pos = (warp * ITEMS + i) * 32 + lane;
+            const bool valid = pos < P;
+            k[i] = valid ? sm.keys[pos] : 0u;
+            sq[i] = valid ? sm.seqs[pos] : uint16_t{0};
+            const uint32_t d = valid ? (((k[i] - cmin) >> shift) & kMask) : kMask;
+            rk[i] = rank_item<NB>(d, &hist[hidx<W>(d, warp)], lane);
+        }
+        row_sync<W>();
+        scan_counters<W, (1 << NB)>(hist, sm.warp_tmp);
+        row_sync<W>();
 #pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                // Padding items were ranked under the largest digit, after every
-                // real item of that digit; they are not stored.
-                const int pos = (warp * ITEMS + i) * 32 + lane;
-                if (pos < P) {
-                    const uint32_t d = (k[i] >> (kSeqBits + shift)) & kMask;
-                    sm.keys[hist[hidx<W>(d, warp)] + rk[i]] = k[i];
-                }
-            }
-        } else {
-            uint16_t sq[ITEMS];
-#pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const int pos = (warp * ITEMS + i) * 32 + lane;
-                const bool valid = pos < P;
-                k[i] = valid ? sm.keys[pos] : 0u;
-                sq[i] = valid ? sm.seqs[pos] : uint16_t{0};
-                const uint32_t d = valid ? (((k[i] - cmin) >> shift) & kMask) : kMask;
-                rk[i] = rank_item<NB>(d, &hist[hidx<W>(d, warp)], lane);
-            }
-            row_sync<W>();
-            scan_counters<W, (1 << NB)>(hist, sm.warp_tmp);
-            row_sync<W>();
-#pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const int pos = (warp * ITEMS + i) * 32 + lane;
-                const uint32_t d = pos < P ? (((k[i] - cmin) >> shift) & kMask) : kMask;
-                const uint32_t dst = hist[hidx<W>(d, warp)] + rk[i];
-                if (dst < static_cast<uint32_t>(P)) {
-                    sm.keys[dst] = k[i];
-                    sm.seqs[dst] = sq[i];
-                }
+        for (int i = 0; i < ITEMS; ++i) {
+            const int pos = (warp * ITEMS + i) * 32 + lane;
+            const uint32_t d = pos < P ? (((k[i] - cmin) >> shift) & kMask) : kMask;
+            const uint32_t dst = hist[hidx<W>(d, warp)] + rk[i];
+            if (dst < static_cast<uint32_t>(P)) {  // padding ranks last
+                sm.keys[dst] = k[i];
+                sm.seqs[dst] = sq[i];
             }
         }
     };
@@ -616,53 +495,148 @@ __device__ __forceinline__ void radix_sort_row(RowSmem<W, ITEMS, SV>& sm, int P,
             if constexpr (kNarrow) pass(std::integral_constant<int, 4>{}, shift);
             shift += 4;
         }
-        const bool more = shift < nbits;
-        if constexpr (W == 1) {
-            __syncwarp();
-            if (more) clear_counters<W>(sm.hist[0], digits_from(shift), tid);
-        } else if constexpr (kHistSets == 2) {
-            if (more) clear_counters<W>(sm.hist[hb ^ 1], digits_from(shift), tid);
-            hb ^= 1;
-        } else {
-            __syncthreads();  // the scatter above still reads the counters
-            if (more) clear_counters<W>(sm.hist[0], digits_from(shift), tid);
-        }
+        row_sync<W>();  // the scatter above still reads the counters
+        if (shift < nbits) clear_counters<W>(sm.hist, digits_from(shift), tid);
         row_sync<W>();
     }
-
 }
 
-// The radix sort of CTA rows that the bucket sort declined (a column repeated
-// more than kMaxFine times): rare, so it keeps the code small rather than fast
-// -- one key layout (columns and sequence numbers) and 8-bit digits only, then
-// the packed words when the row's layout is packed.  Less code in the CTA
-// kernels measured 0.25 ms faster on the power-law product than the full radix
-// sort inline.
-template <int W, int ITEMS, bool SV, bool PACKED>
-__device__ __forceinline__ void radix_sort_fallback(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits,
-                                                    int lane, int warp, int tid) {
-    constexpr int kSeqBits = RowSmem<W, ITEMS, SV>::kSeqBits;
-    radix_sort_row<W, ITEMS, SV, false, false>(sm, P, cmin, nbits, lane, warp, tid);
-    if constexpr (PACKED) {
-        for (int i = tid; i < P; i += W * 32) sm.keys[i] = ((sm.keys[i] - cmin) << kSeqBits) | sm.seqs[i];
-        row_sync<W>();  // a warp row's team is its warp: never a CTA barrier there
+constexpr uint32_t kDeadKey = 0xffffffffu;
+
+// Step 3 of a sorted region of n positions, by one warp: lane l holds the words
+// (column offset << S | sequence number) of positions l * N ... in k.  Stores
+// them at keys[0..n), sums every run of equal column offsets in product order
+// into the value of its first product, and turns the words of the run's other
+// products into kDeadKey (no word's column offset is all ones).  The runs of
+// more than one product are first listed (list: n 16-bit words), so that the
+// warp sums 32 of them at a time: an FP64 instruction takes 16 cycles of an SM
+// whether one lane needs it or all.
+template <int N, int S>
+__device__ __forceinline__ void fold_runs(const uint32_t (&k)[N], uint32_t* keys, uint16_t* list, double* vals, int n,
+                                          int lane) {
+    using Mask = std::conditional_t<(N < 32), uint32_t, unsigned long long>;
+    const uint32_t before = __shfl_up_sync(0xffffffffu, k[N - 1], 1);
+    Mask same = 0;  // positions that continue a run
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint32_t p = i ? k[i - 1] : before;
+        if (((k[i] ^ p) >> S) == 0u) same |= Mask{1} << i;
+        if (lane * N + i < n) keys[lane * N + i] = k[i];
     }
+    if (lane == 0) same &= ~Mask{1};
+    const int mine = min(max(n - lane * N, 0), N);
+    same &= (Mask{1} << mine) - 1;
+    const uint32_t next = __shfl_down_sync(0xffffffffu, static_cast<uint32_t>(same), 1);
+    Mask starts = ~same & ((same >> 1) | (lane < 31 ? static_cast<Mask>(next & 1u) << (N - 1) : Mask{0}));
+    __syncwarp();
+    if (!__any_sync(0xffffffffu, starts != 0)) return;
+    const uint32_t count = N < 32 ? __popc(static_cast<uint32_t>(starts)) : __popcll(starts);
+    const uint32_t incl = warp_incl_scan(count, lane);
+    const uint32_t runs = __shfl_sync(0xffffffffu, incl, 31);
+    for (uint32_t at = incl - count; starts; starts &= starts - 1) {
+        const int i = (N < 32 ? __ffs(static_cast<uint32_t>(starts)) : __ffsll(static_cast<long long>(starts))) - 1;
+        list[at++] = static_cast<uint16_t>(lane * N + i);
+    }
+    __syncwarp();
+    constexpr uint32_t kSeq = (1u << S) - 1u;
+    for (uint32_t j = lane; j < runs; j += 32) {
+        int q = list[j];
+        const uint32_t key = keys[q];
+        double acc = vals[key & kSeq];
+        for (++q; q < n; ++q) {
+            const uint32_t other = keys[q];
+            if ((other ^ key) >> S) break;
+            acc = __dadd_rn(acc, vals[other & kSeq]);
+            keys[q] = kDeadKey;
+        }
+        vals[key & kSeq] = acc;
+    }
+    __syncwarp();
+}
+
+// Upper-bound mode, step 4 of a region after fold_runs: position p owns slot p
+// of [oc, ov); a run's first position writes (column, sum) when the sum is != 0,
+// every other slot column -1.  A slot without an entry gets its value written
+// all the same: a sector of DRAM written in part costs a read.  Returns the
+// region's kept sums.
+template <int S>
+__device__ __forceinline__ uint32_t write_slots(const uint32_t* keys, const double* vals, int n, uint32_t first,
+                                                int32_t* __restrict__ oc, double* __restrict__ ov, int lane) {
+    constexpr int U = 4;
+    uint32_t kept = 0;
+    for (int p0 = lane; p0 - lane < n; p0 += 32 * U) {
+        uint32_t key[U];
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int p = p0 + u * 32;
+            key[u] = p < n ? keys[p] : kDeadKey;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = key[u] != kDeadKey ? vals[key[u] & ((1u << S) - 1u)] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int p = p0 + u * 32;
+            const bool keep = nonzero(v[u]);
+            if (p < n) {
+                oc[p] = keep ? static_cast<int32_t>((key[u] >> S) + first) : -1;
+                ov[p] = v[u];
+            }
+            kept += __popc(__ballot_sync(0xffffffffu, keep));
+        }
+    }
+    return kept;
+}
+
+// write_slots for the rows that keep columns and sequence numbers apart: slots
+// [x0, x1) of a row whose runs may start or end anywhere in [lo, hi).  Returns
+// the warp's kept sums.
+__device__ __noinline__ uint32_t write_slots_plain(const uint32_t* keys, const uint16_t* seqs, const double* vals, int x0,
+                                                   int x1, int lo, int hi, int32_t* oc, double* ov, int lane) {
+    uint32_t kept = 0;
+    for (int p = x0 + lane; p < x1; p += 32) {
+        const uint32_t c = keys[p];
+        double acc = 0.0;
+        if (p == lo || keys[p - 1] != c) {
+            acc = vals[seqs[p]];
+            for (int q = p + 1; q < hi && keys[q] == c; ++q) acc = __dadd_rn(acc, vals[seqs[q]]);
+        }
+        const bool keep = nonzero(acc);
+        oc[p] = keep ? static_cast<int32_t>(c) : -1;
+        ov[p] = acc;
+        kept += keep;
+    }
+    __syncwarp();
+    return __reduce_add_sync(0xffffffffu, kept);
+}
+
+// The radix sort of the CTA rows with a large bucket (a column repeated more
+// than kMaxFine times): out of line, so that it takes no registers from the
+// rows that do not need it.
+template <int W, int ITEMS, bool SV>
+__device__ __noinline__ void radix_sort_cta(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits, int lane, int warp,
+                                            int tid) {
+    radix_sort_row<W, ITEMS, SV, false>(sm, P, cmin, nbits, lane, warp, tid);
 }
 
 // Steps 2-4 of a row for one key layout (PACKED: (col - cmin) << kSeqBits | seq
-// words; otherwise columns and 16-bit sequence numbers).  Returns the stored
-// entries this thread accounts for (its warp's on lane 0 in upper-bound mode,
-// the row's on thread 0 in exact mode, else 0).  No barrier ends the row: the
-// next row's enumeration passes a barrier before it writes what this phase
-// reads (keys, values, sequence numbers, kept counts).
+// words, warp rows only; otherwise columns and 16-bit sequence numbers).
+// Returns the stored entries this thread accounts for (its warp's on lane 0 in
+// upper-bound mode, the row's on thread 0 in exact mode, else 0).  No barrier
+// ends the row: the next row's enumeration passes a barrier before it writes
+// what this phase reads (keys, values, sequence numbers, bucket starts, kept
+// counts).
 template <int W, int ITEMS, bool SV, bool PACKED>
-__device__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, double* vals, int P, uint32_t cmin,
-                           int nbits, int lane, int warp, int tid) {
+__device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, double* vals, int P,
+                                               uint32_t cmin, uint32_t range, int nbits, int lane, int warp, int tid) {
     using Sm = RowSmem<W, ITEMS, SV>;
     constexpr int kSeqBits = Sm::kSeqBits;
+    constexpr uint32_t kMaxRange = 0xffffffffu >> kSeqBits;  // below it no packed word is kDeadKey
     // 2. sort by column: warp rows in registers (the padding words above P sort
     //    last: a real word is all ones only when P is the row's capacity), CTA
-    //    rows by the bucket sort, and by the radix sort where that declines
+    //    rows by bucket and then, inside the buckets, in registers, and by the
+    //    radix sort where a bucket is large
+    uint32_t kept = 0;
     if constexpr (W == 1 && PACKED) {
         uint32_t k[ITEMS];
 #pragma unroll
@@ -670,16 +644,101 @@ __device__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, dou
             const int pos = i * 32 + lane;
             k[i] = pos < P ? ((sm.keys[pos] - cmin) << kSeqBits) | static_cast<uint32_t>(pos) : 0xffffffffu;
         }
-        warp_sort<ITEMS>(k, lane);
+        warp_sort(k, lane);
         __syncwarp();
+        if (out.holes) {
+            fold_runs<ITEMS, kSeqBits>(k, sm.keys, sm.seqs, vals, P, lane);
+            kept = write_slots<kSeqBits>(sm.keys, vals, P, cmin, out.c_col + out.out0, out.c_val + out.out0, lane);
+            if (lane == 0) *out.nz = kept;
+            return lane == 0 ? kept : 0u;
+        }
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) sm.keys[lane * ITEMS + i] = k[i];
         __syncwarp();
     } else if constexpr (W == 1) {
-        radix_sort_row<W, ITEMS, SV, PACKED, true>(sm, P, cmin, nbits, lane, warp, tid);
+        radix_sort_row<W, ITEMS, SV, true>(sm, P, cmin, nbits, lane, warp, tid);
     } else {
-        if (nbits == 0 || !bucket_sort<W, ITEMS, SV, PACKED>(sm, P, cmin, nbits, lane, warp, tid))
-            radix_sort_fallback<W, ITEMS, SV, PACKED>(sm, P, cmin, nbits, lane, warp, tid);
+        constexpr int N = kShareItems<ITEMS>;
+        int x0 = warp * ((P + W - 1) / W), x1 = x0 + (P + W - 1) / W, nfine = 0;
+        bool by_share = false, written = false;
+        if (nbits == 0) {
+            for (int i = tid; i < P; i += W * 32) sm.seqs[i] = static_cast<uint16_t>(i);
+            __syncthreads();
+        } else {
+            const uint32_t biggest = bucket_order(sm, P, cmin, nbits, lane, warp, tid, nfine);
+            if (biggest > kMaxFine) {
+                radix_sort_cta(sm, P, cmin, nbits, lane, warp, tid);
+            } else {
+                // Every warp settles the order inside the buckets of its share:
+                // from here on the warps work without a barrier.
+                by_share = true;
+                warp_share(sm, P, nfine, lane, warp, x0, x1);
+                const int n = x1 - x0;
+                uint32_t* keys = sm.keys + x0;
+                uint16_t* seqs = sm.seqs + x0;
+                // column offsets from `first`: the row's smallest column where the row's
+                // range and sequence numbers fit 32 bits, else the share's
+                uint32_t first = cmin;
+                bool wide = false;
+                if (range >= kMaxRange) {
+                    uint32_t lo = 0xffffffffu, hi = 0;
+                    for (int p = lane; p < n; p += 32) {
+                        const uint32_t c = sm.keys[seqs[p]];
+                        lo = min(lo, c);
+                        hi = max(hi, c);
+                    }
+                    first = __reduce_min_sync(0xffffffffu, lo);
+                    hi = __reduce_max_sync(0xffffffffu, hi);
+                    wide = n > 0 && hi - first >= kMaxRange;
+                }
+                uint32_t k[N];
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    const int p = lane * N + i;
+                    k[i] = kDeadKey;
+                    if (p < n) {
+                        const uint32_t s = seqs[p];
+                        k[i] = wide ? sm.keys[s] : ((sm.keys[s] - first) << kSeqBits) | s;
+                    }
+                }
+                __syncthreads();  // every warp has read its columns: keys is free
+                if (wide) {
+#pragma unroll
+                    for (int i = 0; i < N; ++i)
+                        if (lane * N + i < n) keys[lane * N + i] = k[i];
+                    __syncwarp();
+                    settle_wide<N>(keys, seqs, n, static_cast<int>(biggest), lane);
+                } else {
+                    settle(k, static_cast<int>(biggest), lane);
+                    if (out.holes) {
+                        fold_runs<N, kSeqBits>(k, keys, seqs, vals, n, lane);
+                        kept = write_slots<kSeqBits>(keys, vals, n, first, out.c_col + out.out0 + x0,
+                                                     out.c_val + out.out0 + x0, lane);
+                        written = true;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < N; ++i) {
+                            const int p = lane * N + i;
+                            if (p < n) {
+                                keys[p] = (k[i] >> kSeqBits) + first;
+                                seqs[p] = static_cast<uint16_t>(k[i] & ((1u << kSeqBits) - 1u));
+                            }
+                        }
+                    }
+                }
+                if (!out.holes) __syncthreads();
+            }
+        }
+        if (out.holes) {
+            x0 = min(x0, P);
+            x1 = min(x1, P);
+            if (!written)  // shares cut anywhere unless they are whole buckets: runs may cross them
+                kept = write_slots_plain(sm.keys, sm.seqs, vals, x0, x1, by_share ? x0 : 0, by_share ? x1 : P,
+                                         out.c_col + out.out0, out.c_val + out.out0, lane);
+            if (lane == 0 && kept)  // the row's count was zeroed before its enumeration
+                atomicAdd(reinterpret_cast<unsigned long long*>(out.nz), static_cast<unsigned long long>(kept));
+            return lane == 0 ? kept : 0u;
+        }
     }
 
     // Column and sequence number of sorted position pos.
@@ -690,38 +749,12 @@ __device__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, dou
         return PACKED ? (sm.keys[pos] & ((1u << kSeqBits) - 1u)) : sm.seqs[pos];
     };
 
-    if (out.holes) {
-        // 3+4 in one pass (upper-bound mode): sorted position pos owns slot
-        // out0 + pos of the row's reserved range; the first position of every run
-        // writes (column, sum) when the sum is != 0, every other slot column -1.
-        const int64_t out0 = out.out0;
-        uint32_t kept = 0;
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            const int pos = (warp * ITEMS + i) * 32 + lane;
-            if (pos < P) {
-                const uint32_t c = col_at(pos);
-                int32_t oc = -1;
-                double acc = 0.0;
-                if (pos == 0 || col_at(pos - 1) != c) {
-                    acc = vals[seq_at(pos)];
-                    for (int q = pos + 1; q < P && col_at(q) == c; ++q) acc = __dadd_rn(acc, vals[seq_at(q)]);
-                    if (acc != 0.0) {
-                        oc = static_cast<int32_t>(c + cmin);
-                        ++kept;
-                    }
-                }
-                out.c_col[out0 + pos] = oc;
-                if (oc >= 0) out.c_val[out0 + pos] = acc;
-            }
-        }
-        kept = __reduce_add_sync(0xffffffffu, kept);
-        if (W == 1) {
+    if constexpr (W == 1 && !PACKED) {
+        if (out.holes) {
+            kept = write_slots_plain(sm.keys, sm.seqs, vals, 0, P, 0, P, out.c_col + out.out0, out.c_val + out.out0, lane);
             if (lane == 0) *out.nz = kept;
-        } else if (lane == 0 && kept) {  // the row's count was zeroed before its enumeration
-            atomicAdd(reinterpret_cast<unsigned long long*>(out.nz), static_cast<unsigned long long>(kept));
+            return lane == 0 ? kept : 0u;
         }
-        return lane == 0 ? kept : 0u;
     }
 
     // 3. runs of equal columns summed in product order; each run's sum is stored
@@ -737,7 +770,7 @@ __device__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, dou
                 double acc = vals[s0];
                 for (int q = pos + 1; q < P && col_at(q) == c; ++q) acc = __dadd_rn(acc, vals[seq_at(q)]);
                 vals[s0] = acc;
-                keep = acc != 0.0;
+                keep = nonzero(acc);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -759,7 +792,7 @@ __device__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITEMS, SV>& sm, dou
             c = col_at(pos);
             if (pos == 0 || col_at(pos - 1) != c) {
                 v = vals[seq_at(pos)];
-                keep = v != 0.0;
+                keep = nonzero(v);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -804,7 +837,6 @@ __device__ uint32_t numeric_row(const Job& J, int row, RowSmem<W, ITEMS, SV>& sm
         // barriers below (a piece's row count was zeroed by the planner)
         if (!PIECE && J.holes && tid == 0) J.nz[row] = 0;
     }
-    if constexpr (kBucketRows<W, ITEMS>) clear_buckets(sm, P, tid);
 
     // 1. products into shared memory
     int32_t lo = INT32_MAX, hi = INT32_MIN;
@@ -831,6 +863,8 @@ __device__ uint32_t numeric_row(const Job& J, int row, RowSmem<W, ITEMS, SV>& sm
                                             [&](int32_t seq, int32_t c, double b, double a) {
                                                 put(seq, c, __dmul_rn(a, b));
                                             });
+    // (the enumeration's barriers come after every warp's last use of the starts)
+    if constexpr (W > 1) clear_buckets(sm, P, tid);
     lo = __reduce_min_sync(0xffffffffu, lo);  // one warp-wide reduction instruction each
     hi = __reduce_max_sync(0xffffffffu, hi);
     if (W > 1) {
@@ -853,8 +887,9 @@ __device__ uint32_t numeric_row(const Job& J, int row, RowSmem<W, ITEMS, SV>& sm
     const uint32_t range = P ? static_cast<uint32_t>(hi - lo) : 0u;
     const int nbits = range ? 32 - __clz(range) : 0;
     const RowOut out{J.c_col, J.c_val, J.cnt[row] + (PIECE ? pc->slot_off : 0), J.nz + row, J.holes, PIECE ? 1 : 0};
-    if (nbits + kSeqBits <= 32) return finish_row<W, ITEMS, SV, true>(out, sm, vals, P, cmin, nbits, lane, warp, tid);
-    return finish_row<W, ITEMS, SV, false>(out, sm, vals, P, cmin, nbits, lane, warp, tid);
+    if constexpr (W == 1)
+        if (range < (0xffffffffu >> kSeqBits)) return finish_row<W, ITEMS, SV, true>(out, sm, vals, P, cmin, range, nbits, lane, warp, tid);
+    return finish_row<W, ITEMS, SV, false>(out, sm, vals, P, cmin, range, nbits, lane, warp, tid);
 }
 
 constexpr int kWarpKernelThreads = 256;

@@ -31,7 +31,7 @@ struct MergeExchange {
                         if ((i + j) / (2 * p) == (i + j + k) / (2 * p)) ++c;
         return c;
     }
-    CePair pair[N > 1 ? 128 : 1] = {};
+    CePair pair[N > 1 ? 256 : 1] = {};
     constexpr MergeExchange() {
         int c = 0;
         for (int p = 1; p < N; p *= 2)
@@ -52,7 +52,7 @@ struct BitonicMerge {
         if (n == 3) c += N;
         return c;
     }
-    CePair pair[N > 1 ? 128 : 1] = {};
+    CePair pair[N > 1 ? 256 : 1] = {};
     constexpr BitonicMerge() {
         int c = 0, n = N;
         for (; n > 1 && n % 2 == 0; n /= 2)
@@ -67,29 +67,29 @@ struct BitonicMerge {
     }
 };
 
-template <int N>
-__device__ __forceinline__ void compare_exchange(uint32_t (&k)[N], int a, int b) {
-    const uint32_t lo = min(k[a], k[b]);
+template <typename K, int N>
+__device__ __forceinline__ void compare_exchange(K (&k)[N], int a, int b) {
+    const K lo = min(k[a], k[b]);
     k[b] = max(k[a], k[b]);
     k[a] = lo;
 }
 
-template <typename Net, int N, int... I>
-__device__ __forceinline__ void run_network(uint32_t (&k)[N], std::integer_sequence<int, I...>) {
+template <typename Net, typename K, int N, int... I>
+__device__ __forceinline__ void run_network(K (&k)[N], std::integer_sequence<int, I...>) {
     constexpr Net net{};
     (compare_exchange(k, std::integral_constant<int, net.pair[I].a>::value, std::integral_constant<int, net.pair[I].b>::value),
      ...);
 }
 
-template <int ITEMS>
-__device__ __forceinline__ void warp_sort(uint32_t (&k)[ITEMS], int lane) {
+template <typename K, int ITEMS>
+__device__ __forceinline__ void warp_sort(K (&k)[ITEMS], int lane) {
     if constexpr (ITEMS > 1)
         run_network<MergeExchange<ITEMS>>(k, std::make_integer_sequence<int, MergeExchange<ITEMS>::count()>{});
 #pragma unroll
     for (int m = 1; m < 32; m *= 2) {  // runs of m lanes into runs of 2m
         {
             const bool low = (lane & m) == 0;
-            uint32_t t[ITEMS];
+            K t[ITEMS];
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) t[i] = __shfl_xor_sync(0xffffffffu, k[ITEMS - 1 - i], 2 * m - 1);
 #pragma unroll
@@ -100,7 +100,7 @@ __device__ __forceinline__ void warp_sort(uint32_t (&k)[ITEMS], int lane) {
             const bool low = (lane & d) == 0;
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) {
-                const uint32_t t = __shfl_xor_sync(0xffffffffu, k[i], d);
+                const K t = __shfl_xor_sync(0xffffffffu, k[i], d);
                 k[i] = low ? min(k[i], t) : max(k[i], t);
             }
         }
