@@ -250,11 +250,13 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     const int njobs = static_cast<int>(in.size());
     std::vector<Job> jobs(njobs);
     std::vector<int64_t> row_base(njobs + 1, 0);
+    int64_t entries = 0;
     for (int j = 0; j < njobs; ++j) {
         check_view(in[j].A, "A");
         check_view(in[j].B, "B");
         require(in[j].A->cols == in[j].B->rows, SPG_INVALID_ARGUMENT, "SpGEMM requires A.cols == B.rows");
         row_base[j + 1] = row_base[j] + in[j].A->rows;
+        entries += in[j].A->nnz;
     }
     const int64_t total_rows = row_base[njobs];
     for (int j = 0; j < njobs; ++j) {
@@ -292,7 +294,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     Ctrl* hc = static_cast<Ctrl*>(h->ctrl);
     int64_t launches = total_rows > 0 ? 3 : 1;
     cudaEventRecord(h->ev[0], st);
-    launch_rowwork(d_jobs, njobs, d_row_base, total_rows, &d_ctrl->stats, &d_ctrl->err, st);
+    launch_rowwork(d_jobs, njobs, d_row_base, total_rows, entries, &d_ctrl->stats, &d_ctrl->err, st);
     launch_bin_offsets(&d_ctrl->stats, d_ctrl->bin_off, st);
     launch_bin_scatter(d_jobs, njobs, d_row_base, total_rows, d_ctrl->bin_off, d_ctrl->cursor, items, st);
     check_cuda(cudaGetLastError(), "K1 launch");
@@ -438,7 +440,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
             final_col = ar.alloc<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
             final_val = ar.alloc<double>(static_cast<size_t>(nz_total), "C val (compact)");
             if (exact) launch_compact(d_jobs, in[0].A->rows, final_col, final_val, st);
-            else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, final_col, final_val, st);
+            else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, final_col, final_val, st);
             check_cuda(cudaGetLastError(), "K5 launch");
             final_rp = nz;
             ar.free_now(c_col);
@@ -495,7 +497,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         if (exact) {
             for (int j = 0; j < njobs; ++j) launch_compact(d_jobs + j, in[j].A->rows, nullptr, nullptr, st);
         } else {
-            launch_compact_holes(d_jobs, njobs, d_row_base, total_rows, nullptr, nullptr, st);
+            launch_compact_holes(d_jobs, njobs, d_row_base, total_rows, products, nullptr, nullptr, st);
         }
         check_cuda(cudaGetLastError(), "K5 launch");
         ar.free_now(c_col);
@@ -925,7 +927,7 @@ spg_status spg_partition_rows(spg_handle* h, const spg_csr_view* A, const spg_cs
         check_cuda(cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st), "memset ctrl");
         check_cuda(cudaMemcpyAsync(d_row_base, rb, sizeof rb, cudaMemcpyHostToDevice, st), "H2D row base");
         check_cuda(cudaMemcpyAsync(d_job, &job, sizeof job, cudaMemcpyHostToDevice, st), "H2D job");
-        launch_rowwork(d_job, 1, d_row_base, m, &d_ctrl->stats, &d_ctrl->err, st);
+        launch_rowwork(d_job, 1, d_row_base, m, A->nnz, &d_ctrl->stats, &d_ctrl->err, st);
         launch_scan(ub, m, partials, st);  // exclusive, ub[m] = all scalar products
         launch_partition(ub, m, parts, d_first, st);
         check_cuda(cudaGetLastError(), "partition launch");
@@ -1319,6 +1321,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     cudaStream_t st = h->stream;
     p->njobs = n;
     p->row_base.assign(n + 1, 0);
+    int64_t entries = 0;
     std::vector<Job> jobs(n);
     for (int j = 0; j < n; ++j) {
         check_view(&A[j], "A");
@@ -1327,6 +1330,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
                 "a plan needs device-resident operands");
         require(A[j].cols == B[j].rows, SPG_INVALID_ARGUMENT, "SpGEMM requires A.cols == B.rows");
         p->row_base[j + 1] = p->row_base[j] + A[j].rows;
+        entries += A[j].nnz;
         p->rows.push_back(A[j].rows);
         p->cols.push_back(B[j].cols);
         auto view = [](const spg_csr_view& m) {
@@ -1367,7 +1371,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
                "H2D");
     check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * n, cudaMemcpyHostToDevice, st), "H2D");
     // structure: row work, bins, the upper-bound offsets
-    launch_rowwork(d_jobs, n, d_row_base, total_rows, &d_ctrl->stats, &d_ctrl->err, st);
+    launch_rowwork(d_jobs, n, d_row_base, total_rows, entries, &d_ctrl->stats, &d_ctrl->err, st);
     launch_bin_offsets(&d_ctrl->stats, d_ctrl->bin_off, st);
     launch_bin_scatter(d_jobs, n, d_row_base, total_rows, d_ctrl->bin_off, d_ctrl->cursor, items, st);
     launch_job_products(d_jobs, n, d_row_base, d_jp, st);
@@ -1432,7 +1436,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
         cudaStreamWaitEvent(st, h->join[i], 0);
     }
     launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
-    launch_compact_holes(d_jobs, n, d_row_base, total_rows, p->col, p->val, st);
+    launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, p->col, p->val, st);
     launch_gather(nz, d_idx, d_starts, n, st);
     launch_rebase_jobs(nz, p->rp, d_row_base, n, max_rows, st);
     launch_readback(d_starts, p->h_starts, sizeof(int64_t) * n, st);

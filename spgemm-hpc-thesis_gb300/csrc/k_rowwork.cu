@@ -7,6 +7,9 @@
 // outside B's row range", spgemm_common.cpp:141-143) and the offsets of every
 // referenced B row.  HBM traffic: A.rp (8 B/row), A.ci (4 B/entry) and one B.rp
 // pair per A entry (16 B/entry).
+#include <algorithm>
+#include <type_traits>
+
 #include "spg_common.cuh"
 
 namespace spg {
@@ -24,12 +27,50 @@ __device__ inline int job_of_row(const int64_t* job_row_base, int njobs, int64_t
     return lo;
 }
 
+// Scalar products of the A entries [p0, a1) that a lane takes every `step` from
+// p0 on, at most U of them, their loads issued together.
+template <int U>
+__device__ __forceinline__ int64_t entry_products(const Job& J, int64_t p0, int64_t a1, int step, ErrWord* err) {
+    int32_t k[U];
+    int64_t s[U], e[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) k[u] = p0 + u * step < a1 ? J.A.ci[p0 + u * step] : 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        s[u] = e[u] = 0;
+        if (p0 + u * step < a1) {
+            if (k[u] < 0 || k[u] >= J.B.rows) {
+                raise_error(err, kErrColumnRange, 1, p0 + u * step);
+            } else {
+                s[u] = J.B.rp[k[u]];
+                e[u] = J.B.rp[k[u] + 1];
+            }
+        }
+    }
+    int64_t len = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (s[u] < 0 || e[u] < s[u] || e[u] > J.B.nnz) raise_error(err, kErrInvalid, 2, k[u]);
+        else len += e[u] - s[u];
+    }
+    return len;
+}
+
+// T lanes per row, 32 / T rows per warp at a time; a row of more than 4 T
+// entries gives the rest to the whole warp, so that a long row among short ones
+// does not keep T lanes busy alone.  Bound by the gathers of B's offsets (and, at
+// one warp per row, by the lanes that a short row leaves idle): see
+// launch_rowwork for the choice of T.  The counters are kept per lane and per
+// CTA: a 64-bit atomic in shared memory is a compare-and-swap loop, and four of
+// them per row took as long as the row.
+template <int T>
 __global__ void __launch_bounds__(kRowworkThreads)
 rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ job_row_base,
                int64_t total_rows, Stats* __restrict__ stats, ErrWord* __restrict__ err) {
-    __shared__ unsigned long long s_bins[kNumBins];
+    constexpr int U = 4, kRows = 32 / T;
+    __shared__ unsigned int s_bins[kNumBins];
     __shared__ unsigned long long s_products, s_max, s_split;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, tl = lane % T;
     if (threadIdx.x < kNumBins) s_bins[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         s_products = 0;
@@ -38,45 +79,61 @@ rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restric
     }
     __syncthreads();
 
-    const int64_t warps = static_cast<int64_t>(gridDim.x) * (kRowworkThreads / 32);
-    for (int64_t g = static_cast<int64_t>(blockIdx.x) * (kRowworkThreads / 32) + (threadIdx.x >> 5);
-         g < total_rows; g += warps) {
-        const int j = job_of_row(job_row_base, njobs, g);
-        const Job& J = jobs[j];
-        const int row = static_cast<int>(g - job_row_base[j]);
-        const int64_t a0 = J.A.rp[row], a1 = J.A.rp[row + 1];
-        bool bad_row = a0 < 0 || a1 < a0 || a1 > J.A.nnz;
-        int64_t len = 0;
-        if (!bad_row) {
-            for (int64_t p = a0 + lane; p < a1; p += 32) {
-                const int32_t k = J.A.ci[p];
-                if (k < 0 || k >= J.B.rows) {
-                    raise_error(err, kErrColumnRange, 1, p);
-                    continue;
-                }
-                const int64_t s = J.B.rp[k], e = J.B.rp[k + 1];
-                if (s < 0 || e < s || e > J.B.nnz) {
-                    raise_error(err, kErrInvalid, 2, k);
-                    continue;
-                }
-                len += e - s;
+    int64_t products = 0, most = 0, split = 0;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * (kRowworkThreads / 32) * kRows;
+    for (int64_t g0 = (static_cast<int64_t>(blockIdx.x) * (kRowworkThreads / 32) + (threadIdx.x >> 5)) * kRows;
+         g0 < total_rows; g0 += stride) {
+        const int64_t g = g0 + lane / T;
+        int j = 0, row = 0;
+        int64_t a0 = 0, a1 = 0, len = 0;
+        if (g < total_rows) {
+            j = job_of_row(job_row_base, njobs, g);
+            row = static_cast<int>(g - job_row_base[j]);
+            a0 = jobs[j].A.rp[row];
+            a1 = jobs[j].A.rp[row + 1];
+            if (a0 < 0 || a1 < a0 || a1 > jobs[j].A.nnz) {
+                if (tl == 0) raise_error(err, kErrInvalid, 3, row);
+                a0 = a1 = 0;
             }
+            len = entry_products<U>(jobs[j], a0 + tl, a1, T, err);
         }
-        len = warp_sum(len);
-        if (lane == 0) {
-            if (bad_row) raise_error(err, kErrInvalid, 3, row);
+        unsigned rest = __ballot_sync(0xffffffffu, tl == 0 && a1 - a0 > U * T);
+        while (rest) {
+            const int src = __ffs(rest) - 1;
+            rest &= rest - 1u;
+            const Job& J = jobs[__shfl_sync(0xffffffffu, j, src)];
+            const int64_t p1 = __shfl_sync(0xffffffffu, a1, src);
+            int64_t more = 0;
+            for (int64_t p = __shfl_sync(0xffffffffu, a0, src) + U * T + lane; p - lane < p1; p += 32 * U)
+                more += entry_products<U>(J, p, p1, 32, err);
+            more = warp_sum(more);
+            if (lane == src) len += more;
+        }
+#pragma unroll
+        for (int o = T / 2; o > 0; o >>= 1) len += __shfl_xor_sync(0xffffffffu, len, o);
+        if (tl == 0 && g < total_rows) {
+            const Job& J = jobs[j];
             if (J.S.rp) len += J.S.rp[row + 1] - J.S.rp[row];
             J.ub[row] = len;
             J.cnt[row] = len;  // upper-bound layout; the exact mode's symbolic phase overwrites it
-            atomicAdd(&s_bins[bin_of(len)], 1ull);
-            atomicAdd(&s_products, static_cast<unsigned long long>(len));
-            atomicMax(&s_max, static_cast<unsigned long long>(len));
-            if (len > kSplitThreshold) atomicAdd(&s_split, static_cast<unsigned long long>(len));
+            atomicAdd(&s_bins[bin_of(len)], 1u);
+            products += len;
+            most = len > most ? len : most;
+            if (len > kSplitThreshold) split += len;
         }
     }
+    products = warp_sum(products);
+    most = warp_max(most);
+    split = warp_sum(split);
+    if (lane == 0 && products) {
+        atomicAdd(&s_products, static_cast<unsigned long long>(products));
+        atomicMax(&s_max, static_cast<unsigned long long>(most));
+        if (split) atomicAdd(&s_split, static_cast<unsigned long long>(split));
+    }
     __syncthreads();
-    if (threadIdx.x < kNumBins && s_bins[threadIdx.x]) atomicAdd(&stats->bin_count[threadIdx.x], s_bins[threadIdx.x]);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < kNumBins && s_bins[threadIdx.x])
+        atomicAdd(&stats->bin_count[threadIdx.x], static_cast<unsigned long long>(s_bins[threadIdx.x]));
+    if (threadIdx.x == 0 && s_products) {
         atomicAdd(&stats->products, s_products);
         atomicMax(&stats->max_ub, s_max);
         if (s_split) atomicAdd(&stats->split_products, s_split);
@@ -230,36 +287,45 @@ compact_kernel(const Job* __restrict__ job, int rows, int32_t* __restrict__ out_
     }
 }
 
-// K5 for rows written with holes (upper-bound mode): warp per row, the row's
-// reserved slots [cnt[r], cnt[r+1]) are read in order and the slots with a
-// column >= 0 are packed at the row's final offset nz[r] (ballot + popc).
-// Each warp loads its next row's offsets while it copies the current one, and
-// issues eight chunks of 32 slots per step (2.70 -> 2.45 ms on the power-law
-// workload, 89% of the measured copy bandwidth; either change alone gave < 2%).
+// K5 for rows written with holes (upper-bound mode): a warp takes `group`
+// consecutive rows, whose reserved slots [cnt[r], cnt[r + group]) are contiguous
+// as their entries in C are: the slots are read in order and those with a column
+// >= 0 packed from the first row's final offset nz[r] on (ballot + popc).  Each
+// warp loads its next group's offsets while it copies the current one, and issues
+// eight chunks of 32 slots per step.  Power-law product: 6.1 TB/s, 89% of the
+// measured copy bandwidth; 262,144 rows of 56 and of 32 slots: 0.068 ms together
+// (0.188 with one row per warp, whose eight chunks were mostly empty).
 __global__ void __launch_bounds__(256)
 compact_holes_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ job_row_base,
-                     int64_t total_rows, int32_t* __restrict__ out_col, double* __restrict__ out_val) {
+                     int64_t total_rows, int group, int32_t* __restrict__ out_col, double* __restrict__ out_val) {
     constexpr int kChunks = 8;
     const int lane = threadIdx.x & 31;
-    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    int64_t g = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5) * group;
+    int64_t g = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * group;
+    int64_t group_end = min(g + group, total_rows);
     int j = 0;
-    int64_t n_src = 0, n_end = 0, n_dst = 0;
-    auto load_row = [&](int64_t row) {
+    int64_t n_src = 0, n_end = 0, n_dst = 0, n_row = 0;
+    auto load_rows = [&](int64_t row) {  // the group's rows from `row` on, of one product
         j = job_of_row(job_row_base, njobs, row);
-        const int r = static_cast<int>(row - job_row_base[j]);
+        n_row = min(group_end, job_row_base[j + 1]);
+        const int r = static_cast<int>(row - job_row_base[j]), r1 = static_cast<int>(n_row - job_row_base[j]);
         n_src = jobs[j].cnt[r];
-        n_end = jobs[j].cnt[r + 1];
+        n_end = jobs[j].cnt[r1];
         n_dst = jobs[j].nz[r] - (out_col ? 0 : jobs[j].nz[0]);  // the job's own arrays start at its first row
     };
-    if (g < total_rows) load_row(g);
-    for (; g < total_rows; g += warps) {
+    if (g < total_rows) load_rows(g);
+    while (g < total_rows) {
         const Job& J = jobs[j];
         int32_t* __restrict__ oc = out_col ? out_col : J.out_col;
         double* __restrict__ ov = out_col ? out_val : J.out_val;
         const int64_t src = n_src, end = n_end;
         int64_t dst = n_dst;
-        if (g + warps < total_rows) load_row(g + warps);
+        g = n_row;
+        if (g >= group_end) {
+            g = group_end - group + stride;  // only the last group is shorter, and no group follows it
+            group_end = min(g + group, total_rows);
+        }
+        if (g < total_rows) load_rows(g);
         // columns and values are loaded together (a hole's value is read and
         // dropped) so the loads do not wait on each other
         for (int64_t q0 = src; q0 < end; q0 += kChunks * 32) {
@@ -350,11 +416,21 @@ int grid_for(int64_t work, int per_block, int cap) {
 
 }  // namespace
 
-void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
+void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows, int64_t entries,
                     Stats* d_stats, ErrWord* d_err, cudaStream_t stream) {
     if (total_rows <= 0) return;
-    const int grid = grid_for(total_rows, kRowworkThreads / 32, 152 * 16);
-    rowwork_kernel<<<grid, kRowworkThreads, 0, stream>>>(d_jobs, njobs, d_job_row_base, total_rows, d_stats, d_err);
+    // Lanes per row.  Measured with 4 / 8 lanes (2 and 32 were slower everywhere;
+    // one warp per row with 64-bit shared atomics before): 65,536 rows of 16
+    // entries 13.3 / 15.8 us (21), power-law rows of 24 on average 244 / 255 us
+    // (323), uneven rows of 34 38 / 35 us (34), R and R*A of the 128^3 Galerkin
+    // chain (8 and 32 entries) 110 / 86 us (143).
+    auto run = [&](auto t) {
+        constexpr int T = decltype(t)::value;
+        rowwork_kernel<T><<<grid_for(total_rows, kRowworkThreads / T, 152 * 8), kRowworkThreads, 0, stream>>>(
+            d_jobs, njobs, d_job_row_base, total_rows, d_stats, d_err);
+    };
+    if (entries / total_rows <= 24) run(std::integral_constant<int, 4>{});
+    else run(std::integral_constant<int, 8>{});
 }
 
 void launch_bin_scatter(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
@@ -391,10 +467,13 @@ void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_va
 }
 
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                          int32_t* out_col, double* out_val, cudaStream_t stream) {
+                          int64_t slots, int32_t* out_col, double* out_val, cudaStream_t stream) {
     if (total_rows <= 0) return;
-    compact_holes_kernel<<<grid_for(total_rows, 8, 152 * 32), 256, 0, stream>>>(d_jobs, njobs, d_job_row_base,
-                                                                              total_rows, out_col, out_val);
+    // Rows per warp: about two steps of 256 slots.
+    const int64_t mean = slots / total_rows + 1;
+    const int group = static_cast<int>(std::min<int64_t>(std::max<int64_t>(512 / mean, 1), 64));
+    compact_holes_kernel<<<grid_for(total_rows, 8 * group, 152 * 32), 256, 0, stream>>>(
+        d_jobs, njobs, d_job_row_base, total_rows, group, out_col, out_val);
 }
 
 void launch_gather(const int64_t* d_src, const int64_t* d_idx, int64_t* d_dst, int n, cudaStream_t stream) {

@@ -168,7 +168,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         (ce = cudaMemcpyAsync(d_row_base, row_base, sizeof row_base, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (ce = cudaMemcpyAsync(d_job, &job, sizeof job, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return from_cuda(ce, "scratch set-up", err, err_len);
-    launch_rowwork(d_job, 1, d_row_base, m, &d_ctrl->stats, &d_ctrl->err, st);
+    launch_rowwork(d_job, 1, d_row_base, m, A->nnz, &d_ctrl->stats, &d_ctrl->err, st);
     launch_bin_offsets(&d_ctrl->stats, d_ctrl->bin_off, st);
     launch_bin_scatter(d_job, 1, d_row_base, m, d_ctrl->bin_off, d_ctrl->cursor, items, st);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "row work launch", err, err_len);

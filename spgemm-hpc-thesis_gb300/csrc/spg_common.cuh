@@ -187,7 +187,8 @@ __host__ __device__ inline int item_row(int64_t it) { return static_cast<int>(it
 
 // K1: products per row (ub), bin histogram, product total and input checks.
 // Rows of all jobs are flattened: job j owns rows [row_base_j, row_base_j + A_j.rows).
-void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
+// entries: stored entries of all A (sets the lanes per row only).
+void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows, int64_t entries,
                     Stats* d_stats, ErrWord* d_err, cudaStream_t stream);
 // K1b: scatter work items into per-bin lists (d_bin_off from the bin histogram).
 void launch_bin_scatter(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
@@ -231,9 +232,10 @@ inline SplitTotals split_totals(const Stats& st) {
 // K5: move rows from C_tmp (offsets job.cnt) to C (offsets job.nz, scanned);
 // with out_col == nullptr, into the job's own arrays (Job::out_col / out_val).
 void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_val, cudaStream_t stream);
-// K5 for rows written with holes: keeps the slots whose column is >= 0.
+// K5 for rows written with holes: keeps the slots (of which there are `slots`)
+// whose column is >= 0.
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                          int32_t* out_col, double* out_val, cudaStream_t stream);
+                          int64_t slots, int32_t* out_col, double* out_val, cudaStream_t stream);
 // Bin list offsets from the bin histogram.
 void launch_bin_offsets(const Stats* d_stats, int64_t* d_bin_off, cudaStream_t stream);
 
