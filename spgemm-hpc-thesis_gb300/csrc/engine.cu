@@ -33,11 +33,11 @@ struct spg_handle {
     std::string err;
     cudaEvent_t ev[6] = {};
     cudaEvent_t bin_ev[kNumBins] = {};  // end of each bin's numeric launch
-    // numeric bins run on three streams (warp bins on `stream`; shared-memory
-    // CTA bins; slab and heavy bins, which share the scratch), so that one
-    // launch's tail overlaps the others; fork/join events
-    cudaStream_t aux[2] = {};
-    cudaEvent_t fork = nullptr, join[2] = {};
+    // streams of the bins beside `stream` (bin_stream), so that one launch's tail
+    // overlaps the others; fork/join events
+    static constexpr int kAux = 7;
+    cudaStream_t aux[kAux] = {};
+    cudaEvent_t fork = nullptr, join[kAux] = {};
     bool serial_bins = false;  // spg_tune times bins one after the other
     bool one_bin_stream = false;  // spg_config.bin_streams == 1
     spg_timings last{};
@@ -241,6 +241,95 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
     return ms;
 }
 
+// Products up to which a call's bins each get a stream of their own: below, a
+// bin does not fill the GPU and its launch takes the time of its slowest row,
+// which the others need not wait for; above, three streams (warp bins; CTA bins
+// up to 8192 products, whose slabs then share memory; rows above 8192 products)
+// fill it.  K4 on three streams / one per bin: 1.1 M products in 11 bins 102 /
+// 62 us, 8.3 M in 8 bins of warp rows 178 / 126 us, 56 M in 19 bins 0.90 / 0.92-1.0
+// ms, 595 M 10.72 / 10.80 ms.
+constexpr int64_t kSpreadProducts = int64_t{1} << 25;
+
+// The streams of one call's bins: forked from and joined back into the handle's.
+struct BinStreams {
+    spg_handle* h;
+    BinOrder order;
+    bool used[spg_handle::kAux] = {};
+    int next = 0;
+
+    BinStreams(spg_handle* handle, int64_t products) : h(handle) {
+        order = h->serial_bins || h->one_bin_stream ? BinOrder::kSerial
+                : products <= kSpreadProducts       ? BinOrder::kSpread
+                                                    : BinOrder::kThreeStreams;
+    }
+    // On several streams each starts with its largest rows; on one (server lanes,
+    // the tuner) the bins go from the smallest rows up (measured faster for
+    // overlapping server lanes).
+    template <typename F>
+    void for_each_bin(F&& f) const {
+        for (int i = 1; i < kNumBins; ++i) f(order == BinOrder::kSerial ? i : kNumBins - i);
+    }
+    void begin() {
+        std::fill(used, used + spg_handle::kAux, false);
+        next = 0;
+        if (order != BinOrder::kSerial) cudaEventRecord(h->fork, h->stream);
+    }
+    cudaStream_t aux(int i) {
+        if (!used[i]) cudaStreamWaitEvent(h->aux[i], h->fork, 0);
+        used[i] = true;
+        return h->aux[i];
+    }
+    // The stream of bin b's launch (called once per launch, in launch order).
+    // The rows above 8192 products share scratch: always one stream.
+    cudaStream_t of(int b) {
+        if (order == BinOrder::kSerial) return h->stream;
+        if (b > kLastSmemBin) return aux(1);
+        if (order == BinOrder::kThreeStreams) return b <= kLastWarpBin ? h->stream : aux(0);
+        const int i = next++ % spg_handle::kAux;
+        return i == 1 ? h->stream : aux(i);
+    }
+    void end() {
+        for (int i = 0; i < spg_handle::kAux; ++i) {
+            if (!used[i]) continue;
+            cudaEventRecord(h->join[i], h->aux[i]);
+            cudaStreamWaitEvent(h->stream, h->join[i], 0);
+        }
+    }
+};
+
+// K4 of every bin.  In the upper-bound layout the rows of neighbouring bins
+// 17-19 are split in one launch (apart for the tuner, which times each bin).
+// Returns the kernels launched.
+int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, const int64_t* bin_count,
+                    const int64_t* bin_off, int64_t max_ub, const SplitTotals& split, void* scratch,
+                    const NumericScratch& ns, Ctrl* d_ctrl, bool holes, bool timed) {
+    spg_handle* h = bs.h;
+    int64_t launches = 0;
+    bs.begin();
+    bool done[kNumBins] = {};
+    bs.for_each_bin([&](int b) {
+        if (done[b] || !bin_count[b]) return;
+        cudaStream_t st = bs.of(b);
+        int first = b;
+        int64_t count = bin_count[b];
+        const bool split_rows = holes && b > kLastSmemBin && !(b < kBinHeavy && h->bin_variant[b]);
+        if (split_rows && bs.order != BinOrder::kSerial)  // the bins below join: their items precede b's
+            while (first - 1 > kLastSmemBin && !h->bin_variant[first - 1]) {
+                --first;
+                count += bin_count[first];
+                done[first] = true;
+            }
+        launch_numeric(b, d_jobs, items + bin_off[first], count, max_ub, split, scratch,
+                       static_cast<unsigned char*>(scratch) + ns.slab[b], &d_ctrl->stats, &d_ctrl->err, st, h->num_sms,
+                       holes, h->bin_variant[b]);
+        launches += split_rows ? 3 : 1;  // planner, pieces, global-slab rows
+        if (timed)
+            for (int i = first; i <= b; ++i) cudaEventRecord(h->bin_ev[i], st);
+    });
+    bs.end();
+    return launches;
+}
+
 // The phase pipeline for one or more products.  Results stay on the device.
 // products_out (optional) receives the scalar products of every product.
 void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
@@ -340,44 +429,24 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     // symbolic phase counts the distinct columns of every row first.
     const SplitTotals split = split_totals(hc->stats);
     const bool exact = use_exact_mode(h, products + split.products, ar.bytes());
-    size_t scratch_bytes = numeric_scratch_bytes(bin_count, max_ub, split, h->num_sms, !exact);
+    // K2 and K4 run their bins on several streams (BinStreams)
+    BinStreams streams(h, products);
+    const NumericScratch ns = numeric_scratch(bin_count, max_ub, split, h->num_sms, !exact, streams.order);
+    size_t scratch_bytes = ns.bytes;
     if (exact) scratch_bytes = std::max(scratch_bytes, symbolic_scratch_bytes(bin_count, max_ub, h->num_sms));
-    void* scratch = scratch_bytes ? ar.alloc<unsigned char>(scratch_bytes, "heavy scratch") : nullptr;
+    void* scratch = scratch_bytes ? ar.alloc<unsigned char>(scratch_bytes, "numeric scratch") : nullptr;
     int64_t* partials = ar.alloc<int64_t>(scan_partials_count(static_cast<int64_t>(slots)), "scan partials");
-    // K2 and K4 per bin; in the upper-bound layout the split rows take three
-    // K4 launches (planner, pieces, global-slab rows)
-    for (int b = 1; b < kNumBins; ++b) launches += bin_count[b] > 0 ? (exact ? 2 : (b > kLastSmemBin ? 3 : 1)) : 0;
     launches += 3;  // scan
     int64_t tmp_total = products;
-    // The bins of K2 and K4 run on three streams (warp bins; shared-memory CTA
-    // bins; slab and heavy bins, which share the scratch), forked from and
-    // joined back into the main stream, so that the tail of one launch overlaps
-    // the others.  On one stream (server lanes, the tuner) they run in order.
-    const bool one_stream = h->serial_bins || h->one_bin_stream;
-    auto stream_of = [&](int b) {
-        if (one_stream) return st;
-        return b <= kLastWarpBin ? st : (b <= kLastSmemBin ? h->aux[0] : h->aux[1]);
-    };
-    auto fork = [&] {
-        if (one_stream) return;
-        cudaEventRecord(h->fork, st);
-        for (cudaStream_t a : h->aux) cudaStreamWaitEvent(a, h->fork, 0);
-    };
-    auto join = [&] {
-        if (one_stream) return;
-        for (int i = 0; i < 2; ++i) {
-            cudaEventRecord(h->join[i], h->aux[i]);
-            cudaStreamWaitEvent(st, h->join[i], 0);
-        }
-    };
     if (exact) {
-        fork();
-        for (int i = 1; i < kNumBins; ++i) {
-            const int b = one_stream ? i : kNumBins - i;
+        streams.begin();
+        streams.for_each_bin([&](int b) {
+            if (!bin_count[b]) return;
             launch_symbolic(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, scratch, scratch_bytes,
-                            &d_ctrl->stats, &d_ctrl->err, stream_of(b), h->num_sms);
-        }
-        join();
+                            &d_ctrl->stats, &d_ctrl->err, streams.of(b), h->num_sms);
+            ++launches;
+        });
+        streams.end();
         check_cuda(cudaGetLastError(), "K2 launch");
     }
     cudaEventRecord(h->ev[2], st);
@@ -406,18 +475,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         jobs[j].holes = exact ? 0 : 1;
     }
     check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D jobs");
-    fork();
-    // on three streams each stream starts with its largest rows; on one stream the
-    // bins go from the smallest rows up (measured faster for overlapping server lanes)
-    for (int i = 1; i < kNumBins; ++i) {
-        const int b = one_stream ? i : kNumBins - i;
-        if (!bin_count[b]) continue;
-        cudaStream_t bs = stream_of(b);
-        launch_numeric(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, split, scratch, scratch_bytes,
-                       &d_ctrl->stats, &d_ctrl->err, bs, h->num_sms, !exact, h->bin_variant[b]);
-        cudaEventRecord(h->bin_ev[b], bs);
-    }
-    join();
+    launches += launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, !exact, true);
     check_cuda(cudaGetLastError(), "K4 launch");
     cudaEventRecord(h->ev[4], st);
     launch_readback(d_ctrl, hc, sizeof(Ctrl), st);
@@ -527,13 +585,12 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     // per-bin times: launch to launch when the bins ran in sequence (spg_tune),
     // else the time from the fork to the end of each bin
     cudaEvent_t prev = h->ev[3];
-    for (int i = 1; i < kNumBins; ++i) {
-        const int b = one_stream ? i : kNumBins - i;
+    streams.for_each_bin([&](int b) {
         h->last.ms_numeric_bin[b] = 0.0f;
-        if (!bin_count[b]) continue;
+        if (!bin_count[b]) return;
         h->last.ms_numeric_bin[b] = elapsed(prev, h->bin_ev[b]);
-        if (one_stream) prev = h->bin_ev[b];
-    }
+        if (streams.order == BinOrder::kSerial) prev = h->bin_ev[b];
+    });
     h->last.ms_numeric_bin[kBinEmpty] = 0.0f;
     h->last.products = products;
     h->last.nnz = nz_total;
@@ -678,7 +735,7 @@ void spg_destroy(spg_handle* h) {
         cudaStreamSynchronize(a);
         cudaStreamDestroy(a);
     }
-    cudaEventDestroy(h->fork);
+    if (h->fork) cudaEventDestroy(h->fork);
     for (auto e : h->join) cudaEventDestroy(e);
     cudaStreamDestroy(h->stream);
     cudaFreeHost(h->ctrl);
@@ -1404,8 +1461,9 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     }
     check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * n, cudaMemcpyHostToDevice, st), "H2D");
     const SplitTotals split = split_totals(p->hc->stats);
-    const size_t scratch_bytes = numeric_scratch_bytes(bin_count, max_ub, split, h->num_sms, true);
-    void* scratch = scratch_bytes ? plan_alloc<unsigned char>(p, scratch_bytes, "plan scratch") : nullptr;
+    BinStreams streams(h, products);
+    const NumericScratch ns = numeric_scratch(bin_count, max_ub, split, h->num_sms, true, streams.order);
+    void* scratch = ns.bytes ? plan_alloc<unsigned char>(p, ns.bytes, "plan scratch") : nullptr;
     p->col = plan_alloc<int32_t>(p, static_cast<size_t>(products), "plan C col");
     p->val = plan_alloc<double>(p, static_cast<size_t>(products), "plan C val");
     p->rp = plan_alloc<int64_t>(p, slots, "plan C row_ptr");
@@ -1422,19 +1480,8 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed), "begin capture");
     cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st);
     cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st);
-    // the bins on three streams, as in run_products (the fork/join is part of the graph)
-    cudaEventRecord(h->fork, st);
-    for (cudaStream_t a : h->aux) cudaStreamWaitEvent(a, h->fork, 0);
-    for (int b = kNumBins - 1; b >= 1; --b)
-        if (bin_count[b])
-            launch_numeric(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, split, scratch, scratch_bytes,
-                           &d_ctrl->stats, &d_ctrl->err,
-                           b <= kLastWarpBin ? st : (b <= kLastSmemBin ? h->aux[0] : h->aux[1]), h->num_sms, true,
-                           h->bin_variant[b]);
-    for (int i = 0; i < 2; ++i) {
-        cudaEventRecord(h->join[i], h->aux[i]);
-        cudaStreamWaitEvent(st, h->join[i], 0);
-    }
+    // (the bins' fork and join are part of the graph)
+    launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, true, false);
     launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
     launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, p->col, p->val, st);
     launch_gather(nz, d_idx, d_starts, n, st);

@@ -444,8 +444,8 @@ constexpr int64_t slab_cap(int bin) { return bin == 17 ? 16 * 32 * 24 : 16 * 32 
 //   4096: 8x16, 3 CTAs, slab 0.65, 4 CTAs 0.74; 16x8, 2 CTAs 0.81
 //   6144: 16x12, 2 CTAs, slab 0.74, 3 CTAs 0.76; 8x24, 3 CTAs 0.86
 //   8192: 16x16, 1 CTA 0.41, 2 CTAs with a slab 0.43
-// The slabs of these bins share one region: the bins run one after the other
-// on one stream.
+// The slabs of these bins share one region where the bins run one after the
+// other on one stream (numeric_scratch).
 constexpr int kB10W = 4, kB10I = 8, kB10MinB = 8;
 constexpr bool kB10SV = true;
 constexpr int kB11W = 4, kB11I = 12, kB11MinB = 8;
@@ -480,35 +480,30 @@ size_t cta_slab_bytes(int bin, int64_t count, int num_sms) {
 
 }  // namespace
 
-size_t numeric_scratch_bytes(const int64_t* bin_count, int64_t max_ub, const SplitTotals& split, int num_sms,
-                             bool holes, bool concurrent) {
-    // Bins 17-19 share the front of the scratch (they run one after the other);
-    // bins 10, 11 and 13-16 take their slabs from its end (also one after the
-    // other), after that region when the two groups run on concurrent streams.
-    size_t cta = 0;
-    for (int b = 10; b <= 16; ++b) cta = std::max(cta, cta_slab_bytes(b, bin_count[b], num_sms));
-    size_t need = 0;
+NumericScratch numeric_scratch(const int64_t* bin_count, int64_t max_ub, const SplitTotals& split, int num_sms,
+                               bool holes, BinOrder order) {
+    NumericScratch ns;
+    size_t front = 0;
+    // bins 17 and 18 as whole rows (in the upper-bound layout where the autotuner
+    // chose it): these launches run one after the other on one stream
+    for (int b = kLastSmemBin + 1; b < kBinHeavy; ++b)
+        if (bin_count[b])
+            front = std::max(front, static_cast<size_t>(slab_grid(bin_count[b], num_sms)) * slab_cap(b) * sizeof(double));
     if (holes) {
-        if (split.rows > 0) need = split_layout(max_ub, split, num_sms).bytes;
-        // bins 17 and 18 run whole where the autotuner chose it (same region:
-        // these launches run one after the other on one stream)
-        for (int b = kLastSmemBin + 1; b < kBinHeavy; ++b)
-            if (bin_count[b])
-                need = std::max(need, static_cast<size_t>(slab_grid(bin_count[b], num_sms)) * slab_cap(b) * sizeof(double));
-    } else {
-        for (int b = kLastSmemBin + 1; b < kBinHeavy; ++b)  // the launches run one after the other
-            if (bin_count[b])
-                need = std::max(need, static_cast<size_t>(slab_grid(bin_count[b], num_sms)) * slab_cap(b) * sizeof(double));
-        const int64_t heavy = bin_count[kBinHeavy];
-        if (heavy)
-            need = std::max(need, static_cast<size_t>(heavy_grid(heavy, num_sms)) * 24 * static_cast<size_t>(max_ub));
+        if (split.rows > 0) front = std::max(front, split_layout(max_ub, split, num_sms).bytes);
+    } else if (bin_count[kBinHeavy]) {
+        front = std::max(front, static_cast<size_t>(heavy_grid(bin_count[kBinHeavy], num_sms)) * 24 * static_cast<size_t>(max_ub));
     }
-    return concurrent ? ((need + 255) & ~size_t{255}) + cta : std::max(need, cta);
-}
-
-// The last `need` bytes of the scratch (nullptr when none are needed).
-static double* tail_slab(void* d_scratch, size_t scratch_bytes, size_t need) {
-    return need ? reinterpret_cast<double*>(static_cast<unsigned char*>(d_scratch) + (scratch_bytes - need)) : nullptr;
+    auto up = [](size_t x) { return (x + 255) & ~size_t{255}; };
+    size_t at = order == BinOrder::kSerial ? 0 : up(front);
+    ns.bytes = std::max(front, at);
+    for (int b = 10; b <= kLastSmemBin; ++b) {
+        const size_t bytes = cta_slab_bytes(b, bin_count[b], num_sms);
+        ns.slab[b] = at;
+        ns.bytes = std::max(ns.bytes, at + bytes);
+        if (order == BinOrder::kSpread) at = up(at + bytes);
+    }
+    return ns;
 }
 
 // Rows of more than kSplitThreshold products in upper-bound mode: plan and
@@ -534,7 +529,7 @@ static void launch_split(int bin, const Job* d_jobs, const int64_t* d_items, int
     const int smem = static_cast<int>(sizeof(PieceSm));
     auto kern = num_piece_kernel<kPieceW, kPieceItems, kPieceMinB>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    // the bin's own queue: bins 17-19 each plan and run their pieces, one after the other
+    // the bin's own queue: where bins 17-19 run apart, they run one after the other
     kern<<<num_sms * kPieceMinB, kPieceW * 32, smem, st>>>(d_jobs, plan, d_stats, d_err, static_cast<double*>(slabs),
                                                           &d_stats->ticket[bin]);
     num_heavy_kernel<<<heavy_grid(count, num_sms), kHeavyThreads, 0, st>>>(
@@ -542,7 +537,7 @@ static void launch_split(int bin, const Job* d_jobs, const int64_t* d_items, int
 }
 
 void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
-                    const SplitTotals& split, void* d_scratch, size_t scratch_bytes, Stats* d_stats, ErrWord* d_err,
+                    const SplitTotals& split, void* d_scratch, void* d_slab, Stats* d_stats, ErrWord* d_err,
                     cudaStream_t st, int num_sms, bool holes, int variant) {
     if (count <= 0) return;
     if (variant == 1 && launch_numeric_alt(bin, d_jobs, d_items, count, d_stats, d_err, st, num_sms)) return;
@@ -559,37 +554,23 @@ void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t 
         launch_split(bin, d_jobs, d_items, count, max_ub, split, d_scratch, d_stats, d_err, st, num_sms);
         return;
     }
-    double* slab = static_cast<double*>(d_scratch);
+    double* const front = static_cast<double*>(d_scratch);
+    double* const slab = static_cast<double*>(d_slab);
     unsigned long long* const tk = &d_stats->ticket[bin];  // the bin's row queue
+    auto run = [&](auto kernel_launch, double* values) {
+        kernel_launch(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk, values);
+    };
     switch (bin) {
-        case 9: run_block<3, 8, 10>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk); break;     // <= 768
-        case 10:  // <= 1024
-            run_block<kB10W, kB10I, kB10MinB, kB10SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
-                                                     tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(10, count, num_sms)));
-            break;
-        case 11:  // <= 1536
-            run_block<kB11W, kB11I, kB11MinB, kB11SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
-                                                     tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(11, count, num_sms)));
-            break;
-        case 12: run_block<8, 8, 4>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk); break;    // <= 2048
-        case 13:  // <= 3072
-            run_block<kB13W, kB13I, kB13MinB, kB13SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
-                                                     tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(13, count, num_sms)));
-            break;
-        case 14:  // <= 4096
-            run_block<kB14W, kB14I, kB14MinB, kB14SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
-                                                     tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(14, count, num_sms)));
-            break;
-        case 15:  // <= 6144
-            run_block<kB15W, kB15I, kB15MinB, kB15SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
-                                                     tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(15, count, num_sms)));
-            break;
-        case 16:  // <= 8192
-            run_block<kB16W, kB16I, kB16MinB, kB16SV>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk,
-                                                     tail_slab(d_scratch, scratch_bytes, cta_slab_bytes(16, count, num_sms)));
-            break;
-        case 17: run_block<16, 24, 1, false>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk, slab); break;
-        case 18: run_block<16, 32, 1, false>(d_jobs, d_items, count, d_stats, d_err, st, num_sms, tk, slab); break;
+        case 9: run(run_block<3, 8, 10, true>, nullptr); break;                     // <= 768
+        case 10: run(run_block<kB10W, kB10I, kB10MinB, kB10SV>, slab); break;       // <= 1024
+        case 11: run(run_block<kB11W, kB11I, kB11MinB, kB11SV>, slab); break;       // <= 1536
+        case 12: run(run_block<8, 8, 4, true>, nullptr); break;                     // <= 2048
+        case 13: run(run_block<kB13W, kB13I, kB13MinB, kB13SV>, slab); break;       // <= 3072
+        case 14: run(run_block<kB14W, kB14I, kB14MinB, kB14SV>, slab); break;       // <= 4096
+        case 15: run(run_block<kB15W, kB15I, kB15MinB, kB15SV>, slab); break;       // <= 6144
+        case 16: run(run_block<kB16W, kB16I, kB16MinB, kB16SV>, slab); break;       // <= 8192
+        case 17: run(run_block<16, 24, 1, false>, front); break;
+        case 18: run(run_block<16, 32, 1, false>, front); break;
         case kBinHeavy:  // exact layout (the upper-bound layout splits these rows)
             num_heavy_kernel<<<heavy_grid(count, num_sms), kHeavyThreads, 0, st>>>(
                 d_jobs, d_items, count, d_scratch, max_ub, d_stats, d_err, nullptr);

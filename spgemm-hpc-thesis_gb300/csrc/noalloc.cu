@@ -181,8 +181,8 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         return ret(SPG_OVERFLOW, "an output row has more than 2^30 scalar products", err, err_len);
     int64_t bin_count[kNumBins];
     for (int b = 0; b < kNumBins; ++b) bin_count[b] = static_cast<int64_t>(hc.stats.bin_count[b]);
-    const size_t slab = std::max(symbolic_scratch_bytes(bin_count, max_ub, num_sms),
-                                 numeric_scratch_bytes(bin_count, max_ub, SplitTotals{}, num_sms, false, false));
+    const NumericScratch ns = numeric_scratch(bin_count, max_ub, SplitTotals{}, num_sms, false, BinOrder::kSerial);
+    const size_t slab = std::max(symbolic_scratch_bytes(bin_count, max_ub, num_sms), ns.bytes);
     unsigned char* d_slab = slab ? cv.take<unsigned char>(slab) : nullptr;
     if (!cv.fits())
         return ret(SPG_BUDGET_EXCEEDED, "heavy rows need more than the 32 MiB allocation-free scratch", err, err_len);
@@ -206,7 +206,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         return from_cuda(ce, "job update", err, err_len);
     for (int b = 1; b < kNumBins; ++b)
         launch_numeric(b, d_job, items + hc.bin_off[b], static_cast<int64_t>(hc.stats.bin_count[b]), max_ub, SplitTotals{}, d_slab,
-                       slab, &d_ctrl->stats, &d_ctrl->err, st, num_sms, false);
+                       d_slab + ns.slab[b], &d_ctrl->stats, &d_ctrl->err, st, num_sms, false);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "numeric launch", err, err_len);
     if ((ce = cudaMemcpyAsync(&hc, d_ctrl, sizeof hc, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (ce = cudaStreamSynchronize(st)) != cudaSuccess)

@@ -207,10 +207,12 @@ size_t scan_partials_count(int64_t n);
 // holes: upper-bound layout (rows above kSplitThreshold products are then
 // split into column-range pieces; in the exact layout they keep their CTA
 // kernels and the global-slab sort).  split: the call's totals of those rows
-// (they size the staging of split rows).  variant: 0 the default team shape of
-// the bin, 1 its alternative (where the bin has one; see launch_numeric_alt).
+// (they size the staging of split rows; one launch may take the rows of all of
+// bins 17-19).  d_scratch and d_slab: the call's numeric scratch and the bin's
+// slab in it (numeric_scratch).  variant: 0 the default team shape of the bin,
+// 1 its alternative (where the bin has one; see launch_numeric_alt).
 void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
-                    const SplitTotals& split, void* d_scratch, size_t scratch_bytes, Stats* d_stats, ErrWord* d_err,
+                    const SplitTotals& split, void* d_scratch, void* d_slab, Stats* d_stats, ErrWord* d_err,
                     cudaStream_t stream, int num_sms, bool holes, int variant = 0);
 // The alternative shape of a bin; false if the bin has none.
 bool launch_numeric_alt(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, Stats* d_stats,
@@ -219,11 +221,20 @@ constexpr int kNumVariants = 2;
 // K4 for the warp-per-row bins (1..kLastWarpBin), compiled separately.
 void launch_numeric_warp(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, Stats* d_stats,
                          ErrWord* d_err, cudaStream_t stream, int num_sms);
-// Global scratch of the numeric phase: value slabs of the CTA bins, and for
-// the rows above 8192 products the staging and pieces of split rows (upper-
-// bound layout) or the slabs of their CTA kernels and global-slab sort.
-size_t numeric_scratch_bytes(const int64_t* bin_count, int64_t max_ub, const SplitTotals& split, int num_sms,
-                             bool holes, bool concurrent = true);
+// How the bins of one call run beside one another, which is what their scratch
+// may share: one after the other; the bins above 8192 products beside the
+// others; every bin beside every other (bins 17-19 excepted).
+enum class BinOrder { kSerial, kThreeStreams, kSpread };
+// Global scratch of the numeric phase: at its front, for the rows above 8192
+// products, the staging and pieces of split rows (upper-bound layout) or the
+// slabs of their CTA kernels and global-slab sort; then the value slabs of the
+// CTA bins (byte offsets).
+struct NumericScratch {
+    size_t bytes = 0;
+    size_t slab[kNumBins] = {};
+};
+NumericScratch numeric_scratch(const int64_t* bin_count, int64_t max_ub, const SplitTotals& split, int num_sms,
+                               bool holes, BinOrder order);
 // Totals of the split rows from the row-work statistics.
 inline SplitTotals split_totals(const Stats& st) {
     return SplitTotals{static_cast<int64_t>(st.split_products),
