@@ -1211,8 +1211,13 @@ spg_status spg_transpose(spg_handle* h, const spg_csr_view* A, int32_t out_locat
         r.ci = ar.alloc<int32_t>(static_cast<size_t>(A->nnz), "transpose col");
         r.v = ar.alloc<double>(static_cast<size_t>(A->nnz), "transpose val");
         void* scratch = ar.alloc<unsigned char>(transpose_scratch_bytes(A->nnz, A->cols), "transpose scratch");
-        launch_transpose(a.rp, a.ci, a.v, A->rows, A->cols, A->nnz, r.rp, r.ci, r.v, scratch, st);
-        check_cuda(cudaGetLastError(), "transpose launch");
+        check_cuda(cudaEventRecord(h->fork, st), "event");
+        check_cuda(cudaStreamWaitEvent(h->aux[0], h->fork, 0), "stream wait");
+        launch_transpose(a.rp, a.ci, a.v, A->rows, A->cols, A->nnz, r.rp, r.ci, r.v, scratch, st, h->aux[0]);
+        const cudaError_t launched = cudaGetLastError();
+        cudaEventRecord(h->join[0], h->aux[0]);
+        cudaStreamWaitEvent(st, h->join[0], 0);
+        check_cuda(launched, "transpose launch");
         ar.release(r.rp);
         ar.release(r.ci);
         ar.release(r.v);

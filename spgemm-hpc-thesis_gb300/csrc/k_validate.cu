@@ -18,6 +18,8 @@
 // products in stored order into an open-addressing table of its own (global
 // memory, 2^ceil(log2(2 ub)) cells), exactly as buildFullRow (:695-717) fills
 // its hash map; then the row of C is merged against the table.
+#include <algorithm>
+
 #include "spg_common.cuh"
 
 namespace spg {
@@ -246,6 +248,29 @@ __global__ void validate_csr_kernel(CsrView M, int ordered, int finite, int* __r
     }
 }
 
+// The same without the checks inside rows: offsets by row, columns by entry in
+// one flat pass (offsets that pass cover every entry).  A thread that walks a
+// row's entries reads them alone: 12.4 M entries 250 -> 19 us.
+__global__ void __launch_bounds__(256)
+validate_flat_kernel(CsrView M, int* __restrict__ flag) {
+    constexpr int U = 8;
+    const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    bool bad = false;
+    for (int64_t r = t; r < M.rows; r += threads) {
+        const int64_t first = M.rp[r], end = M.rp[r + 1];
+        bad |= (r == 0 && first != 0) || (r == M.rows - 1 && end != M.nnz) || first < 0 || end < first || end > M.nnz;
+    }
+    for (int64_t p = t; p < M.nnz; p += U * threads) {
+        int32_t c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) c[u] = p + u * threads < M.nnz ? M.ci[p + u * threads] : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) bad |= p + u * threads < M.nnz && (c[u] < 0 || c[u] >= M.cols);
+    }
+    if (bad) *flag = 1;
+}
+
 int grid_rows(int64_t rows, int threads) {
     const int64_t g = (rows + threads - 1) / threads;
     return static_cast<int>(g < 1 ? 1 : (g > 152 * 32 ? 152 * 32 : g));
@@ -258,6 +283,10 @@ int validate_hist_buckets() { return kHistBuckets; }
 
 void launch_validate_csr(const CsrView& M, bool ordered, int* d_flag, cudaStream_t st, bool finite) {
     if (M.rows <= 0) return;
+    if (!ordered && !finite) {
+        validate_flat_kernel<<<grid_rows(std::max<int64_t>(M.nnz / 8, M.rows), 256), 256, 0, st>>>(M, d_flag);
+        return;
+    }
     validate_csr_kernel<<<grid_rows(M.rows, 128), 128, 0, st>>>(M, ordered ? 1 : 0, finite ? 1 : 0, d_flag);
 }
 
