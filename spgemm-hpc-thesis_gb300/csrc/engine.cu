@@ -192,7 +192,6 @@ struct DevResult {
 struct Ctrl {  // layout of the pinned control block and its device twin
     Stats stats;
     ErrWord err;
-    int64_t bin_off[kNumBins + 1];
     unsigned long long cursor[kNumBins];
     int64_t totals[2];  // scanned totals (symbolic, numeric)
 };
@@ -381,11 +380,10 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D jobs");
 
     Ctrl* hc = static_cast<Ctrl*>(h->ctrl);
-    int64_t launches = total_rows > 0 ? 3 : 1;
+    int64_t launches = total_rows > 0 ? 2 : 0;  // K1, K1b
     cudaEventRecord(h->ev[0], st);
     launch_rowwork(d_jobs, njobs, d_row_base, total_rows, entries, &d_ctrl->stats, &d_ctrl->err, st);
-    launch_bin_offsets(&d_ctrl->stats, d_ctrl->bin_off, st);
-    launch_bin_scatter(d_jobs, njobs, d_row_base, total_rows, d_ctrl->bin_off, d_ctrl->cursor, items, st);
+    launch_bin_scatter(d_jobs, njobs, d_row_base, total_rows, &d_ctrl->stats, d_ctrl->cursor, items, st);
     check_cuda(cudaGetLastError(), "K1 launch");
     cudaEventRecord(h->ev[1], st);
     std::vector<int64_t> job_products(njobs, 0);
@@ -420,8 +418,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     require(max_ub < (int64_t{1} << 30), SPG_OVERFLOW,
             "an output row has more than 2^30 scalar products (engine limit)");
     int64_t bin_count[kNumBins], bin_off[kNumBins + 1];
-    for (int b = 0; b < kNumBins; ++b) bin_count[b] = static_cast<int64_t>(hc->stats.bin_count[b]);
-    for (int b = 0; b <= kNumBins; ++b) bin_off[b] = hc->bin_off[b];
+    bin_lists(hc->stats, bin_count, bin_off);
 
     // Output layout: in the upper-bound mode every row is written at the prefix
     // of its product count (ub) and compacted afterwards, and the products of
@@ -436,7 +433,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     if (exact) scratch_bytes = std::max(scratch_bytes, symbolic_scratch_bytes(bin_count, max_ub, h->num_sms));
     void* scratch = scratch_bytes ? ar.alloc<unsigned char>(scratch_bytes, "numeric scratch") : nullptr;
     int64_t* partials = ar.alloc<int64_t>(scan_partials_count(static_cast<int64_t>(slots)), "scan partials");
-    launches += 3;  // scan
+    launches += scan_launches(static_cast<int64_t>(slots) - 1);
     int64_t tmp_total = products;
     if (exact) {
         streams.begin();
@@ -494,7 +491,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         double* final_val = c_val;
         if (nz_total != tmp_total) {  // rows with fewer entries than reserved: compact
             launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
-            launches += 4;
+            launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
             final_col = ar.alloc<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
             final_val = ar.alloc<double>(static_cast<size_t>(nz_total), "C val (compact)");
             if (exact) launch_compact(d_jobs, in[0].A->rows, final_col, final_val, st);
@@ -530,7 +527,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         launch_gather(nz, d_idx, d_starts, njobs, st);
         int64_t* h_starts = static_cast<int64_t*>(host_staging(h, sizeof(int64_t) * njobs));
         launch_readback(d_starts, h_starts, sizeof(int64_t) * njobs, st);
-        launches += 5;
+        launches += scan_launches(static_cast<int64_t>(slots) - 1) + 2;
         sync(h);  // every product's first offset: the sizes of its arrays
         std::vector<int64_t> starts(h_starts, h_starts + njobs);
         starts.push_back(nz_total);
@@ -1434,8 +1431,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * n, cudaMemcpyHostToDevice, st), "H2D");
     // structure: row work, bins, the upper-bound offsets
     launch_rowwork(d_jobs, n, d_row_base, total_rows, entries, &d_ctrl->stats, &d_ctrl->err, st);
-    launch_bin_offsets(&d_ctrl->stats, d_ctrl->bin_off, st);
-    launch_bin_scatter(d_jobs, n, d_row_base, total_rows, d_ctrl->bin_off, d_ctrl->cursor, items, st);
+    launch_bin_scatter(d_jobs, n, d_row_base, total_rows, &d_ctrl->stats, d_ctrl->cursor, items, st);
     launch_job_products(d_jobs, n, d_row_base, d_jp, st);
     int64_t* partials = plan_alloc<int64_t>(p, scan_partials_count(static_cast<int64_t>(slots)), "plan partials");
     launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
@@ -1453,8 +1449,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     const int64_t max_ub = static_cast<int64_t>(p->hc->stats.max_ub);
     require(max_ub < (int64_t{1} << 30), SPG_OVERFLOW, "an output row has more than 2^30 scalar products (engine limit)");
     int64_t bin_count[kNumBins], bin_off[kNumBins + 1];
-    for (int b = 0; b < kNumBins; ++b) bin_count[b] = static_cast<int64_t>(p->hc->stats.bin_count[b]);
-    for (int b = 0; b <= kNumBins; ++b) bin_off[b] = p->hc->bin_off[b];
+    bin_lists(p->hc->stats, bin_count, bin_off);
     if (h->cfg.hbm_budget_bytes)
         require(static_cast<uint64_t>(products) * 24 <= h->cfg.hbm_budget_bytes, SPG_BUDGET_EXCEEDED,
                 "plan footprint exceeds the handle's HBM budget");

@@ -48,7 +48,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratch
 struct NoallocCtrl {
     Stats stats;
     ErrWord err;
-    int64_t bin_off[kNumBins + 1];
     unsigned long long cursor[kNumBins];
 };
 
@@ -169,8 +168,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         (ce = cudaMemcpyAsync(d_job, &job, sizeof job, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return from_cuda(ce, "scratch set-up", err, err_len);
     launch_rowwork(d_job, 1, d_row_base, m, A->nnz, &d_ctrl->stats, &d_ctrl->err, st);
-    launch_bin_offsets(&d_ctrl->stats, d_ctrl->bin_off, st);
-    launch_bin_scatter(d_job, 1, d_row_base, m, d_ctrl->bin_off, d_ctrl->cursor, items, st);
+    launch_bin_scatter(d_job, 1, d_row_base, m, &d_ctrl->stats, d_ctrl->cursor, items, st);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "row work launch", err, err_len);
     if ((ce = cudaMemcpyAsync(&hc, d_ctrl, sizeof hc, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (ce = cudaStreamSynchronize(st)) != cudaSuccess)
@@ -179,8 +177,8 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
     const int64_t max_ub = static_cast<int64_t>(hc.stats.max_ub);
     if (max_ub >= (int64_t{1} << 30))
         return ret(SPG_OVERFLOW, "an output row has more than 2^30 scalar products", err, err_len);
-    int64_t bin_count[kNumBins];
-    for (int b = 0; b < kNumBins; ++b) bin_count[b] = static_cast<int64_t>(hc.stats.bin_count[b]);
+    int64_t bin_count[kNumBins], bin_off[kNumBins + 1];
+    bin_lists(hc.stats, bin_count, bin_off);
     const NumericScratch ns = numeric_scratch(bin_count, max_ub, SplitTotals{}, num_sms, false, BinOrder::kSerial);
     const size_t slab = std::max(symbolic_scratch_bytes(bin_count, max_ub, num_sms), ns.bytes);
     unsigned char* d_slab = slab ? cv.take<unsigned char>(slab) : nullptr;
@@ -188,7 +186,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         return ret(SPG_BUDGET_EXCEEDED, "heavy rows need more than the 32 MiB allocation-free scratch", err, err_len);
 
     for (int b = 1; b < kNumBins; ++b)
-        launch_symbolic(b, d_job, items + hc.bin_off[b], static_cast<int64_t>(hc.stats.bin_count[b]), max_ub, d_slab,
+        launch_symbolic(b, d_job, items + bin_off[b], bin_count[b], max_ub, d_slab,
                         slab, &d_ctrl->stats, &d_ctrl->err, st, num_sms);
     launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "symbolic launch", err, err_len);
@@ -205,7 +203,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
     if ((ce = cudaMemcpyAsync(d_job, &job, sizeof job, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return from_cuda(ce, "job update", err, err_len);
     for (int b = 1; b < kNumBins; ++b)
-        launch_numeric(b, d_job, items + hc.bin_off[b], static_cast<int64_t>(hc.stats.bin_count[b]), max_ub, SplitTotals{}, d_slab,
+        launch_numeric(b, d_job, items + bin_off[b], bin_count[b], max_ub, SplitTotals{}, d_slab,
                        d_slab + ns.slab[b], &d_ctrl->stats, &d_ctrl->err, st, num_sms, false);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "numeric launch", err, err_len);
     if ((ce = cudaMemcpyAsync(&hc, d_ctrl, sizeof hc, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||

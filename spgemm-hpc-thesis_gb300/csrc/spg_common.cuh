@@ -190,19 +190,31 @@ __host__ __device__ inline int item_row(int64_t it) { return static_cast<int>(it
 // entries: stored entries of all A (sets the lanes per row only).
 void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows, int64_t entries,
                     Stats* d_stats, ErrWord* d_err, cudaStream_t stream);
-// K1b: scatter work items into per-bin lists (d_bin_off from the bin histogram).
+// K1b: scatter work items into per-bin lists, which follow one another in bin
+// order (Stats::bin_count, the empty rows' bin left out).
 void launch_bin_scatter(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                        const int64_t* d_bin_off, unsigned long long* d_bin_cursor, int64_t* d_items,
-                        cudaStream_t stream);
+                        const Stats* d_stats, unsigned long long* d_bin_cursor, int64_t* d_items, cudaStream_t stream);
+// Rows of every bin and the places of their lists (launch_bin_scatter).
+inline void bin_lists(const Stats& stats, int64_t* count, int64_t* off) {
+    int64_t at = 0;
+    for (int b = 0; b < kNumBins; ++b) {
+        count[b] = static_cast<int64_t>(stats.bin_count[b]);
+        off[b] = at;
+        if (b != kBinEmpty) at += count[b];
+    }
+    off[kNumBins] = at;
+}
 // K2: distinct columns per row into job.cnt[row] for the items of one bin.
 void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
                      void* d_scratch, size_t scratch_bytes, Stats* d_stats, ErrWord* d_err,
                      cudaStream_t stream, int num_sms);
 // Global scratch of the symbolic phase (hash slabs of rows above 8192 products).
 size_t symbolic_scratch_bytes(const int64_t* bin_count, int64_t max_ub, int num_sms);
-// K3: exclusive scan of n+1 int64 counts in place (last entry becomes the total).
+// K3: exclusive scan of n+1 int64 counts (16-byte aligned) in place (last entry
+// becomes the total).
 void launch_scan(int64_t* d_data, int64_t n, int64_t* d_partials, cudaStream_t stream);
 size_t scan_partials_count(int64_t n);
+int scan_launches(int64_t n);  // kernels of launch_scan
 // K4: sorted, summed, zero-free rows into job.c_col/c_val and job.nz[row].
 // holes: upper-bound layout (rows above kSplitThreshold products are then
 // split into column-range pieces; in the exact layout they keep their CTA
@@ -247,9 +259,6 @@ void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_va
 // whose column is >= 0.
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
                           int64_t slots, int32_t* out_col, double* out_val, cudaStream_t stream);
-// Bin list offsets from the bin histogram.
-void launch_bin_offsets(const Stats* d_stats, int64_t* d_bin_off, cudaStream_t stream);
-
 // Batched results: dst[i] = src[idx[i]] and per-product offset rebasing.
 struct RebaseItem {
     int64_t* rp;     // rows + 1 offsets of one product
