@@ -257,9 +257,10 @@ struct BinStreams {
     int next = 0;
 
     BinStreams(spg_handle* handle, int64_t products) : h(handle) {
-        order = h->serial_bins || h->one_bin_stream ? BinOrder::kSerial
-                : products <= kSpreadProducts       ? BinOrder::kSpread
-                                                    : BinOrder::kThreeStreams;
+        // (a handle with a budget keeps its slabs in one place)
+        order = h->serial_bins || h->one_bin_stream                             ? BinOrder::kSerial
+                : products <= kSpreadProducts && h->cfg.hbm_budget_bytes == 0 ? BinOrder::kSpread
+                                                                                : BinOrder::kThreeStreams;
     }
     // On several streams each starts with its largest rows; on one (server lanes,
     // the tuner) the bins go from the smallest rows up (measured faster for
@@ -296,12 +297,20 @@ struct BinStreams {
     }
 };
 
+// In the exact layout the rows above 8192 products may take the upper-bound
+// layout's way too, through C_tmp arrays of their own.
+struct ExactSplit {
+    const Job* d_jobs = nullptr;
+    void* scratch = nullptr;
+    int slab_ctas = 0;  // slabs of the whole-row kernels in the numeric scratch, for rows that cannot be split
+};
+
 // K4 of every bin.  In the upper-bound layout the rows of neighbouring bins
 // 17-19 are split in one launch (apart for the tuner, which times each bin).
 // Returns the kernels launched.
 int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, const int64_t* bin_count,
                     const int64_t* bin_off, int64_t max_ub, const SplitTotals& split, void* scratch,
-                    const NumericScratch& ns, Ctrl* d_ctrl, bool holes, bool timed) {
+                    const NumericScratch& ns, Ctrl* d_ctrl, bool holes, bool timed, const ExactSplit* exact_split = nullptr) {
     spg_handle* h = bs.h;
     int64_t launches = 0;
     bs.begin();
@@ -311,6 +320,18 @@ int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, con
         cudaStream_t st = bs.of(b);
         int first = b;
         int64_t count = bin_count[b];
+        if (exact_split && b > kLastSmemBin) {
+            for (first = kLastSmemBin + 1, count = 0; first < kNumBins; ++first) {
+                count += bin_count[first];
+                done[first] = true;
+            }
+            launch_split_exact(d_jobs, exact_split->d_jobs, items + bin_off[kLastSmemBin + 1], count, max_ub, split,
+                               exact_split->scratch, scratch, exact_split->slab_ctas, &d_ctrl->stats, &d_ctrl->err, st, h->num_sms);
+            launches += 5;
+            if (timed)
+                for (int i = kLastSmemBin + 1; i < kNumBins; ++i) cudaEventRecord(h->bin_ev[i], st);
+            return;
+        }
         const bool split_rows = holes && b > kLastSmemBin && !(b < kBinHeavy && h->bin_variant[b]);
         if (split_rows && bs.order != BinOrder::kSerial)  // the bins below join: their items precede b's
             while (first - 1 > kLastSmemBin && !h->bin_variant[first - 1]) {
@@ -436,14 +457,17 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     launches += scan_launches(static_cast<int64_t>(slots) - 1);
     int64_t tmp_total = products;
     if (exact) {
-        streams.begin();
-        streams.for_each_bin([&](int b) {
+        // K2's bins share no scratch: a stream each (0.86 -> 0.71 ms for 74 M products
+        // in 19 bins)
+        BinStreams k2(h, 0);
+        k2.begin();
+        k2.for_each_bin([&](int b) {
             if (!bin_count[b]) return;
             launch_symbolic(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, scratch, scratch_bytes,
-                            &d_ctrl->stats, &d_ctrl->err, streams.of(b), h->num_sms);
+                            &d_ctrl->stats, &d_ctrl->err, k2.of(b), h->num_sms);
             ++launches;
         });
-        streams.end();
+        k2.end();
         check_cuda(cudaGetLastError(), "K2 launch");
     }
     cudaEventRecord(h->ev[2], st);
@@ -472,7 +496,39 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         jobs[j].holes = exact ? 0 : 1;
     }
     check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D jobs");
-    launches += launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, !exact, true);
+    ExactSplit exact_split;
+    if (exact && split.rows > 0 && streams.order != BinOrder::kSerial) {
+        // only while it adds little to C's own memory and stays in the budget
+        const size_t staged = split_scratch_bytes(max_ub, split, h->num_sms);
+        const size_t tmp = static_cast<size_t>(split.products);
+        const size_t extra = staged + 12 * tmp + 8 * slots, c_bytes = 12 * static_cast<size_t>(tmp_total);
+        const int slab_ctas = static_cast<int>(std::min<size_t>(ns.front / (24 * static_cast<size_t>(max_ub)), 1 << 16));
+        if (slab_ctas > 0 && extra <= c_bytes / 4 + (size_t{64} << 20) &&
+            (!h->cfg.hbm_budget_bytes || ar.bytes() + extra <= h->cfg.hbm_budget_bytes)) {
+            try {
+                std::vector<Job> sj = jobs;
+                int64_t* off = ar.alloc<int64_t>(slots, "split offsets");
+                int32_t* col = ar.alloc<int32_t>(tmp, "split C_tmp col");
+                double* val = ar.alloc<double>(tmp, "split C_tmp val");
+                void* split_mem = ar.alloc<unsigned char>(staged, "split scratch");
+                Job* d_sj = ar.alloc<Job>(static_cast<size_t>(njobs), "split jobs");
+                for (int j = 0; j < njobs; ++j) {
+                    sj[j].cnt = off + row_base[j] + j;
+                    sj[j].c_col = col;
+                    sj[j].c_val = val;
+                    sj[j].holes = 1;
+                }
+                // (pageable source: the call returns once sj has been read)
+                check_cuda(cudaMemcpyAsync(d_sj, sj.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D split jobs");
+                exact_split = ExactSplit{d_sj, split_mem, slab_ctas};
+            } catch (const Failure& f) {
+                if (f.status != SPG_OUT_OF_MEMORY) throw;
+                cudaGetLastError();  // the whole-row kernels need no more memory
+            }
+        }
+    }
+    launches += launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, !exact, true,
+                            exact_split.d_jobs ? &exact_split : nullptr);
     check_cuda(cudaGetLastError(), "K4 launch");
     cudaEventRecord(h->ev[4], st);
     launch_readback(d_ctrl, hc, sizeof(Ctrl), st);

@@ -397,7 +397,8 @@ num_piece_kernel(const Job* __restrict__ jobs, SplitPlan plan, Stats* __restrict
 // fallback rows | staged columns | staged values | slabs (the pieces' value
 // slabs, then the global-slab sort of the fallback rows: one after the other).
 struct SplitLayout {
-    size_t pieces_off, fallback_off, col_off, val_off, slab_off, bytes;
+    size_t pieces_off, fallback_off, col_off, val_off, slab_off;
+    size_t staged, bytes;  // with the pieces' slabs; with those of the fallback rows too
     int64_t max_pieces;
 };
 
@@ -419,6 +420,7 @@ SplitLayout split_layout(int64_t max_ub, const SplitTotals& split, int num_sms) 
     L.slab_off = up(L.val_off + static_cast<size_t>(split_products) * sizeof(double));
     const size_t piece_slab = static_cast<size_t>(num_sms) * kPieceMinB * kPieceW * 32 * kPieceItems * sizeof(double);
     const size_t global_slab = static_cast<size_t>(heavy_grid(rows, num_sms)) * 24 * static_cast<size_t>(max_ub);
+    L.staged = L.slab_off + piece_slab;
     L.bytes = L.slab_off + std::max(piece_slab, global_slab);
     return L;
 }
@@ -496,6 +498,7 @@ NumericScratch numeric_scratch(const int64_t* bin_count, int64_t max_ub, const S
     }
     auto up = [](size_t x) { return (x + 255) & ~size_t{255}; };
     size_t at = order == BinOrder::kSerial ? 0 : up(front);
+    ns.front = front;
     ns.bytes = std::max(front, at);
     for (int b = 10; b <= kLastSmemBin; ++b) {
         const size_t bytes = cta_slab_bytes(b, bin_count[b], num_sms);
@@ -508,9 +511,10 @@ NumericScratch numeric_scratch(const int64_t* bin_count, int64_t max_ub, const S
 
 // Rows of more than kSplitThreshold products in upper-bound mode: plan and
 // stage, the pieces, then the rows left to the global-slab sort.
+// The latter's slabs: after the staging, or fallback_ctas of them elsewhere.
 static void launch_split(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
                          const SplitTotals& split, void* d_scratch, Stats* d_stats, ErrWord* d_err, cudaStream_t st,
-                         int num_sms) {
+                         int num_sms, void* fallback_slabs = nullptr, int fallback_ctas = 0) {
     const SplitLayout L = split_layout(max_ub, split, num_sms);
     unsigned char* base = static_cast<unsigned char*>(d_scratch);
     SplitPlan plan;
@@ -532,8 +536,91 @@ static void launch_split(int bin, const Job* d_jobs, const int64_t* d_items, int
     // the bin's own queue: where bins 17-19 run apart, they run one after the other
     kern<<<num_sms * kPieceMinB, kPieceW * 32, smem, st>>>(d_jobs, plan, d_stats, d_err, static_cast<double*>(slabs),
                                                           &d_stats->ticket[bin]);
-    num_heavy_kernel<<<heavy_grid(count, num_sms), kHeavyThreads, 0, st>>>(
-        d_jobs, plan.fallback, count, slabs, max_ub, d_stats, d_err, plan.counters + 1);
+    const int ctas = fallback_slabs ? std::min(fallback_ctas, heavy_grid(count, num_sms)) : heavy_grid(count, num_sms);
+    num_heavy_kernel<<<ctas, kHeavyThreads, 0, st>>>(d_jobs, plan.fallback, count, fallback_slabs ? fallback_slabs : slabs,
+                                                     max_ub, d_stats, d_err, plan.counters + 1);
+}
+
+namespace {
+
+// C_tmp slots of the split rows, in any order.
+__global__ void place_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count,
+                                  unsigned long long* __restrict__ cursor) {
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const Job& J = jobs[item_job(items[i])];
+        const int row = item_row(items[i]);
+        J.cnt[row] = static_cast<int64_t>(atomicAdd(cursor, static_cast<unsigned long long>(J.ub[row])));
+    }
+}
+
+// The slots of a split row with a column >= 0 to the row's place in the exact
+// layout, one CTA per row: warp w reads slots 128 w ... 128 w + 127 of every step.
+constexpr int kMoveW = 8;
+__global__ void __launch_bounds__(kMoveW * 32)
+move_rows_kernel(const Job* __restrict__ from, const Job* __restrict__ to, const int64_t* __restrict__ items,
+                 int64_t count) {
+    constexpr int U = 4, kStep = kMoveW * 32 * U;
+    __shared__ int s_kept[2][kMoveW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int par = 0;
+    for (int64_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const Job& F = from[item_job(items[i])];
+        const Job& T = to[item_job(items[i])];
+        const int row = item_row(items[i]);
+        const int64_t src = F.cnt[row], n = F.ub[row];
+        int64_t dst = T.cnt[row];
+        for (int64_t q0 = 0; q0 < n; q0 += kStep, par ^= 1) {
+            int32_t c[U];
+            double v[U];
+            unsigned m[U];
+            int mine = 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t q = q0 + (warp * U + u) * 32 + lane;
+                c[u] = q < n ? F.c_col[src + q] : -1;
+                v[u] = q < n ? F.c_val[src + q] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                m[u] = __ballot_sync(0xffffffffu, c[u] >= 0);
+                mine += __popc(m[u]);
+            }
+            if (lane == 0) s_kept[par][warp] = mine;
+            __syncthreads();  // the two rows of s_kept alternate: one barrier per step
+            int64_t at = dst;
+            for (int w = 0; w < kMoveW; ++w) {
+                if (w < warp) at += s_kept[par][w];
+                dst += s_kept[par][w];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (c[u] >= 0) {
+                    T.c_col[at + __popc(m[u] & lanemask_lt())] = c[u];
+                    T.c_val[at + __popc(m[u] & lanemask_lt())] = v[u];
+                }
+                at += __popc(m[u]);
+            }
+        }
+    }
+}
+
+}  // namespace
+
+size_t split_scratch_bytes(int64_t max_ub, const SplitTotals& split, int num_sms) {
+    return split.rows > 0 ? split_layout(max_ub, split, num_sms).staged : 0;
+}
+
+void launch_split_exact(const Job* d_jobs, const Job* d_split_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
+                        const SplitTotals& split, void* d_scratch, void* d_slabs, int slab_ctas, Stats* d_stats,
+                        ErrWord* d_err, cudaStream_t stream, int num_sms) {
+    if (count <= 0) return;
+    place_rows_kernel<<<static_cast<int>(std::min<int64_t>((count + 255) / 256, num_sms)), 256, 0, stream>>>(
+        d_split_jobs, d_items, count, &d_stats->ticket[kBinEmpty]);
+    launch_split(kBinHeavy, d_split_jobs, d_items, count, max_ub, split, d_scratch, d_stats, d_err, stream, num_sms, d_slabs,
+                 slab_ctas);
+    move_rows_kernel<<<static_cast<int>(std::min<int64_t>(count, 8 * num_sms)), kMoveW * 32, 0, stream>>>(
+        d_split_jobs, d_jobs, d_items, count);
 }
 
 void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,

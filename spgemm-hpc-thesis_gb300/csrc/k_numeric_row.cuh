@@ -588,6 +588,57 @@ __device__ __forceinline__ uint32_t write_slots(const uint32_t* keys, const doub
     return kept;
 }
 
+// Exact layout, step 4 of a region after fold_runs: the kept sums of the region
+// counted, or packed at [oc, ov).
+template <int S>
+__device__ __forceinline__ uint32_t count_kept(const uint32_t* keys, const double* vals, int n, int lane) {
+    uint32_t kept = 0;
+    for (int p0 = 0; p0 < n; p0 += 32) {
+        const uint32_t key = p0 + lane < n ? keys[p0 + lane] : kDeadKey;
+        kept += __popc(__ballot_sync(0xffffffffu, key != kDeadKey && nonzero(vals[key & ((1u << S) - 1u)])));
+    }
+    return kept;
+}
+template <int S>
+__device__ __forceinline__ uint32_t write_kept(const uint32_t* keys, const double* vals, int n, uint32_t first,
+                                               int32_t* __restrict__ oc, double* __restrict__ ov, int lane) {
+    uint32_t kept = 0;
+#pragma unroll 4
+    for (int p0 = 0; p0 < n; p0 += 32) {
+        const uint32_t key = p0 + lane < n ? keys[p0 + lane] : kDeadKey;
+        const double v = key != kDeadKey ? vals[key & ((1u << S) - 1u)] : 0.0;
+        const bool keep = nonzero(v);
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            const uint32_t at = kept + __popc(m & lanemask_lt());
+            oc[at] = static_cast<int32_t>((key >> S) + first);
+            ov[at] = v;
+        }
+        kept += __popc(m);
+    }
+    return kept;
+}
+
+// The kept sums of a CTA row in the exact layout, every warp its share's after
+// those of the warps before it.  Returns the row's kept sums.  (Out of line: the
+// upper-bound layout's kernels ran 1-4% slower with it inline.)
+template <int W, int S>
+__device__ __noinline__ int32_t write_share(const uint32_t* keys, const double* vals, int n, uint32_t first, int32_t* oc,
+                                            double* ov, int32_t* red, int lane, int warp) {
+    const uint32_t kept = count_kept<S>(keys, vals, n, lane);
+    if (lane == 0) red[warp] = static_cast<int32_t>(kept);
+    __syncthreads();
+    int at = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        const int32_t m = red[w];
+        at += w < warp ? m : 0;
+        all += m;
+    }
+    write_kept<S>(keys, vals, n, first, oc + at, ov + at, lane);
+    return all;
+}
+
 // write_slots for the rows that keep columns and sequence numbers apart: slots
 // [x0, x1) of a row whose runs may start or end anywhere in [lo, hi).  Returns
 // the warp's kept sums.
@@ -608,6 +659,58 @@ __device__ __noinline__ uint32_t write_slots_plain(const uint32_t* keys, const u
     }
     __syncwarp();
     return __reduce_add_sync(0xffffffffu, kept);
+}
+
+// The same in the exact layout, for a whole row by its team: steps 3 and 4.
+// Returns the row's kept sums.
+template <int W, int ITEMS, bool SV>
+__device__ __forceinline__ uint32_t write_kept_plain(RowSmem<W, ITEMS, SV>& sm, double* vals, int P, int32_t* oc, double* ov,
+                                                  int lane, int warp) {
+    // runs of equal columns summed in product order; each run's sum is stored in
+    // place of its first product's value
+#pragma unroll 1
+    for (int i = 0; i < ITEMS; ++i) {
+        const int pos = (warp * ITEMS + i) * 32 + lane;
+        bool keep = false;
+        if (pos < P) {
+            const uint32_t c = sm.keys[pos];
+            if (pos == 0 || sm.keys[pos - 1] != c) {
+                const uint32_t s0 = sm.seqs[pos];
+                double acc = vals[s0];
+                for (int q = pos + 1; q < P && sm.keys[q] == c; ++q) acc = __dadd_rn(acc, vals[sm.seqs[q]]);
+                vals[s0] = acc;
+                keep = nonzero(acc);
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) sm.cnt[warp * ITEMS + i] = __popc(m);
+    }
+    row_sync<W>();
+    scan_kept<W, ITEMS>(sm.cnt, sm.red, warp, lane);
+    row_sync<W>();
+    // kept (column, sum) pairs in sorted order
+#pragma unroll 1
+    for (int i = 0; i < ITEMS; ++i) {
+        const int pos = (warp * ITEMS + i) * 32 + lane;
+        bool keep = false;
+        uint32_t c = 0;
+        double v = 0.0;
+        if (pos < P) {
+            c = sm.keys[pos];
+            if (pos == 0 || sm.keys[pos - 1] != c) {
+                v = vals[sm.seqs[pos]];
+                keep = nonzero(v);
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            const int idx = static_cast<int>(sm.cnt[warp * ITEMS + i]) + __popc(m & lanemask_lt());
+            oc[idx] = static_cast<int32_t>(c);
+            ov[idx] = v;
+        }
+    }
+    if constexpr (W == 1) __syncwarp();
+    return static_cast<uint32_t>(sm.red[0]);
 }
 
 // The radix sort of the CTA rows with a large bucket (a column repeated more
@@ -646,15 +749,14 @@ __device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITE
         }
         warp_sort(k, lane);
         __syncwarp();
-        if (out.holes) {
-            fold_runs<ITEMS, kSeqBits>(k, sm.keys, sm.seqs, vals, P, lane);
-            kept = write_slots<kSeqBits>(sm.keys, vals, P, cmin, out.c_col + out.out0, out.c_val + out.out0, lane);
-            if (lane == 0) *out.nz = kept;
-            return lane == 0 ? kept : 0u;
-        }
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) sm.keys[lane * ITEMS + i] = k[i];
+        fold_runs<ITEMS, kSeqBits>(k, sm.keys, sm.seqs, vals, P, lane);
+        int32_t* oc = out.c_col + out.out0;
+        double* ov = out.c_val + out.out0;
+        kept = out.holes ? write_slots<kSeqBits>(sm.keys, vals, P, cmin, oc, ov, lane)
+                         : write_kept<kSeqBits>(sm.keys, vals, P, cmin, oc, ov, lane);
         __syncwarp();
+        if (lane == 0) *out.nz = kept;
+        return lane == 0 ? kept : 0u;
     } else if constexpr (W == 1) {
         radix_sort_row<W, ITEMS, SV, true>(sm, P, cmin, nbits, lane, warp, tid);
     } else {
@@ -710,8 +812,14 @@ __device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITE
                     settle_wide<N>(keys, seqs, n, static_cast<int>(biggest), lane);
                 } else {
                     settle(k, static_cast<int>(biggest), lane);
-                    if (out.holes) {
+                    if (out.holes || range < kMaxRange) {  // exact layout: no warp of the row is wide
                         fold_runs<N, kSeqBits>(k, keys, seqs, vals, n, lane);
+                        if (!out.holes) {
+                            const int32_t all = write_share<W, kSeqBits>(keys, vals, n, first, out.c_col + out.out0,
+                                                                         out.c_val + out.out0, sm.red, lane, warp);
+                            if (tid == 0) *out.nz = all;
+                            return tid == 0 ? static_cast<uint32_t>(all) : 0u;
+                        }
                         kept = write_slots<kSeqBits>(keys, vals, n, first, out.c_col + out.out0 + x0,
                                                      out.c_val + out.out0 + x0, lane);
                         written = true;
@@ -741,70 +849,16 @@ __device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITE
         }
     }
 
-    // Column and sequence number of sorted position pos.
-    auto col_at = [&](int pos) -> uint32_t {
-        return PACKED ? (sm.keys[pos] >> kSeqBits) : sm.keys[pos] - cmin;
-    };
-    auto seq_at = [&](int pos) -> uint32_t {
-        return PACKED ? (sm.keys[pos] & ((1u << kSeqBits) - 1u)) : sm.seqs[pos];
-    };
-
-    if constexpr (W == 1 && !PACKED) {
+    if constexpr (W == 1) {
         if (out.holes) {
             kept = write_slots_plain(sm.keys, sm.seqs, vals, 0, P, 0, P, out.c_col + out.out0, out.c_val + out.out0, lane);
             if (lane == 0) *out.nz = kept;
             return lane == 0 ? kept : 0u;
         }
     }
-
-    // 3. runs of equal columns summed in product order; each run's sum is stored
-    //    in place of its first product's value
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int pos = (warp * ITEMS + i) * 32 + lane;
-        bool keep = false;
-        if (pos < P) {
-            const uint32_t c = col_at(pos);
-            if (pos == 0 || col_at(pos - 1) != c) {
-                const uint32_t s0 = seq_at(pos);
-                double acc = vals[s0];
-                for (int q = pos + 1; q < P && col_at(q) == c; ++q) acc = __dadd_rn(acc, vals[seq_at(q)]);
-                vals[s0] = acc;
-                keep = nonzero(acc);
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) sm.cnt[warp * ITEMS + i] = __popc(m);
-    }
-    row_sync<W>();
-    scan_kept<W, ITEMS>(sm.cnt, sm.red, warp, lane);
-    row_sync<W>();
-
-    // 4. kept (column, sum) pairs in sorted order
-    const int64_t out0 = out.out0;
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int pos = (warp * ITEMS + i) * 32 + lane;
-        bool keep = false;
-        uint32_t c = 0;
-        double v = 0.0;
-        if (pos < P) {
-            c = col_at(pos);
-            if (pos == 0 || col_at(pos - 1) != c) {
-                v = vals[seq_at(pos)];
-                keep = nonzero(v);
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-            const int64_t idx = out0 + sm.cnt[warp * ITEMS + i] + __popc(m & lanemask_lt());
-            out.c_col[idx] = static_cast<int32_t>(c + cmin);
-            out.c_val[idx] = v;
-        }
-    }
-    if (tid == 0) *out.nz = sm.red[0];
-    if constexpr (W == 1) __syncwarp();
-    return tid == 0 ? static_cast<uint32_t>(sm.red[0]) : 0u;
+    kept = write_kept_plain(sm, vals, P, out.c_col + out.out0, out.c_val + out.out0, lane, warp);
+    if (tid == 0) *out.nz = kept;
+    return tid == 0 ? kept : 0u;
 }
 
 

@@ -22,12 +22,8 @@ namespace {
 constexpr int kSymWarpThreads = 256;
 constexpr int kSymHeavyThreads = 512;
 constexpr int kLastSymSmemBin = 18;  // rows of <= 16384 products: shared-memory tables
-#ifndef SPG_SYM_B64
-#define SPG_SYM_B64 10
-#endif
-#ifndef SPG_SYM_B128
-#define SPG_SYM_B128 12
-#endif
+// Last bins of the 64- and 128-thread CTAs (rows of <= 1024 and 2048 products).
+constexpr int kSymB64 = 10, kSymB128 = 12;
 
 // Table slots reserved per row (warp bins) or per CTA (CTA bins) for bin b:
 // the power of two >= twice its capacity, at least 64.
@@ -60,7 +56,7 @@ __global__ void __launch_bounds__(kSymWarpThreads)
 sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count, int tiny,
                 int wtab, ErrWord* __restrict__ err) {
     extern __shared__ int32_t s_dyn[];  // kSymWarpThreads / 32 tables of wtab slots
-    __shared__ SegTab<32, int32_t> s_seg[kSymWarpThreads / 32];
+    __shared__ RowSegs<32, 512> s_seg[kSymWarpThreads / 32];  // rows of at most 512 products
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (kSymWarpThreads / 32);
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * (kSymWarpThreads / 32) + w; i < count; i += warps) {
@@ -72,7 +68,7 @@ sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
         if (tiny) {
             // <= 32 products: product t goes to lane t; count the first lane of each column group.
             int32_t* stage = s_dyn + w * wtab;
-            team_products<32, false, int32_t>(J, row, s_seg[w], nullptr, lane, [&](int32_t seq, int32_t c, double, double) {
+            team_row_products<32, 512, 4, false>(J, row, s_seg[w], nullptr, lane, [&](int32_t seq, int32_t c, double, double) {
                 stage[seq] = c;
             });
             __syncwarp();
@@ -90,7 +86,7 @@ sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
             for (uint32_t s = lane; s < tsize; s += 32) tab[s] = -1;
             __syncwarp();
             int mine = 0;
-            team_products<32, false, int32_t>(J, row, s_seg[w], nullptr, lane, [&](int32_t, int32_t c, double, double) {
+            team_row_products<32, 512, 4, false>(J, row, s_seg[w], nullptr, lane, [&](int32_t, int32_t c, double, double) {
                 if (col_ok(c, J.B.cols, err)) mine += hash_insert(tab, mask, log2t, c);
             });
             found = warp_sum(mine);
@@ -100,12 +96,12 @@ sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
     }
 }
 
-template <int NT>
+template <int NT, int CAP>
 __global__ void __launch_bounds__(NT)
 sym_block_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count,
                  ErrWord* __restrict__ err) {
     extern __shared__ int32_t s_tab[];  // the bin's table slots
-    __shared__ SegTab<NT, int32_t> s_seg;
+    __shared__ RowSegs<NT, CAP> s_seg;
     __shared__ int64_t s_warp[NT / 32 + 1];
     __shared__ int s_found;
     for (int64_t i = blockIdx.x; i < count; i += gridDim.x) {
@@ -118,8 +114,7 @@ sym_block_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items
         if (threadIdx.x == 0) s_found = 0;
         __syncthreads();
         int mine = 0;
-        team_products<NT, false, int32_t>(J, row, s_seg, s_warp, threadIdx.x,
-                                                        [&](int32_t, int32_t c, double, double) {
+        team_row_products<NT, CAP, 4, false>(J, row, s_seg, s_warp, threadIdx.x, [&](int32_t, int32_t c, double, double) {
             if (col_ok(c, J.B.cols, err)) mine += hash_insert(s_tab, mask, log2t, c);
         });
         mine = warp_sum(mine);
@@ -190,10 +185,10 @@ void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t
             kernel<<<capped_grid(count, 1, num_sms * (2048 / nt)), nt, smem, stream>>>(d_jobs, d_items, count, d_err);
         };
         // CTA size by row size: 6-12 products per thread on the bins below 4096 products
-        if (bin <= SPG_SYM_B64) run(sym_block_kernel<64>, 64);
-        else if (bin <= SPG_SYM_B128) run(sym_block_kernel<128>, 128);
-        else if (bin <= kLastSmemBin) run(sym_block_kernel<256>, 256);
-        else run(sym_block_kernel<512>, 512);
+        if (bin <= kSymB64) run(sym_block_kernel<64, 1024>, 64);
+        else if (bin <= kSymB128) run(sym_block_kernel<128, 2048>, 128);
+        else if (bin <= kLastSmemBin) run(sym_block_kernel<256, 8192>, 256);
+        else run(sym_block_kernel<512, 16384>, 512);
     } else {
         const int grid = heavy_ctas(count, num_sms);
         const int64_t slots = int64_t{1} << ceil_log2(2 * max_ub);

@@ -226,6 +226,15 @@ int scan_launches(int64_t n);  // kernels of launch_scan
 void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
                     const SplitTotals& split, void* d_scratch, void* d_slab, Stats* d_stats, ErrWord* d_err,
                     cudaStream_t stream, int num_sms, bool holes, int variant = 0);
+// The rows of bins 17-19 in the exact layout by way of the split: d_split_jobs
+// are the jobs with holes set, C_tmp arrays of split.products slots and cnt
+// arrays of their own; the kept entries then move to d_jobs' places.  Scratch:
+// split_scratch_bytes, and slab_ctas slabs of 24 max_ub bytes for the rows that
+// cannot be split.
+size_t split_scratch_bytes(int64_t max_ub, const SplitTotals& split, int num_sms);
+void launch_split_exact(const Job* d_jobs, const Job* d_split_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
+                        const SplitTotals& split, void* d_scratch, void* d_slabs, int slab_ctas, Stats* d_stats,
+                        ErrWord* d_err, cudaStream_t stream, int num_sms);
 // The alternative shape of a bin; false if the bin has none.
 bool launch_numeric_alt(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, Stats* d_stats,
                         ErrWord* d_err, cudaStream_t stream, int num_sms);
@@ -242,7 +251,7 @@ enum class BinOrder { kSerial, kThreeStreams, kSpread };
 // slabs of their CTA kernels and global-slab sort; then the value slabs of the
 // CTA bins (byte offsets).
 struct NumericScratch {
-    size_t bytes = 0;
+    size_t bytes = 0, front = 0;
     size_t slab[kNumBins] = {};
 };
 NumericScratch numeric_scratch(const int64_t* bin_count, int64_t max_ub, const SplitTotals& split, int num_sms,

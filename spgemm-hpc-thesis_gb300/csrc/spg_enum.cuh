@@ -181,8 +181,9 @@ struct RowSegs {
 // product a thread takes (the team strides by multiples of 32), so the mask bits
 // at or below the product's position are lanemask_le.  The last batch ends
 // without a barrier: the caller's next barrier (or, for a warp, __syncwarp)
-// orders the products' shared-memory stores before their readers.
-template <int NT, int CAP, int U = 4, typename F>
+// orders the products' shared-memory stores before their readers.  kLoadVal =
+// false skips the values (b and a are then 0).
+template <int NT, int CAP, int U = 4, bool kLoadVal = true, typename F>
 __device__ inline void team_row_products(const Job& J, int row, RowSegs<NT, CAP>& tab, int64_t* s_warp, int tid,
                                          F&& f) {
     const bool has_s = J.S.rp != nullptr;
@@ -223,8 +224,10 @@ __device__ inline void team_row_products(const Job& J, int row, RowSegs<NT, CAP>
             const uint32_t s = (incl & 0xffffu) - static_cast<uint32_t>(len);
             const uint32_t r = (incl >> 16) - 1u;
             tab.colb[r] = reinterpret_cast<uint64_t>(cp) - 4u * static_cast<uint64_t>(s);
-            tab.valb[r] = reinterpret_cast<uint64_t>(vp) - 8u * static_cast<uint64_t>(s);
-            tab.scale[r] = sc;
+            if constexpr (kLoadVal) {
+                tab.valb[r] = reinterpret_cast<uint64_t>(vp) - 8u * static_cast<uint64_t>(s);
+                tab.scale[r] = sc;
+            }
             atomicOr(&tab.word[s >> 5].x, 1u << (s & 31u));
             for (uint32_t w = (s + 31u) >> 5; (w << 5) < s + static_cast<uint32_t>(len); ++w) tab.word[w].y = r;
         }
@@ -248,11 +251,11 @@ __device__ inline void team_row_products(const Job& J, int row, RowSegs<NT, CAP>
                 const int32_t t = t0 + u * NT;
                 const bool ok = t < total;
                 c[u] = ok ? __ldg(reinterpret_cast<const int32_t*>(tab.colb[r[u]] + 4u * static_cast<uint64_t>(t))) : 0;
-                b[u] = ok ? __ldg(reinterpret_cast<const double*>(tab.valb[r[u]] + 8u * static_cast<uint64_t>(t))) : 0.0;
+                b[u] = kLoadVal && ok ? __ldg(reinterpret_cast<const double*>(tab.valb[r[u]] + 8u * static_cast<uint64_t>(t))) : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (t0 + u * NT < total) f(seq_base + t0 + u * NT, c[u], b[u], tab.scale[r[u]]);
+                if (t0 + u * NT < total) f(seq_base + t0 + u * NT, c[u], b[u], kLoadVal ? tab.scale[r[u]] : 0.0);
         }
         seq_base += total;
         if (e0 + NT < nseg) team_sync<NT>();  // the next batch rewrites the table
