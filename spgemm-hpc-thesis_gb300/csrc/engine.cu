@@ -7,8 +7,9 @@
 //   -> (K5 compaction only if some sum was an exact zero) -> result.
 // All rows of all products of a call are flattened into one set of bin lists,
 // so a batch of products costs the same number of launches as one product.
-// Device memory comes from the device's stream-ordered pool (cudaMallocAsync),
-// whose release threshold is raised so that repeated calls reuse memory.
+// Device memory comes from the handle's kept blocks (blocks.h) and the device's
+// stream-ordered pool (cudaMallocAsync), whose release threshold is raised so
+// that repeated calls reuse memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -16,10 +17,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include "../../include/spgemm_gb300.h"
+#include "blocks.h"
 #include "spg_common.cuh"
 
 
@@ -29,6 +32,7 @@ struct spg_handle {
     int device = 0;
     int num_sms = 152;
     cudaStream_t stream = nullptr;
+    std::unique_ptr<BlockCache> blocks;  // device memory of the handle's calls
     spg_config cfg{};
     std::string err;
     cudaEvent_t ev[6] = {};
@@ -40,6 +44,7 @@ struct spg_handle {
     cudaEvent_t fork = nullptr, join[kAux] = {};
     bool serial_bins = false;  // spg_tune times bins one after the other
     bool one_bin_stream = false;  // spg_config.bin_streams == 1
+    bool force_exact = false, assumed_fit = false;  // use_exact_mode of the call in progress
     spg_timings last{};
     // accumulate mode: the running sum S (device result) and its shape
     bool acc_active = false;
@@ -50,6 +55,9 @@ struct spg_handle {
     void* ctrl = nullptr;
     // spg_multiply_to_host: copies of finished row blocks run on their own stream
     cudaStream_t copy_stream = nullptr;
+    // page-locked source of a call's row bases and jobs (grown on demand)
+    void* setup = nullptr;
+    size_t setup_bytes = 0;
     // page-locked staging for per-product reads of batches (grown on demand)
     void* host_scratch = nullptr;
     size_t host_scratch_bytes = 0;
@@ -77,18 +85,18 @@ void check_cuda(cudaError_t e, const char* what) {
     throw Failure{s, std::string(what) + ": " + cudaGetErrorString(e)};
 }
 
-// Device allocations of one call; freed on the stream unless released to a result.
+// Device allocations of one call; freed unless released to a result.
 class Arena {
 public:
     explicit Arena(spg_handle* h) : h_(h) {}
     ~Arena() {
         for (void* p : live_)
-            if (p) cudaFreeAsync(p, h_->stream);
+            if (p) h_->blocks->free(p);
     }
     template <typename T>
     T* alloc(size_t count, const char* what) {
         void* p = nullptr;
-        check_cuda(cudaMallocAsync(&p, std::max<size_t>(count * sizeof(T), 16), h_->stream), what);
+        check_cuda(h_->blocks->alloc(&p, std::max<size_t>(count * sizeof(T), 16)), what);
         live_.push_back(p);
         bytes_ += count * sizeof(T);
         return static_cast<T*>(p);
@@ -100,7 +108,7 @@ public:
     void free_now(void* p) {
         for (auto& q : live_)
             if (q == p) {
-                cudaFreeAsync(q, h_->stream);
+                h_->blocks->free(q);
                 q = nullptr;
             }
     }
@@ -221,11 +229,20 @@ spg_status map_err(const ErrWord& e, std::string& msg) {
 // The exact (symbolic) mode when asked for, or in auto mode when reserving
 // 12 bytes per slot would not fit the budget or half the free memory (slots:
 // the scalar products, plus the staged ones of rows above 8192 products).
+// Small needs are not compared with the free memory, whose query takes as long as
+// all the launches of a small call: if the memory runs out, the call is made again
+// in the exact mode (run_products).
+constexpr size_t kSmallNeed = size_t{2} << 30;
+
 bool use_exact_mode(spg_handle* h, int64_t products, size_t reserved) {
-    if (h->cfg.mode == SPG_MODE_EXACT) return true;
+    if (h->cfg.mode == SPG_MODE_EXACT || h->force_exact) return true;
     if (h->cfg.mode == SPG_MODE_UPPER_BOUND) return false;
     const size_t need = static_cast<size_t>(products) * 12;
     if (h->cfg.hbm_budget_bytes && reserved + need > h->cfg.hbm_budget_bytes) return true;
+    if (need <= kSmallNeed) {
+        h->assumed_fit = true;
+        return false;
+    }
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
@@ -350,10 +367,46 @@ int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, con
     return launches;
 }
 
+// Row bases and jobs of a call, in one device block, uploaded in one copy from
+// page-locked memory (whose previous copy has finished: every upload of a call is
+// followed by a wait before the next).
+struct CallSetup {
+    spg_handle* h;
+    size_t job_off, bytes;
+    unsigned char* host;
+    unsigned char* dev;
+
+    CallSetup(spg_handle* handle, Arena& ar, const std::vector<int64_t>& row_base) : h(handle) {
+        const size_t njobs = row_base.size() - 1;
+        job_off = sizeof(int64_t) * row_base.size();
+        bytes = job_off + sizeof(Job) * njobs;
+        if (bytes > h->setup_bytes) {
+            sync(h);
+            if (h->setup) cudaFreeHost(h->setup);
+            h->setup = nullptr;
+            h->setup_bytes = 0;
+            const size_t want = std::max<size_t>(bytes, 16 << 10);
+            check_cuda(cudaMallocHost(&h->setup, want), "host setup");
+            h->setup_bytes = want;
+        }
+        host = static_cast<unsigned char*>(h->setup);
+        std::memcpy(host, row_base.data(), job_off);
+        dev = ar.alloc<unsigned char>(bytes, "row_base and jobs");
+    }
+    int64_t* row_base() const { return reinterpret_cast<int64_t*>(dev); }
+    Job* jobs() const { return reinterpret_cast<Job*>(dev + job_off); }
+    void upload(const std::vector<Job>& jobs, bool all) const {
+        std::memcpy(host + job_off, jobs.data(), bytes - job_off);
+        const size_t from = all ? 0 : job_off;
+        check_cuda(cudaMemcpyAsync(dev + from, host + from, bytes - from, cudaMemcpyHostToDevice, h->stream), "H2D jobs");
+    }
+};
+static_assert(alignof(Job) <= 8, "jobs follow 8-byte row bases");
+
 // The phase pipeline for one or more products.  Results stay on the device.
 // products_out (optional) receives the scalar products of every product.
-void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                  int64_t* products_out) {
+void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
+                       int64_t* products_out) {
     cudaStream_t st = h->stream;
     Arena ar(h);
     const int njobs = static_cast<int>(in.size());
@@ -385,20 +438,23 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     int64_t* cnt = ar.alloc<int64_t>(slots, "cnt");
     int64_t* nz = ar.alloc<int64_t>(slots, "nz");
     int64_t* items = ar.alloc<int64_t>(static_cast<size_t>(total_rows), "items");
-    int64_t* d_row_base = ar.alloc<int64_t>(static_cast<size_t>(njobs) + 1, "row_base");
     Ctrl* d_ctrl = ar.alloc<Ctrl>(1, "ctrl");
-    Job* d_jobs = ar.alloc<Job>(static_cast<size_t>(njobs), "jobs");
+    bool empty_job = false;
     for (int j = 0; j < njobs; ++j) {
         jobs[j].ub = ub + row_base[j];
         jobs[j].cnt = cnt + row_base[j] + j;
         jobs[j].nz = nz + row_base[j] + j;
+        empty_job = empty_job || in[j].A->rows == 0;
     }
-    check_cuda(cudaMemsetAsync(cnt, 0, slots * sizeof(int64_t), st), "memset cnt");
-    check_cuda(cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st), "memset nz");
+    if (empty_job) {  // K1 zeroes nz and the entries past the last row of every other job
+        check_cuda(cudaMemsetAsync(cnt, 0, slots * sizeof(int64_t), st), "memset cnt");
+        check_cuda(cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st), "memset nz");
+    }
     check_cuda(cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st), "memset ctrl");
-    check_cuda(cudaMemcpyAsync(d_row_base, row_base.data(), sizeof(int64_t) * (njobs + 1), cudaMemcpyHostToDevice, st),
-               "H2D row_base");
-    check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D jobs");
+    const CallSetup setup(h, ar, row_base);
+    const int64_t* d_row_base = setup.row_base();
+    Job* d_jobs = setup.jobs();
+    setup.upload(jobs, true);
 
     Ctrl* hc = static_cast<Ctrl*>(h->ctrl);
     int64_t launches = total_rows > 0 ? 2 : 0;  // K1, K1b
@@ -495,7 +551,7 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         jobs[j].c_val = c_val;
         jobs[j].holes = exact ? 0 : 1;
     }
-    check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D jobs");
+    setup.upload(jobs, false);
     ExactSplit exact_split;
     if (exact && split.rows > 0 && streams.order != BinOrder::kSerial) {
         // only while it adds little to C's own memory and stays in the budget
@@ -599,12 +655,10 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
             r.v = ar.alloc<double>(static_cast<size_t>(r.nnz), "result val");
             jobs[j].out_col = r.ci;
             jobs[j].out_val = r.v;
-            check_cuda(cudaMemcpyAsync(r.rp, nz + row_base[j] + j, sizeof(int64_t) * (r.rows + 1),
-                                       cudaMemcpyDeviceToDevice, st), "D2D row_ptr");
-            rb[j] = RebaseItem{r.rp, starts[j], r.rows};
+            rb[j] = RebaseItem{r.rp, nz + row_base[j] + j, starts[j], r.rows};
             max_rows = std::max<int64_t>(max_rows, r.rows);
         }
-        check_cuda(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st), "H2D jobs");
+        setup.upload(jobs, false);
         if (exact) {
             for (int j = 0; j < njobs; ++j) launch_compact(d_jobs + j, in[j].A->rows, nullptr, nullptr, st);
         } else {
@@ -652,12 +706,42 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
     for (int b = 0; b < kNumBins; ++b) h->last.bin_rows[b] = bin_count[b];
 }
 
+void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
+                  int64_t* products_out) {
+    h->force_exact = false;
+    h->assumed_fit = false;
+    const auto drain = [&] {  // nothing of the failed attempt still reads what it freed or what it uploads from
+        for (auto a : h->aux) cudaStreamSynchronize(a);
+        cudaStreamSynchronize(h->stream);
+        cudaGetLastError();
+        out.clear();
+    };
+    try {
+        run_products_once(h, in, out, count_only, products_out);
+    } catch (const Failure& f) {
+        drain();
+        if (f.status != SPG_OUT_OF_MEMORY || !h->assumed_fit) throw;
+        h->force_exact = true;
+        try {
+            run_products_once(h, in, out, count_only, products_out);
+        } catch (...) {
+            h->force_exact = false;
+            drain();
+            throw;
+        }
+        h->force_exact = false;
+    } catch (...) {
+        drain();
+        throw;
+    }
+}
+
 void free_result_arrays(spg_handle* h, spg_csr_result* c) {
     if (!c) return;
     if (c->location == SPG_DEVICE) {
-        if (c->row_ptr) cudaFreeAsync(c->row_ptr, h->stream);
-        if (c->col) cudaFreeAsync(c->col, h->stream);
-        if (c->val) cudaFreeAsync(c->val, h->stream);
+        h->blocks->free(c->row_ptr);
+        h->blocks->free(c->col);
+        h->blocks->free(c->val);
     } else {
         std::free(c->row_ptr);
         std::free(c->col);
@@ -697,9 +781,9 @@ void deliver(spg_handle* h, DevResult& r, int32_t loc, spg_csr_result* C) {
     if (e == cudaSuccess && r.nnz)
         e = cudaMemcpyAsync(C->val, r.v, sizeof(double) * r.nnz, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFreeAsync(r.rp, h->stream);
-    cudaFreeAsync(r.ci, h->stream);
-    cudaFreeAsync(r.v, h->stream);
+    h->blocks->free(r.rp);
+    h->blocks->free(r.ci);
+    h->blocks->free(r.v);
     if (e != cudaSuccess) {
         free_result_arrays(h, C);
         check_cuda(e, "D2H result");
@@ -768,6 +852,7 @@ spg_status spg_create(const spg_config* config, spg_handle** out) {
         uint64_t threshold = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
     }
+    h->blocks = std::make_unique<BlockCache>(h->device, h->stream);
     *out = h;
     return SPG_OK;
 }
@@ -782,6 +867,7 @@ void spg_destroy(spg_handle* h) {
         cudaStreamDestroy(h->copy_stream);
     }
     if (h->host_scratch) cudaFreeHost(h->host_scratch);
+    if (h->setup) cudaFreeHost(h->setup);
     for (auto& e : h->ev) cudaEventDestroy(e);
     for (auto& e : h->bin_ev) cudaEventDestroy(e);
     for (auto a : h->aux) {
@@ -790,6 +876,7 @@ void spg_destroy(spg_handle* h) {
     }
     if (h->fork) cudaEventDestroy(h->fork);
     for (auto e : h->join) cudaEventDestroy(e);
+    h->blocks.reset();
     cudaStreamDestroy(h->stream);
     cudaFreeHost(h->ctrl);
     delete h;
@@ -900,9 +987,9 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
         std::vector<DevResult> held;
         auto release_held = [&] {
             for (auto& q : held) {
-                cudaFreeAsync(q.rp, st);
-                cudaFreeAsync(q.ci, st);
-                cudaFreeAsync(q.v, st);
+                h->blocks->free(q.rp);
+                h->blocks->free(q.ci);
+                h->blocks->free(q.v);
             }
             held.clear();
         };
@@ -1085,9 +1172,9 @@ spg_status spg_tune(spg_handle* h, const spg_csr_view* A, const spg_csr_view* B,
                 std::vector<DevResult> out;
                 run_products(h, in, out, false, nullptr);
                 for (auto& o : out) {
-                    cudaFreeAsync(o.rp, h->stream);
-                    cudaFreeAsync(o.ci, h->stream);
-                    cudaFreeAsync(o.v, h->stream);
+                    h->blocks->free(o.rp);
+                    h->blocks->free(o.ci);
+                    h->blocks->free(o.v);
                 }
             };
             for (int v = 0; v < kNumVariants; ++v) {
@@ -1346,11 +1433,9 @@ spg_status spg_accum_finish(spg_handle* h, int32_t out_location, spg_csr_result*
         r.nnz = h->acc_has ? h->acc.nnz : 0;
         r.products = h->acc_has ? h->acc.products : 0;
         const size_t rp_bytes = sizeof(int64_t) * (static_cast<size_t>(r.rows) + 1);
-        check_cuda(cudaMallocAsync(reinterpret_cast<void**>(&r.rp), rp_bytes, h->stream), "alloc row_ptr");
-        check_cuda(cudaMallocAsync(reinterpret_cast<void**>(&r.ci), std::max<size_t>(16, 4 * r.nnz), h->stream),
-                   "alloc col");
-        check_cuda(cudaMallocAsync(reinterpret_cast<void**>(&r.v), std::max<size_t>(16, 8 * r.nnz), h->stream),
-                   "alloc val");
+        check_cuda(h->blocks->alloc(reinterpret_cast<void**>(&r.rp), rp_bytes), "alloc row_ptr");
+        check_cuda(h->blocks->alloc(reinterpret_cast<void**>(&r.ci), std::max<size_t>(16, 4 * r.nnz)), "alloc col");
+        check_cuda(h->blocks->alloc(reinterpret_cast<void**>(&r.v), std::max<size_t>(16, 8 * r.nnz)), "alloc val");
         if (h->acc_has) {
             check_cuda(cudaMemcpyAsync(r.rp, h->acc.row_ptr, rp_bytes, cudaMemcpyDeviceToDevice, h->stream), "D2D");
             if (r.nnz) {
@@ -1416,7 +1501,7 @@ namespace {
 template <typename T>
 T* plan_alloc(spg_plan* p, size_t count, const char* what) {
     void* q = nullptr;
-    check_cuda(cudaMalloc(&q, std::max<size_t>(count * sizeof(T), 16)), what);
+    check_cuda(device_malloc(&q, std::max<size_t>(count * sizeof(T), 16)), what);
     p->bufs.push_back(q);
     return static_cast<T*>(q);
 }
@@ -1533,7 +1618,10 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     for (int32_t r : p->rows) max_rows = std::max<int64_t>(max_rows, r);
 
     // values: the replayed part
-    check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed), "begin capture");
+    h->blocks->set_capturing(true);
+    const cudaError_t be = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
+    if (be != cudaSuccess) h->blocks->set_capturing(false);
+    check_cuda(be, "begin capture");
     cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st);
     cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st);
     // (the bins' fork and join are part of the graph)
@@ -1546,6 +1634,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     launch_readback(d_ctrl, p->hc, sizeof(Ctrl), st);
     const cudaError_t le = cudaGetLastError();
     const cudaError_t ce = cudaStreamEndCapture(st, &p->graph);
+    h->blocks->set_capturing(false);
     check_cuda(le, "plan capture launches");
     check_cuda(ce, "end capture");
     check_cuda(cudaGraphInstantiate(&p->exec, p->graph, 0), "graph instantiate");

@@ -532,7 +532,7 @@ static void launch_split(int bin, const Job* d_jobs, const int64_t* d_items, int
     using PieceSm = RowSmem<kPieceW, kPieceItems, false>;
     const int smem = static_cast<int>(sizeof(PieceSm));
     auto kern = num_piece_kernel<kPieceW, kPieceItems, kPieceMinB>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem<num_piece_kernel<kPieceW, kPieceItems, kPieceMinB>>(smem);
     // the bin's own queue: where bins 17-19 run apart, they run one after the other
     kern<<<num_sms * kPieceMinB, kPieceW * 32, smem, st>>>(d_jobs, plan, d_stats, d_err, static_cast<double*>(slabs),
                                                           &d_stats->ticket[bin]);

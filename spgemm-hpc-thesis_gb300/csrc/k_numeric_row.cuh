@@ -1034,7 +1034,7 @@ template <int ITEMS>
 void run_warp(const Job* jobs, const int64_t* items, int64_t count, Stats* stats, ErrWord* err, cudaStream_t st,
               int num_sms) {
     const int smem = 8 * static_cast<int>(sizeof(RowSmem<1, ITEMS>));
-    cudaFuncSetAttribute(num_warp_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem<num_warp_kernel<ITEMS>>(smem);
     num_warp_kernel<ITEMS><<<capped(count, 8, num_sms * 16), kWarpKernelThreads, smem, st>>>(jobs, items, count, stats,
                                                                                            err);
 }
@@ -1043,7 +1043,7 @@ template <int W, int ITEMS, int MINB, bool SV = true>
 void run_block(const Job* jobs, const int64_t* items, int64_t count, Stats* stats, ErrWord* err, cudaStream_t st,
                int num_sms, unsigned long long* ticket, double* gvals = nullptr) {
     const int smem = static_cast<int>(sizeof(RowSmem<W, ITEMS, SV>));
-    cudaFuncSetAttribute(num_block_kernel<W, ITEMS, MINB, SV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem<num_block_kernel<W, ITEMS, MINB, SV>>(smem);
     // One wave of resident CTAs: with the row queue, CTAs beyond it would start
     // only once the queue has run dry (slab bins: one slab per resident CTA).
     static std::atomic<int> resident{0};  // per instantiation (every device of this build is an sm_103a)

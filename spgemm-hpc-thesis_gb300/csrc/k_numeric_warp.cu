@@ -344,7 +344,7 @@ template <int I, int G>
 void run_rows(const Job* jobs, const int64_t* items, int64_t count, Stats* stats, ErrWord* err, cudaStream_t st,
               int num_sms) {
     const int smem = 8 * static_cast<int>(sizeof(RowsSmem<I, G>));
-    cudaFuncSetAttribute(num_rows_kernel<I, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem<num_rows_kernel<I, G>>(smem);
     num_rows_kernel<I, G><<<capped(count, 8 * G, num_sms * 16), kWarpKernelThreads, smem, st>>>(jobs, items, count, stats,
                                                                                               err);
 }

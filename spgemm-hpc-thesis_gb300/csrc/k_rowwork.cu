@@ -116,6 +116,11 @@ rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restric
             if (J.S.rp) len += J.S.rp[row + 1] - J.S.rp[row];
             J.ub[row] = len;
             J.cnt[row] = len;  // upper-bound layout; the exact mode's symbolic phase overwrites it
+            if (J.nz) J.nz[row] = 0;
+            if (row == J.A.rows - 1) {  // the entries past the last row, which the scans turn into totals
+                J.cnt[row + 1] = 0;
+                if (J.nz) J.nz[row + 1] = 0;
+            }
             atomicAdd(&s_bins[bin_of(len)], 1u);
             products += len;
             most = len > most ? len : most;
@@ -454,7 +459,7 @@ __global__ void rebase_kernel(const RebaseItem* __restrict__ items) {
     const RebaseItem it = items[blockIdx.y];
     for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r <= it.rows;
          r += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        it.rp[r] -= it.start;
+        it.rp[r] = it.src[r] - it.start;
 }
 
 int grid_for(int64_t work, int per_block, int cap) {

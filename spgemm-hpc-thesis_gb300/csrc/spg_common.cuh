@@ -10,6 +10,7 @@
 // bit-identical to the reference's serial product.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -182,6 +183,18 @@ __host__ __device__ inline int64_t make_item(int job, int row) {
 __host__ __device__ inline int item_job(int64_t it) { return static_cast<int>(it >> 32); }
 __host__ __device__ inline int item_row(int64_t it) { return static_cast<int>(it & 0xffffffff); }
 
+// Lets kernel K take `bytes` of dynamic shared memory, once per device.
+template <auto K>
+void allow_smem(int bytes) {
+    constexpr int kDevices = 64;
+    static std::atomic<int> allowed[kDevices];
+    int d = 0;
+    cudaGetDevice(&d);
+    if (d < kDevices && allowed[d].load(std::memory_order_relaxed) >= bytes) return;
+    if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess && d < kDevices)
+        allowed[d].store(bytes, std::memory_order_relaxed);
+}
+
 // --------------------------------------------------------------------------
 // Host-side launchers (one per phase).  All are asynchronous on `stream`.
 
@@ -268,10 +281,12 @@ void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_va
 // whose column is >= 0.
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
                           int64_t slots, int32_t* out_col, double* out_val, cudaStream_t stream);
-// Batched results: dst[i] = src[idx[i]] and per-product offset rebasing.
+// Batched results: dst[i] = src[idx[i]], and the offsets of every product from
+// those of the whole batch.
 struct RebaseItem {
-    int64_t* rp;     // rows + 1 offsets of one product
-    int64_t start;   // subtracted from every offset
+    int64_t* rp;         // rows + 1 offsets of one product
+    const int64_t* src;  // the same in the batch
+    int64_t start;       // subtracted from every offset
     int64_t rows;
 };
 void launch_gather(const int64_t* d_src, const int64_t* d_idx, int64_t* d_dst, int n, cudaStream_t stream);
