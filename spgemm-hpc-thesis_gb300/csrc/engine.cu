@@ -607,7 +607,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
             final_col = ar.alloc<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
             final_val = ar.alloc<double>(static_cast<size_t>(nz_total), "C val (compact)");
             if (exact) launch_compact(d_jobs, in[0].A->rows, final_col, final_val, st);
-            else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, final_col, final_val, st);
+            else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, final_col, final_val, st);
             check_cuda(cudaGetLastError(), "K5 launch");
             final_rp = nz;
             ar.free_now(c_col);
@@ -662,7 +662,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         if (exact) {
             for (int j = 0; j < njobs; ++j) launch_compact(d_jobs + j, in[j].A->rows, nullptr, nullptr, st);
         } else {
-            launch_compact_holes(d_jobs, njobs, d_row_base, total_rows, products, nullptr, nullptr, st);
+            launch_compact_holes(d_jobs, njobs, d_row_base, total_rows, products, items, bin_off, nullptr, nullptr, st);
         }
         check_cuda(cudaGetLastError(), "K5 launch");
         ar.free_now(c_col);
@@ -1627,7 +1627,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     // (the bins' fork and join are part of the graph)
     launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, true, false);
     launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
-    launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, p->col, p->val, st);
+    launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, items, bin_off, p->col, p->val, st);
     launch_gather(nz, d_idx, d_starts, n, st);
     launch_rebase_jobs(nz, p->rp, d_row_base, n, max_rows, st);
     launch_readback(d_starts, p->h_starts, sizeof(int64_t) * n, st);

@@ -340,28 +340,101 @@ compact_kernel(const Job* __restrict__ job, int rows, int32_t* __restrict__ out_
     }
 }
 
+// The rows of more than kLongSlots slots (long_rows, items of the bin lists), a
+// CTA each: a step takes kChunks chunks of 32 slots per warp, whose counts place the
+// warps' entries after one another.
+__device__ void compact_long_rows(const Job* __restrict__ jobs, const int64_t* __restrict__ long_rows, int64_t n_long,
+                                  int64_t first, int64_t step, int32_t* __restrict__ out_col,
+                                  double* __restrict__ out_val) {
+    constexpr int kChunks = 8, kWarps = 8;
+    __shared__ int s_count[2][kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int side = 0;
+    for (int64_t i = first; i < n_long; i += step) {
+        const Job& J = jobs[item_job(long_rows[i])];
+        const int r = item_row(long_rows[i]);
+        int32_t* __restrict__ oc = out_col ? out_col : J.out_col;
+        double* __restrict__ ov = out_col ? out_val : J.out_val;
+        const int64_t end = J.cnt[r + 1];
+        int64_t dst = J.nz[r] - (out_col ? 0 : J.nz[0]);
+        for (int64_t q0 = J.cnt[r]; q0 < end; q0 += kWarps * kChunks * 32) {
+            int32_t c[kChunks];
+            double v[kChunks];
+            const int64_t at = q0 + warp * (kChunks * 32) + lane;
+#pragma unroll
+            for (int u = 0; u < kChunks; ++u) {
+                c[u] = at + u * 32 < end ? J.c_col[at + u * 32] : -1;
+                v[u] = at + u * 32 < end ? J.c_val[at + u * 32] : 0.0;
+            }
+            int count = 0;
+#pragma unroll
+            for (int u = 0; u < kChunks; ++u) count += __popc(__ballot_sync(0xffffffffu, c[u] >= 0));
+            if (lane == 0) s_count[side][warp] = count;
+            __syncthreads();  // the other side's counts are written only after the next one
+            int64_t to = dst;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const int n = s_count[side][w];
+                dst += n;
+                if (w < warp) to += n;
+            }
+            side ^= 1;
+#pragma unroll
+            for (int u = 0; u < kChunks; ++u) {
+                const unsigned m = __ballot_sync(0xffffffffu, c[u] >= 0);
+                if (c[u] >= 0) {
+                    oc[to + __popc(m & lanemask_lt())] = c[u];
+                    ov[to + __popc(m & lanemask_lt())] = v[u];
+                }
+                to += __popc(m);
+            }
+        }
+    }
+}
+
 // K5 for rows written with holes (upper-bound mode): a warp takes `group`
 // consecutive rows, whose reserved slots [cnt[r], cnt[r + group]) are contiguous
 // as their entries in C are: the slots are read in order and those with a column
 // >= 0 packed from the first row's final offset nz[r] on (ballot + popc).  Each
 // warp loads its next group's offsets while it copies the current one, and issues
-// eight chunks of 32 slots per step.  Power-law product: 6.1 TB/s, 89% of the
-// measured copy bandwidth; 262,144 rows of 56 and of 32 slots: 0.068 ms together
-// (0.188 with one row per warp, whose eight chunks were mostly empty).
+// eight chunks of 32 slots per step.  262,144 rows of 56 and of 32 slots: 0.068 ms
+// together (0.188 with one row per warp, whose eight chunks were mostly empty).
+// A step of a warp waits about 1 us for memory, so one row of 100,000 slots alone
+// took a warp as long as the GPU needs for 100 M slots: rows of kLongBin and above
+// are left to the first `long_ctas` CTAs.  Power-law squares of 65,539, 100,003 and
+// 1 M rows (36, 56 and 595 M slots): 165, 244 and 2,205 us (339, 422 and 2,360
+// before); the last is 6.3 TB/s, 94% of the measured copy bandwidth.
 __global__ void __launch_bounds__(256)
 compact_holes_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ job_row_base,
-                     int64_t total_rows, int group, int32_t* __restrict__ out_col, double* __restrict__ out_val) {
+                     int64_t total_rows, int group, const int64_t* __restrict__ long_rows, int64_t n_long,
+                     int long_ctas, int32_t* __restrict__ out_col, double* __restrict__ out_val) {
     constexpr int kChunks = 8;
+    if (static_cast<int>(blockIdx.x) < long_ctas) {
+        compact_long_rows(jobs, long_rows, n_long, blockIdx.x, long_ctas, out_col, out_val);
+        return;
+    }
     const int lane = threadIdx.x & 31;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5) * group;
-    int64_t g = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * group;
+    const int64_t stride = static_cast<int64_t>(gridDim.x - long_ctas) * (blockDim.x >> 5) * group;
+    int64_t g = (static_cast<int64_t>(blockIdx.x - long_ctas) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * group;
     int64_t group_end = min(g + group, total_rows);
     int j = 0;
     int64_t n_src = 0, n_end = 0, n_dst = 0, n_row = 0;
     auto load_rows = [&](int64_t row) {  // the group's rows from `row` on, of one product
         j = job_of_row(job_row_base, njobs, row);
         n_row = min(group_end, job_row_base[j + 1]);
-        const int r = static_cast<int>(row - job_row_base[j]), r1 = static_cast<int>(n_row - job_row_base[j]);
+        const int r = static_cast<int>(row - job_row_base[j]);
+        int r1 = static_cast<int>(n_row - job_row_base[j]);
+        if (long_ctas) {  // up to the next long row, or past one
+            for (int i = r; i < r1; i += 32) {
+                const bool is_long = i + lane < r1 && jobs[j].cnt[i + lane + 1] - jobs[j].cnt[i + lane] > kLongSlots;
+                const unsigned m = __ballot_sync(0xffffffffu, is_long);
+                if (m) {
+                    r1 = i + __ffs(m) - 1;
+                    break;
+                }
+            }
+            n_row = job_row_base[j] + max(r1, r + 1);
+        }
         n_src = jobs[j].cnt[r];
         n_end = jobs[j].cnt[r1];
         n_dst = jobs[j].nz[r] - (out_col ? 0 : jobs[j].nz[0]);  // the job's own arrays start at its first row
@@ -515,13 +588,16 @@ void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_va
 }
 
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                          int64_t slots, int32_t* out_col, double* out_val, cudaStream_t stream) {
+                          int64_t slots, const int64_t* items, const int64_t* bin_off, int32_t* out_col,
+                          double* out_val, cudaStream_t stream) {
     if (total_rows <= 0) return;
+    const int64_t n_long = bin_off[kNumBins] - bin_off[kLongBin];
+    const int long_ctas = static_cast<int>(std::min<int64_t>(n_long, 152 * 8));
     // Rows per warp: about two steps of 256 slots.
     const int64_t mean = slots / total_rows + 1;
     const int group = static_cast<int>(std::min<int64_t>(std::max<int64_t>(512 / mean, 1), 64));
-    compact_holes_kernel<<<grid_for(total_rows, 8 * group, 152 * 32), 256, 0, stream>>>(
-        d_jobs, njobs, d_job_row_base, total_rows, group, out_col, out_val);
+    compact_holes_kernel<<<long_ctas + grid_for(total_rows, 8 * group, 152 * 128), 256, 0, stream>>>(
+        d_jobs, njobs, d_job_row_base, total_rows, group, items + bin_off[kLongBin], n_long, long_ctas, out_col, out_val);
 }
 
 void launch_gather(const int64_t* d_src, const int64_t* d_idx, int64_t* d_dst, int n, cudaStream_t stream) {

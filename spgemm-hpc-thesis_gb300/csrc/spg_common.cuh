@@ -278,9 +278,16 @@ inline SplitTotals split_totals(const Stats& st) {
 // with out_col == nullptr, into the job's own arrays (Job::out_col / out_val).
 void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_val, cudaStream_t stream);
 // K5 for rows written with holes: keeps the slots (of which there are `slots`)
-// whose column is >= 0.
+// whose column is >= 0.  items, bin_off: the bin lists.
+// Rows of kLongBin and above (more than kLongSlots slots) take a CTA each, the
+// others a warp: at 100,003 and 1 M power-law rows 236 and 2,261 us, against 255 and
+// 2,302 with the line at 8192 slots and 234 and 2,265 at 2048, where sixteen products
+// of 20,000 rows lose (323 -> 339 us: a CTA takes one row at a time).
+constexpr int kLongBin = 15;
+constexpr int64_t kLongSlots = 4096;
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                          int64_t slots, int32_t* out_col, double* out_val, cudaStream_t stream);
+                          int64_t slots, const int64_t* items, const int64_t* bin_off, int32_t* out_col,
+                          double* out_val, cudaStream_t stream);
 // Batched results: dst[i] = src[idx[i]], and the offsets of every product from
 // those of the whole batch.
 struct RebaseItem {
