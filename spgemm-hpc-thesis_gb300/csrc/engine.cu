@@ -204,6 +204,11 @@ struct Ctrl {  // layout of the pinned control block and its device twin
     int64_t totals[2];  // scanned totals (symbolic, numeric)
 };
 
+Readback readback_of(const void* d_src, void* h_dst, size_t bytes) {
+    return Readback{static_cast<const unsigned long long*>(d_src), static_cast<unsigned long long*>(h_dst),
+                    static_cast<int>(bytes / 8)};
+}
+
 static_assert(sizeof(Ctrl) % 8 == 0 && sizeof(Ctrl) <= 4096, "Ctrl is read back in 8-byte words into kCtrlBytes");
 
 spg_status map_err(const ErrWord& e, std::string& msg) {
@@ -272,6 +277,7 @@ struct BinStreams {
     BinOrder order;
     bool used[spg_handle::kAux] = {};
     int next = 0;
+    bool alone = false;
 
     BinStreams(spg_handle* handle, int64_t products) : h(handle) {
         // (a handle with a budget keeps its slabs in one place)
@@ -286,10 +292,14 @@ struct BinStreams {
     void for_each_bin(F&& f) const {
         for (int i = 1; i < kNumBins; ++i) f(order == BinOrder::kSerial ? i : kNumBins - i);
     }
-    void begin() {
+    // A lone bin stays on the handle's stream.
+    void begin(const int64_t* bin_count) {
         std::fill(used, used + spg_handle::kAux, false);
         next = 0;
-        if (order != BinOrder::kSerial) cudaEventRecord(h->fork, h->stream);
+        int bins = 0;
+        for (int b = 1; b < kNumBins; ++b) bins += bin_count[b] > 0;
+        alone = bins < 2;
+        if (order != BinOrder::kSerial && !alone) cudaEventRecord(h->fork, h->stream);
     }
     cudaStream_t aux(int i) {
         if (!used[i]) cudaStreamWaitEvent(h->aux[i], h->fork, 0);
@@ -299,7 +309,7 @@ struct BinStreams {
     // The stream of bin b's launch (called once per launch, in launch order).
     // The rows above 8192 products share scratch: always one stream.
     cudaStream_t of(int b) {
-        if (order == BinOrder::kSerial) return h->stream;
+        if (order == BinOrder::kSerial || alone) return h->stream;
         if (b > kLastSmemBin) return aux(1);
         if (order == BinOrder::kThreeStreams) return b <= kLastWarpBin ? h->stream : aux(0);
         const int i = next++ % spg_handle::kAux;
@@ -330,7 +340,7 @@ int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, con
                     const NumericScratch& ns, Ctrl* d_ctrl, bool holes, bool timed, const ExactSplit* exact_split = nullptr) {
     spg_handle* h = bs.h;
     int64_t launches = 0;
-    bs.begin();
+    bs.begin(bin_count);
     bool done[kNumBins] = {};
     bs.for_each_bin([&](int b) {
         if (done[b] || !bin_count[b]) return;
@@ -367,18 +377,28 @@ int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, con
     return launches;
 }
 
-// Row bases and jobs of a call, in one device block, uploaded in one copy from
-// page-locked memory (whose previous copy has finished: every upload of a call is
-// followed by a wait before the next).
+// Scalar products up to which the compaction does not wait for the stored count,
+// whose wait and the launches after it take 20 us (a 1,000-row square of 1.1 M
+// products: 188 -> 171 us a call with the readbacks and memset below taken into other
+// launches; accumulation of four products 894 -> 805).  C's arrays
+// then have the upper bound's size: at most 48 MiB where the caller keeps them, 384
+// where they only live until they have been copied or added to.
+constexpr int64_t kDirectProducts = int64_t{1} << 22;
+constexpr int64_t kDirectTransient = int64_t{1} << 25;
+
+// Row bases, zeroed control block and jobs of a call, in one device block, uploaded
+// in one copy from page-locked memory (whose previous copy has finished: every
+// upload of a call is followed by a wait before the next).
 struct CallSetup {
     spg_handle* h;
-    size_t job_off, bytes;
+    size_t ctrl_off, job_off, bytes;
     unsigned char* host;
     unsigned char* dev;
 
     CallSetup(spg_handle* handle, Arena& ar, const std::vector<int64_t>& row_base) : h(handle) {
         const size_t njobs = row_base.size() - 1;
-        job_off = sizeof(int64_t) * row_base.size();
+        ctrl_off = sizeof(int64_t) * row_base.size();
+        job_off = ctrl_off + sizeof(Ctrl);
         bytes = job_off + sizeof(Job) * njobs;
         if (bytes > h->setup_bytes) {
             sync(h);
@@ -390,10 +410,12 @@ struct CallSetup {
             h->setup_bytes = want;
         }
         host = static_cast<unsigned char*>(h->setup);
-        std::memcpy(host, row_base.data(), job_off);
-        dev = ar.alloc<unsigned char>(bytes, "row_base and jobs");
+        std::memcpy(host, row_base.data(), ctrl_off);
+        std::memset(host + ctrl_off, 0, sizeof(Ctrl));
+        dev = ar.alloc<unsigned char>(bytes, "row_base, ctrl and jobs");
     }
     int64_t* row_base() const { return reinterpret_cast<int64_t*>(dev); }
+    Ctrl* ctrl() const { return reinterpret_cast<Ctrl*>(dev + ctrl_off); }
     Job* jobs() const { return reinterpret_cast<Job*>(dev + job_off); }
     void upload(const std::vector<Job>& jobs, bool all) const {
         std::memcpy(host + job_off, jobs.data(), bytes - job_off);
@@ -401,12 +423,13 @@ struct CallSetup {
         check_cuda(cudaMemcpyAsync(dev + from, host + from, bytes - from, cudaMemcpyHostToDevice, h->stream), "H2D jobs");
     }
 };
-static_assert(alignof(Job) <= 8, "jobs follow 8-byte row bases");
+static_assert(alignof(Job) <= 8 && alignof(Ctrl) <= 8, "both follow 8-byte row bases");
 
 // The phase pipeline for one or more products.  Results stay on the device.
-// products_out (optional) receives the scalar products of every product.
+// products_out (optional) receives the scalar products of every product.  transient:
+// the results do not outlive the call, or the next one's.
 void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                       int64_t* products_out) {
+                       int64_t* products_out, bool transient) {
     cudaStream_t st = h->stream;
     Arena ar(h);
     const int njobs = static_cast<int>(in.size());
@@ -438,7 +461,6 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     int64_t* cnt = ar.alloc<int64_t>(slots, "cnt");
     int64_t* nz = ar.alloc<int64_t>(slots, "nz");
     int64_t* items = ar.alloc<int64_t>(static_cast<size_t>(total_rows), "items");
-    Ctrl* d_ctrl = ar.alloc<Ctrl>(1, "ctrl");
     bool empty_job = false;
     for (int j = 0; j < njobs; ++j) {
         jobs[j].ub = ub + row_base[j];
@@ -450,9 +472,9 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         check_cuda(cudaMemsetAsync(cnt, 0, slots * sizeof(int64_t), st), "memset cnt");
         check_cuda(cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st), "memset nz");
     }
-    check_cuda(cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st), "memset ctrl");
     const CallSetup setup(h, ar, row_base);
     const int64_t* d_row_base = setup.row_base();
+    Ctrl* d_ctrl = setup.ctrl();
     Job* d_jobs = setup.jobs();
     setup.upload(jobs, true);
 
@@ -460,7 +482,8 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     int64_t launches = total_rows > 0 ? 2 : 0;  // K1, K1b
     cudaEventRecord(h->ev[0], st);
     launch_rowwork(d_jobs, njobs, d_row_base, total_rows, entries, &d_ctrl->stats, &d_ctrl->err, st);
-    launch_bin_scatter(d_jobs, njobs, d_row_base, total_rows, &d_ctrl->stats, d_ctrl->cursor, items, st);
+    launch_bin_scatter(d_jobs, njobs, d_row_base, total_rows, &d_ctrl->stats, d_ctrl->cursor, items, st,
+                       readback_of(d_ctrl, hc, offsetof(Ctrl, cursor)));
     check_cuda(cudaGetLastError(), "K1 launch");
     cudaEventRecord(h->ev[1], st);
     std::vector<int64_t> job_products(njobs, 0);
@@ -472,8 +495,21 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         launch_readback(d_jp, h_jp, sizeof(int64_t) * njobs, st);
         launches += 2;
     }
-    launch_readback(d_ctrl, hc, sizeof(Ctrl), st);
-    ++launches;
+    if (total_rows == 0) {
+        launch_readback(d_ctrl, hc, sizeof(Ctrl), st);
+        ++launches;
+    }
+    // K3 of the upper-bound layout needs nothing from the host: it runs while the
+    // host waits for the row work
+    const size_t reserved = ar.bytes();
+    int64_t* partials = nullptr;
+    const bool scanned = !count_only && h->cfg.mode != SPG_MODE_EXACT && !h->force_exact;
+    if (!count_only) partials = ar.alloc<int64_t>(scan_partials_count(static_cast<int64_t>(slots)), "scan partials");
+    if (scanned) {
+        launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
+        launches += scan_launches(static_cast<int64_t>(slots) - 1);
+        cudaEventRecord(h->ev[2], st);
+    }
     check_cuda(cudaGetLastError(), "readback launch");
     sync(h);  // sync 1: bins and input checks
     if (h_jp) std::copy(h_jp, h_jp + njobs, job_products.begin());
@@ -502,21 +538,21 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     // rows above 8192 are also staged (12 more bytes each); in the exact mode a
     // symbolic phase counts the distinct columns of every row first.
     const SplitTotals split = split_totals(hc->stats);
-    const bool exact = use_exact_mode(h, products + split.products, ar.bytes());
+    const bool exact = use_exact_mode(h, products + split.products, reserved);
     // K2 and K4 run their bins on several streams (BinStreams)
     BinStreams streams(h, products);
     const NumericScratch ns = numeric_scratch(bin_count, max_ub, split, h->num_sms, !exact, streams.order);
     size_t scratch_bytes = ns.bytes;
     if (exact) scratch_bytes = std::max(scratch_bytes, symbolic_scratch_bytes(bin_count, max_ub, h->num_sms));
     void* scratch = scratch_bytes ? ar.alloc<unsigned char>(scratch_bytes, "numeric scratch") : nullptr;
-    int64_t* partials = ar.alloc<int64_t>(scan_partials_count(static_cast<int64_t>(slots)), "scan partials");
-    launches += scan_launches(static_cast<int64_t>(slots) - 1);
     int64_t tmp_total = products;
     if (exact) {
+        // (K2 counts the rows of its bins only)
+        if (scanned) check_cuda(cudaMemsetAsync(cnt, 0, slots * sizeof(int64_t), st), "memset cnt");
         // K2's bins share no scratch: a stream each (0.86 -> 0.71 ms for 74 M products
         // in 19 bins)
         BinStreams k2(h, 0);
-        k2.begin();
+        k2.begin(bin_count);
         k2.for_each_bin([&](int b) {
             if (!bin_count[b]) return;
             launch_symbolic(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, scratch, scratch_bytes,
@@ -526,9 +562,12 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         k2.end();
         check_cuda(cudaGetLastError(), "K2 launch");
     }
-    cudaEventRecord(h->ev[2], st);
-    launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
-    check_cuda(cudaGetLastError(), "K3 launch");
+    if (exact) {
+        cudaEventRecord(h->ev[2], st);
+        launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
+        launches += scan_launches(static_cast<int64_t>(slots) - 1);
+        check_cuda(cudaGetLastError(), "K3 launch");
+    }
     cudaEventRecord(h->ev[3], st);
     if (exact) {
         launch_readback(cnt + slots - 1, &hc->totals[0], sizeof(int64_t), st);
@@ -587,8 +626,26 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
                             exact_split.d_jobs ? &exact_split : nullptr);
     check_cuda(cudaGetLastError(), "K4 launch");
     cudaEventRecord(h->ev[4], st);
-    launch_readback(d_ctrl, hc, sizeof(Ctrl), st);
-    ++launches;
+    // Up to kDirectProducts the compaction follows without a wait for the stored
+    // count, into arrays of the upper bound's size; it moves nothing if there is
+    // nothing to close up.
+    const bool direct = !exact && njobs == 1 && total_rows > 0 && !h->cfg.hbm_budget_bytes &&
+                        products <= (transient ? kDirectTransient : kDirectProducts);
+    int32_t* k5_col = nullptr;
+    double* k5_val = nullptr;
+    if (direct) {
+        k5_col = ar.alloc<int32_t>(static_cast<size_t>(products), "C col (compact)");
+        k5_val = ar.alloc<double>(static_cast<size_t>(products), "C val (compact)");
+        launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
+        launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, k5_col, k5_val, st,
+                             readback_of(d_ctrl, hc, offsetof(Ctrl, cursor)), &d_ctrl->stats, &d_ctrl->err);
+        launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
+        check_cuda(cudaGetLastError(), "K5 launch");
+        cudaEventRecord(h->ev[5], st);
+    } else {
+        launch_readback(d_ctrl, hc, sizeof(Ctrl), st);
+        ++launches;
+    }
     sync(h);  // stored count and errors
     if (hc->err.code) {
         std::string msg;
@@ -602,18 +659,22 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         int32_t* final_col = c_col;
         double* final_val = c_val;
         if (nz_total != tmp_total) {  // rows with fewer entries than reserved: compact
-            launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
-            launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
-            final_col = ar.alloc<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
-            final_val = ar.alloc<double>(static_cast<size_t>(nz_total), "C val (compact)");
-            if (exact) launch_compact(d_jobs, in[0].A->rows, final_col, final_val, st);
-            else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, final_col, final_val, st);
-            check_cuda(cudaGetLastError(), "K5 launch");
+            final_col = k5_col;
+            final_val = k5_val;
+            if (!direct) {
+                launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
+                launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
+                final_col = ar.alloc<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
+                final_val = ar.alloc<double>(static_cast<size_t>(nz_total), "C val (compact)");
+                if (exact) launch_compact(d_jobs, in[0].A->rows, final_col, final_val, st);
+                else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, final_col, final_val, st);
+                check_cuda(cudaGetLastError(), "K5 launch");
+            }
             final_rp = nz;
             ar.free_now(c_col);
             ar.free_now(c_val);
         }
-        cudaEventRecord(h->ev[5], st);
+        if (!direct) cudaEventRecord(h->ev[5], st);
         DevResult& r = out[0];
         r.rows = in[0].A->rows;
         r.cols = in[0].B->cols;
@@ -682,10 +743,10 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         sync(h);  // jobs, idx and rb must outlive their copies
     }
     for (int j = 0; j < njobs; ++j) out[j].products = job_products[j];
-    sync(h);
+    if (!direct) sync(h);
     h->last.ms_rowwork = elapsed(h->ev[0], h->ev[1]);
-    h->last.ms_symbolic = elapsed(h->ev[1], h->ev[2]);
-    h->last.ms_scan = elapsed(h->ev[2], h->ev[3]);
+    h->last.ms_symbolic = exact ? elapsed(h->ev[1], h->ev[2]) : elapsed(h->ev[2], h->ev[3]);
+    h->last.ms_scan = exact ? elapsed(h->ev[2], h->ev[3]) : elapsed(h->ev[1], h->ev[2]);
     h->last.ms_numeric = elapsed(h->ev[3], h->ev[4]);
     h->last.ms_compact = elapsed(h->ev[4], h->ev[5]);
     h->last.ms_total = elapsed(h->ev[0], h->ev[5]);
@@ -707,7 +768,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
 }
 
 void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                  int64_t* products_out) {
+                  int64_t* products_out, bool transient = false) {
     h->force_exact = false;
     h->assumed_fit = false;
     const auto drain = [&] {  // nothing of the failed attempt still reads what it freed or what it uploads from
@@ -717,13 +778,13 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         out.clear();
     };
     try {
-        run_products_once(h, in, out, count_only, products_out);
+        run_products_once(h, in, out, count_only, products_out, transient);
     } catch (const Failure& f) {
         drain();
         if (f.status != SPG_OUT_OF_MEMORY || !h->assumed_fit) throw;
         h->force_exact = true;
         try {
-            run_products_once(h, in, out, count_only, products_out);
+            run_products_once(h, in, out, count_only, products_out, transient);
         } catch (...) {
             h->force_exact = false;
             drain();
@@ -910,7 +971,7 @@ spg_status spg_multiply(spg_handle* h, const spg_csr_view* A, const spg_csr_view
         require(out_location == SPG_HOST || out_location == SPG_DEVICE, SPG_INVALID_ARGUMENT, "bad out_location");
         std::vector<JobIn> in{{A, B, CsrView{}}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr);
+        run_products(h, in, out, false, nullptr, out_location == SPG_HOST);
         deliver(h, out[0], out_location, C);
     });
 }
@@ -1013,7 +1074,7 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
                 blk.row_ptr = dv[0].row_ptr + r0;  // absolute offsets into A's column/value arrays
                 std::vector<JobIn> in{{&blk, &dv[1], CsrView{}}};
                 std::vector<DevResult> out;
-                run_products(h, in, out, false, nullptr);
+                run_products(h, in, out, false, nullptr, true);
                 DevResult& r = out[0];
                 held.push_back(r);  // freed by release_held, on success or failure
                 if (off + r.nnz > c_capacity) {
@@ -1413,7 +1474,7 @@ spg_status spg_accum_add(spg_handle* h, const spg_csr_view* A, const spg_csr_vie
         }
         std::vector<JobIn> in{{A, B, S}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr);
+        run_products(h, in, out, false, nullptr, true);
         if (h->acc_has) free_result_arrays(h, &h->acc);
         deliver(h, out[0], SPG_DEVICE, &h->acc);
         h->acc_has = true;

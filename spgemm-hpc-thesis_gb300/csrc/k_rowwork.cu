@@ -145,6 +145,11 @@ rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restric
     }
 }
 
+__device__ __forceinline__ void read_back(const Readback& r) {
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < r.words; i += blockDim.x) r.dst[i] = r.src[i];
+}
+
 // A CTA takes kScatterRows rows at a time, counts them by bin in shared memory
 // (the counter's old value is the row's place among them) and takes one range of
 // every bin's list: one global atomic per bin and CTA.  With one per bin and warp,
@@ -155,7 +160,8 @@ constexpr int kScatterRows = 256 * kScatterItems;
 __global__ void __launch_bounds__(256)
 bin_scatter_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ job_row_base,
                    int64_t total_rows, const Stats* __restrict__ stats,
-                   unsigned long long* __restrict__ cursor, int64_t* __restrict__ items) {
+                   unsigned long long* __restrict__ cursor, int64_t* __restrict__ items, const Readback read) {
+    read_back(read);
     __shared__ int64_t s_list[kNumBins];  // the lists follow one another in bin order
     __shared__ int64_t s_base[kNumBins];
     __shared__ unsigned int s_count[kNumBins];
@@ -407,8 +413,11 @@ __device__ void compact_long_rows(const Job* __restrict__ jobs, const int64_t* _
 __global__ void __launch_bounds__(256)
 compact_holes_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ job_row_base,
                      int64_t total_rows, int group, const int64_t* __restrict__ long_rows, int64_t n_long,
-                     int long_ctas, int32_t* __restrict__ out_col, double* __restrict__ out_val) {
+                     int long_ctas, int32_t* __restrict__ out_col, double* __restrict__ out_val, const Readback read,
+                     const Stats* full, int64_t slots, const ErrWord* err) {
     constexpr int kChunks = 8;
+    read_back(read);
+    if (full && (err->code != 0 || static_cast<int64_t>(full->nz_total) == slots)) return;
     if (static_cast<int>(blockIdx.x) < long_ctas) {
         compact_long_rows(jobs, long_rows, n_long, blockIdx.x, long_ctas, out_col, out_val);
         return;
@@ -560,11 +569,12 @@ void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base,
 }
 
 void launch_bin_scatter(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                        const Stats* d_stats, unsigned long long* d_bin_cursor, int64_t* d_items, cudaStream_t stream) {
+                        const Stats* d_stats, unsigned long long* d_bin_cursor, int64_t* d_items, cudaStream_t stream,
+                        const Readback& read) {
     if (total_rows <= 0) return;
     const int grid = grid_for(total_rows, kScatterRows, 152 * 8);
     bin_scatter_kernel<<<grid, 256, 0, stream>>>(d_jobs, njobs, d_job_row_base, total_rows, d_stats, d_bin_cursor,
-                                                  d_items);
+                                                  d_items, read);
 }
 
 size_t scan_partials_count(int64_t n) { return static_cast<size_t>((n + kScanTile - 1) / kScanTile) + 1; }
@@ -589,7 +599,8 @@ void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_va
 
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
                           int64_t slots, const int64_t* items, const int64_t* bin_off, int32_t* out_col,
-                          double* out_val, cudaStream_t stream) {
+                          double* out_val, cudaStream_t stream, const Readback& read, const Stats* full,
+                          const ErrWord* err) {
     if (total_rows <= 0) return;
     const int64_t n_long = bin_off[kNumBins] - bin_off[kLongBin];
     const int long_ctas = static_cast<int>(std::min<int64_t>(n_long, 152 * 8));
@@ -597,7 +608,8 @@ void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row
     const int64_t mean = slots / total_rows + 1;
     const int group = static_cast<int>(std::min<int64_t>(std::max<int64_t>(512 / mean, 1), 64));
     compact_holes_kernel<<<long_ctas + grid_for(total_rows, 8 * group, 152 * 128), 256, 0, stream>>>(
-        d_jobs, njobs, d_job_row_base, total_rows, group, items + bin_off[kLongBin], n_long, long_ctas, out_col, out_val);
+        d_jobs, njobs, d_job_row_base, total_rows, group, items + bin_off[kLongBin], n_long, long_ctas, out_col,
+        out_val, read, full, slots, err);
 }
 
 void launch_gather(const int64_t* d_src, const int64_t* d_idx, int64_t* d_dst, int n, cudaStream_t stream) {

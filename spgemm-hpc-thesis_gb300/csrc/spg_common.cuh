@@ -198,6 +198,13 @@ void allow_smem(int bytes) {
 // --------------------------------------------------------------------------
 // Host-side launchers (one per phase).  All are asynchronous on `stream`.
 
+// A small device->host read that a kernel makes on its way: its first block copies
+// `words` 8-byte words into page-locked memory (launch_readback without the launch).
+struct Readback {
+    const unsigned long long* src = nullptr;
+    unsigned long long* dst = nullptr;
+    int words = 0;
+};
 // K1: products per row (ub), bin histogram, product total and input checks.
 // Rows of all jobs are flattened: job j owns rows [row_base_j, row_base_j + A_j.rows).
 // entries: stored entries of all A (sets the lanes per row only).
@@ -206,7 +213,8 @@ void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base,
 // K1b: scatter work items into per-bin lists, which follow one another in bin
 // order (Stats::bin_count, the empty rows' bin left out).
 void launch_bin_scatter(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
-                        const Stats* d_stats, unsigned long long* d_bin_cursor, int64_t* d_items, cudaStream_t stream);
+                        const Stats* d_stats, unsigned long long* d_bin_cursor, int64_t* d_items, cudaStream_t stream,
+                        const Readback& read = {});
 // Rows of every bin and the places of their lists (launch_bin_scatter).
 inline void bin_lists(const Stats& stats, int64_t* count, int64_t* off) {
     int64_t at = 0;
@@ -278,7 +286,9 @@ inline SplitTotals split_totals(const Stats& st) {
 // with out_col == nullptr, into the job's own arrays (Job::out_col / out_val).
 void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_val, cudaStream_t stream);
 // K5 for rows written with holes: keeps the slots (of which there are `slots`)
-// whose column is >= 0.  items, bin_off: the bin lists.
+// whose column is >= 0.  items, bin_off: the bin lists.  With full != nullptr the
+// kernel moves nothing after an error or if every slot holds an entry
+// (full->nz_total == slots), for a caller that does not know yet.
 // Rows of kLongBin and above (more than kLongSlots slots) take a CTA each, the
 // others a warp: at 100,003 and 1 M power-law rows 236 and 2,261 us, against 255 and
 // 2,302 with the line at 8192 slots and 234 and 2,265 at 2048, where sixteen products
@@ -287,7 +297,8 @@ constexpr int kLongBin = 15;
 constexpr int64_t kLongSlots = 4096;
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
                           int64_t slots, const int64_t* items, const int64_t* bin_off, int32_t* out_col,
-                          double* out_val, cudaStream_t stream);
+                          double* out_val, cudaStream_t stream, const Readback& read = {},
+                          const Stats* full = nullptr, const ErrWord* err = nullptr);
 // Batched results: dst[i] = src[idx[i]], and the offsets of every product from
 // those of the whole batch.
 struct RebaseItem {
