@@ -59,15 +59,15 @@ __device__ __forceinline__ int hidx(int d, int w) {
     return W == 1 ? d : d * kHistStride<W> + w;
 }
 
-// Buckets of a CTA row (bucket_order below): coarse buckets (their table of two
-// words each, then their counters) and at most one fine bucket per product (and
+// Buckets of a CTA row (bucket_order below): coarse buckets (their table of one
+// word each, then their counters) and at most one fine bucket per product (and
 // one word past the last).
 template <int W>
 constexpr int kCoarseBits = W <= 4 ? 7 : 8;
 template <int W>
 constexpr int kCoarse = 1 << kCoarseBits<W>;
 template <int W, int ITEMS>
-constexpr int kBucketWords = W == 1 ? 4 : 3 * kCoarse<W> + W * 32 * ITEMS + 4;
+constexpr int kBucketWords = W == 1 ? 4 : 2 * kCoarse<W> + W * 32 * ITEMS + 4;
 // A warp finishes the sort of its share of a CTA row's positions, rounded to
 // whole buckets, in registers: kShareItems per lane.  A fine bucket larger than
 // the rounding allows sends the row to the radix sort.
@@ -95,7 +95,7 @@ struct RowSmem {
     double vals[SV ? kCap : 1];  // product values by sequence number; run sums in place
     RowSegs<W * 32, W * 32 * ITEMS> seg;  // enumeration batch
     int64_t warp_tmp[W + 1];    // block scans
-    uint32_t keys[kCap];        // columns (unpacked) or packed (column, sequence) words
+    alignas(16) uint32_t keys[kCap];  // columns (unpacked) or packed (column, sequence) words
     union {
         alignas(16) uint32_t hist[kHistWords<W>];  // digit counters of the radix sort at hidx<W>(digit, warp)
         alignas(16) uint32_t bk[kBucketWords<W, ITEMS>];  // bucket counters, then bucket starts (CTA rows)
@@ -219,36 +219,25 @@ struct RowOut {
     int32_t nz_add;     // a piece of a split row: add to *nz instead of storing it
 };
 
-// Exclusive scan of v over the W*32 threads of a row's team in thread order,
-// with the total and the team-wide maximum of m (red: 2*W words; one barrier
-// for a CTA, none for a warp).  red is next written after later barriers of
-// the row, so no barrier protects it here.
+// The sum of `all` over the warps before this one, and the team-wide maximum of m
+// (red: 2*W words; one barrier).  red is next written after later barriers of the
+// row, so no barrier protects it here.
 template <int W>
-__device__ inline uint32_t block_excl_scan_max(uint32_t v, uint32_t m, int32_t* red, int lane, int warp,
-                                               uint32_t& total, uint32_t& mx) {
-    const uint32_t incl = warp_incl_scan(v, lane);
+__device__ inline uint32_t block_warps_before(uint32_t all, uint32_t m, int32_t* red, int lane, int warp, uint32_t& mx) {
     const uint32_t wm = __reduce_max_sync(0xffffffffu, m);
-    if constexpr (W == 1) {
-        total = __shfl_sync(0xffffffffu, incl, 31);
-        mx = wm;
-        return incl - v;
-    }
     if (lane == 31) {
-        red[warp] = static_cast<int32_t>(incl);
+        red[warp] = static_cast<int32_t>(all);
         red[W + warp] = static_cast<int32_t>(wm);
     }
     __syncthreads();
-    uint32_t base = 0, tot = 0, gm = 0;
+    uint32_t base = 0, gm = 0;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-        const uint32_t s = static_cast<uint32_t>(red[w]);
-        base += w < warp ? s : 0u;
-        tot += s;
+        base += w < warp ? static_cast<uint32_t>(red[w]) : 0u;
         gm = max(gm, static_cast<uint32_t>(red[W + w]));
     }
-    total = tot;
     mx = gm;
-    return base + incl - v;
+    return base;
 }
 
 // Zeroes the counters of a CTA row of P products, which bucket_order expects to
@@ -256,7 +245,7 @@ __device__ inline uint32_t block_excl_scan_max(uint32_t v, uint32_t m, int32_t* 
 // range.
 template <int W, int ITEMS, bool SV>
 __device__ __forceinline__ void clear_buckets(RowSmem<W, ITEMS, SV>& sm, int P, int tid) {
-    uint4* b4 = reinterpret_cast<uint4*>(sm.bk + 2 * kCoarse<W>);  // coarse counters, fine counters 0 .. P
+    uint4* b4 = reinterpret_cast<uint4*>(sm.bk + kCoarse<W>);  // coarse counters, fine counters 0 .. P
     const int n4 = (kCoarse<W> + P + 4) / 4;
     for (int i = tid; i < n4; i += W * 32) b4[i] = make_uint4(0u, 0u, 0u, 0u);
 }
@@ -273,16 +262,21 @@ __device__ __forceinline__ void clear_buckets(RowSmem<W, ITEMS, SV>& sm, int P, 
 //   * the fine histogram's atomics give every product its arrival index in its
 //     bucket, so that it is placed without a second round of atomics.
 // Instruction cost per product does not grow with the column range, unlike a
-// digit pass.  Returns the largest bucket's size; above kMaxFine seqs is not
-// written.
+// digit pass.  The passes of these kernels over the shared-memory banks (74% of
+// the time busy) bound them as much as the issue slots do.  With the table in one
+// word per bucket instead of two, stored by vectors, and the scan's lanes side by
+// side: rows of 1,537-2,048 products 0.49 -> 0.46 ms, of 1,025-1,536 0.348 -> 0.338
+// (16 uneven uniform products), power-law product, all bins 8.94 -> 8.74.
+// Returns the largest bucket's size; above kMaxFine seqs is not written.
 template <int W, int ITEMS, bool SV>
 __device__ __forceinline__ uint32_t bucket_order(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits, int lane,
                                                  int warp, int tid, int& nfine) {
     constexpr int NT = W * 32;
-    uint2* info = reinterpret_cast<uint2*>(sm.bk);  // fine bucket of k = x + (k >> y)
-    uint32_t* cc = sm.bk + 2 * kCoarse<W>;          // coarse counters
-    uint32_t* fc = sm.bk + 3 * kCoarse<W>;          // fine counters, then starts
+    uint32_t* info = sm.bk;                         // first fine bucket | shift << 16
+    uint32_t* cc = sm.bk + kCoarse<W>;              // coarse counters
+    uint32_t* fc = sm.bk + 2 * kCoarse<W>;          // fine counters, then starts
     const int sc = max(nbits - kCoarseBits<W>, 0);  // column bits inside a coarse bucket
+    const uint32_t inside = (1u << sc) - 1u;
     uint32_t f[ITEMS];
     // Position i * NT + tid: whole steps past P are skipped, and no warp is left
     // with less than its share when P is below the capacity.
@@ -311,10 +305,12 @@ __device__ __forceinline__ uint32_t bucket_order(RowSmem<W, ITEMS, SV>& sm, int 
         uint32_t base = incl - sum;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            info[lane * kPer + j] = make_uint2(base - (static_cast<uint32_t>(lane * kPer + j) << bits[j]),
-                                               static_cast<uint32_t>(sc) - bits[j]);
+            bits[j] = base | (static_cast<uint32_t>(sc) - bits[j]) << 16;
             base += n[j];
         }
+#pragma unroll
+        for (int j = 0; j < kPer; j += 4)
+            *reinterpret_cast<uint4*>(info + lane * kPer + j) = make_uint4(bits[j], bits[j + 1], bits[j + 2], bits[j + 3]);
     }
     __syncwarp();
 #pragma unroll
@@ -322,42 +318,69 @@ __device__ __forceinline__ uint32_t bucket_order(RowSmem<W, ITEMS, SV>& sm, int 
         if (i * NT >= P) break;
         if (i * NT + tid < P) {
             const uint32_t k = sm.keys[i * NT + tid] - cmin;
-            const uint2 in = info[k >> sc];
-            f[i] = in.x + (k >> in.y);
+            const uint32_t in = info[k >> sc];
+            f[i] = (in & 0xffffu) + ((k & inside) >> (in >> 16));
             f[i] |= atomicAdd(&fc[f[i]], 1u) << 16;  // arrival in the high half
         }
     }
     __syncthreads();
-    // exclusive scan of the fine counters, ITEMS consecutive ones per thread
+    // exclusive scan of the fine counters, a warp's 32 * ITEMS consecutive ones by
+    // C chunks: lane l takes those from l * V of every chunk, so that its wide
+    // accesses follow the other lanes' (ITEMS consecutive ones per lane meet in a
+    // half or a quarter of the banks); two chunks share a scan
     uint32_t gmax;
     {
-        const int w0 = tid * ITEMS;
-        const bool act = w0 <= nfine;  // the bucket past the last included: its start is P
-        uint32_t x[ITEMS], sum = 0, mx = 0;
-        constexpr int V = ITEMS % 4 == 0 ? 4 : (ITEMS % 2 == 0 ? 2 : 1);
-        using Vec = std::conditional_t<V == 4, uint4, std::conditional_t<V == 2, uint2, uint32_t>>;
-        if (act) {
+        constexpr int V = ITEMS % 8 == 0 ? 4 : ITEMS, C = ITEMS / V;
+        constexpr int VL = V % 4 == 0 ? 4 : (V % 2 == 0 ? 2 : 1);  // words per access
+        static_assert(C == 1 || C % 2 == 0, "two chunks share a scan");
+        using Vec = std::conditional_t<VL == 4, uint4, std::conditional_t<VL == 2, uint2, uint32_t>>;
+        const int w0 = warp * 32 * ITEMS + lane * V;
+        uint32_t x[ITEMS], sum[C], mx = 0;
 #pragma unroll
-            for (int j = 0; j < ITEMS; j += V) *reinterpret_cast<Vec*>(x + j) = *reinterpret_cast<const Vec*>(fc + w0 + j);
+        for (int c = 0; c < C; ++c) {
+            sum[c] = 0;
+            if (w0 + c * 32 * V > nfine) continue;  // the bucket past the last is needed: its start is P
+            uint32_t* xc = x + c * V;
 #pragma unroll
-            for (int j = 0; j < ITEMS; ++j) {
-                if (w0 + j >= nfine) x[j] = 0u;  // not cleared past P
-                sum += x[j];
-                mx = max(mx, x[j]);
+            for (int j = 0; j < V; j += VL) *reinterpret_cast<Vec*>(xc + j) = *reinterpret_cast<const Vec*>(fc + w0 + c * 32 * V + j);
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                if (w0 + c * 32 * V + j >= nfine) xc[j] = 0u;  // not cleared past P
+                sum[c] += xc[j];
+                mx = max(mx, xc[j]);
             }
         }
-        uint32_t total;
-        uint32_t base = block_excl_scan_max<W>(sum, mx, sm.red, lane, warp, total, gmax);
-        if (gmax > kMaxFine) return gmax;  // uniform: every thread saw the same maximum
-        if (act) {
+        uint32_t at[C], all = 0;  // every chunk's products before the lane's; the warp's
+        if constexpr (C == 1) {
+            const uint32_t incl = warp_incl_scan(sum[0], lane);
+            at[0] = incl - sum[0];
+            all = __shfl_sync(0xffffffffu, incl, 31);
+        } else {
 #pragma unroll
-            for (int j = 0; j < ITEMS; ++j) {
-                const uint32_t n = x[j];
-                x[j] = base;
+            for (int c = 0; c < C; c += 2) {
+                const uint32_t both = sum[c] | sum[c + 1] << 16;
+                const uint32_t incl = warp_incl_scan(both, lane), tot = __shfl_sync(0xffffffffu, incl, 31);
+                at[c] = all + ((incl - both) & 0xffffu);
+                all += tot & 0xffffu;
+                at[c + 1] = all + ((incl - both) >> 16);
+                all += tot >> 16;
+            }
+        }
+        const uint32_t before = block_warps_before<W>(all, mx, sm.red, lane, warp, gmax);
+        if (gmax > kMaxFine) return gmax;  // uniform: every thread saw the same maximum
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            if (w0 + c * 32 * V > nfine) continue;
+            uint32_t* xc = x + c * V;
+            uint32_t base = before + at[c];
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const uint32_t n = xc[j];
+                xc[j] = base;
                 base += n;
             }
 #pragma unroll
-            for (int j = 0; j < ITEMS; j += V) *reinterpret_cast<Vec*>(fc + w0 + j) = *reinterpret_cast<const Vec*>(x + j);
+            for (int j = 0; j < V; j += VL) *reinterpret_cast<Vec*>(fc + w0 + c * 32 * V + j) = *reinterpret_cast<const Vec*>(xc + j);
         }
         if (tid == 0 && nfine == W * 32 * ITEMS) fc[nfine] = static_cast<uint32_t>(P);
     }
@@ -380,7 +403,7 @@ __device__ __forceinline__ uint32_t bucket_order(RowSmem<W, ITEMS, SV>& sm, int 
 template <int W, int ITEMS, bool SV>
 __device__ __forceinline__ void warp_share(const RowSmem<W, ITEMS, SV>& sm, int P, int nfine, int lane, int warp, int& x0,
                                            int& x1) {
-    const uint32_t* fc = sm.bk + 3 * kCoarse<W>;
+    const uint32_t* fc = sm.bk + 2 * kCoarse<W>;
     const int share = (P + W - 1) / W;
     const int half = lane >> 4, l = lane & 15;
     const int m = (warp + half) * share;
@@ -503,6 +526,28 @@ __device__ __forceinline__ void radix_sort_row(RowSmem<W, ITEMS, SV>& sm, int P,
 
 constexpr uint32_t kDeadKey = 0xffffffffu;
 
+// The words of a sorted region, lane l's at keys[l * N ...].  kWhole: the region has
+// room for all 32 * N words and starts at 16 bytes, so that they go in the widest
+// stores: one word at a time the lanes meet in a bank N-fold for N = 4, 8 and 16
+// (rows of 385-512 products: 0.50 -> 0.45 ms, 65,536 rows of 256: 0.146 -> 0.140).
+// A share of a CTA row has an even N twice an odd number: two lanes meet, and pairs
+// of words, with the shares moved to even words, measured 2-7% slower.
+template <int N, bool kWhole>
+__device__ __forceinline__ void store_words(const uint32_t (&k)[N], uint32_t* keys, int n, int lane) {
+    uint32_t* to = keys + lane * N;
+    if constexpr (kWhole && N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) *reinterpret_cast<uint4*>(to + i) = make_uint4(k[i], k[i + 1], k[i + 2], k[i + 3]);
+    } else if constexpr (kWhole && N % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) *reinterpret_cast<uint2*>(to + i) = make_uint2(k[i], k[i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (kWhole || lane * N + i < n) to[i] = k[i];
+    }
+}
+
 // Step 3 of a sorted region of n positions, by one warp: lane l holds the words
 // (column offset << S | sequence number) of positions l * N ... in k.  Stores
 // them at keys[0..n), sums every run of equal column offsets in product order
@@ -511,7 +556,7 @@ constexpr uint32_t kDeadKey = 0xffffffffu;
 // more than one product are first listed (list: n 16-bit words), so that the
 // warp sums 32 of them at a time: an FP64 instruction takes 16 cycles of an SM
 // whether one lane needs it or all.
-template <int N, int S>
+template <int N, int S, bool kWhole>
 __device__ __forceinline__ void fold_runs(const uint32_t (&k)[N], uint32_t* keys, uint16_t* list, double* vals, int n,
                                           int lane) {
     using Mask = std::conditional_t<(N < 32), uint32_t, unsigned long long>;
@@ -521,8 +566,8 @@ __device__ __forceinline__ void fold_runs(const uint32_t (&k)[N], uint32_t* keys
     for (int i = 0; i < N; ++i) {
         const uint32_t p = i ? k[i - 1] : before;
         if (((k[i] ^ p) >> S) == 0u) same |= Mask{1} << i;
-        if (lane * N + i < n) keys[lane * N + i] = k[i];
     }
+    store_words<N, kWhole>(k, keys, n, lane);
     if (lane == 0) same &= ~Mask{1};
     const int mine = min(max(n - lane * N, 0), N);
     same &= (Mask{1} << mine) - 1;
@@ -749,7 +794,7 @@ __device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITE
         }
         warp_sort(k, lane);
         __syncwarp();
-        fold_runs<ITEMS, kSeqBits>(k, sm.keys, sm.seqs, vals, P, lane);
+        fold_runs<ITEMS, kSeqBits, true>(k, sm.keys, sm.seqs, vals, P, lane);
         int32_t* oc = out.c_col + out.out0;
         double* ov = out.c_val + out.out0;
         kept = out.holes ? write_slots<kSeqBits>(sm.keys, vals, P, cmin, oc, ov, lane)
@@ -813,7 +858,7 @@ __device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITE
                 } else {
                     settle(k, static_cast<int>(biggest), lane);
                     if (out.holes || range < kMaxRange) {  // exact layout: no warp of the row is wide
-                        fold_runs<N, kSeqBits>(k, keys, seqs, vals, n, lane);
+                        fold_runs<N, kSeqBits, false>(k, keys, seqs, vals, n, lane);
                         if (!out.holes) {
                             const int32_t all = write_share<W, kSeqBits>(keys, vals, n, first, out.c_col + out.out0,
                                                                          out.c_val + out.out0, sm.red, lane, warp);
