@@ -69,11 +69,22 @@ __device__ __noinline__ uint32_t finish_wide_row(uint32_t* cols, uint16_t* seqs,
     return kept;
 }
 
+template <typename T>
+__device__ __forceinline__ T* shfl_ptr(T* p, int lane) {
+    return reinterpret_cast<T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), lane));
+}
+
 // G rows of at most 32 * I products per warp.  A row this short leaves a warp
 // that works on it alone waiting: five dependent loads (work item, offsets of A,
 // A entry, offsets of B, B entry) for some ten instructions per product.  Here
 // the rows' segments share the lanes of one enumeration and the rows' sorts, one
-// register (or I) per row, are independent chains.  When: launch_numeric_warp.
+// register (or I) per row, are independent chains.  The passes over the L1 banks
+// bound it then (80-88% of the time busy: B's offsets, columns and values lie in
+// lines of their own for every segment, the shuffles and shared memory take the
+// rest), so a row's first segment, result pointers and run marks stay in the lane
+// that has them: 262,144 rows of 32 products 0.205 -> 0.189 ms, of 56 products
+// 0.163 -> 0.159, against every lane holding all rows' segments and reading the
+// job again per row.  When: launch_numeric_warp.
 template <int I, int G>
 __global__ void __launch_bounds__(kWarpKernelThreads, 4)
 num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count,
@@ -96,7 +107,11 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
         // lane g: row g
         const Job* J = jobs;
         int row = 0, P = 0;
-        int64_t a0 = 0, nseg = 0, out0 = 0;
+        int64_t a0 = 0, nseg = 0;
+        int32_t* out_col = nullptr;
+        double* out_val = nullptr;
+        uint32_t ncols = 0;
+        bool slots = false;  // upper-bound layout
         if (lane < G && i0 + lane < count) {
             const int64_t it = items[i0 + lane];
             J = jobs + item_job(it);
@@ -104,7 +119,11 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
             P = static_cast<int>(J->ub[row]);
             a0 = J->A.rp[row];
             nseg = J->A.rp[row + 1] - a0 + (J->S.rp ? 1 : 0);
-            out0 = J->cnt[row];
+            const int64_t out0 = J->cnt[row];
+            out_col = J->c_col + out0;
+            out_val = J->c_val + out0;
+            ncols = static_cast<uint32_t>(J->B.cols);
+            slots = J->holes != 0;
         }
         int p_incl = P;
         int64_t s_incl = nseg;
@@ -118,23 +137,22 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
             }
         }
         const int64_t all_seg = __shfl_sync(0xffffffffu, s_incl, G - 1);
-        int64_t seg0[G];  // first segment of every row
-#pragma unroll
-        for (int g = 0; g < G; ++g) seg0[g] = __shfl_sync(0xffffffffu, s_incl - nseg, g);
+        const int64_t seg0 = s_incl - nseg;  // the row's first segment
+        const unsigned slot_rows = __ballot_sync(0xffffffffu, slots);
         const int row_delta = lane * Sm::kRow - (p_incl - P);
 
         // 1. the rows' products into shared memory (team_row_products for G rows)
         int done = 0;
         for (int64_t e0 = 0; e0 < all_seg; e0 += 32) {
             const int64_t e = e0 + lane;
-            int g = 0;
-            int64_t first = 0;
-#pragma unroll
-            for (int h = 1; h < G; ++h)
-                if (seg0[h] <= e) {
-                    g = h;
-                    first = seg0[h];
-                }
+            // the rows that start before the batch, and in it up to this segment (a
+            // row of the list has a segment: the last of them is the segment's)
+            const int64_t in_batch = seg0 - e0;
+            const unsigned starts_here =
+                __reduce_or_sync(0xffffffffu, nseg > 0 && in_batch >= 0 && in_batch < 32 ? 1u << in_batch : 0u);
+            const int earlier = __popc(__ballot_sync(0xffffffffu, nseg > 0 && in_batch < 0));
+            const int g = earlier + __popc(starts_here & (le_above0 | 1u)) - 1;
+            const int64_t first = __shfl_sync(0xffffffffu, seg0, g);
             const Job* Jg = reinterpret_cast<const Job*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(J), g));
             const int row_g = __shfl_sync(0xffffffffu, row, g);
             const int64_t a0_g = __shfl_sync(0xffffffffu, a0, g);
@@ -209,8 +227,7 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const int Pg = __shfl_sync(0xffffffffu, P, g);
-            const uint32_t ncols = static_cast<uint32_t>(
-                reinterpret_cast<const Job*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(J), g))->B.cols);
+            const uint32_t ncols_g = __shfl_sync(0xffffffffu, ncols, g);
             uint32_t lo = 0xffffffffu, hi = 0;
 #pragma unroll
             for (int i = 0; i < I; ++i) {
@@ -218,7 +235,7 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
                 k[g * I + i] = 0u;
                 if (p < Pg) {
                     uint32_t c = sm.keys[g * Sm::kRow + p];
-                    if (c >= ncols) {  // negative columns included
+                    if (c >= ncols_g) {  // negative columns included
                         raise_error(err, kErrInvalid, 4, static_cast<int32_t>(c));
                         c = 0;
                         sm.keys[g * Sm::kRow + p] = 0u;
@@ -233,11 +250,11 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
             if (lane == g) cmin = lo;
             const bool wide = Pg > 0 && hi - lo >= kMaxRange;
             if (wide) {
-                const Job* Jg = reinterpret_cast<const Job*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(J), g));
-                const int64_t o = __shfl_sync(0xffffffffu, out0, g);
+                int32_t* oc = shfl_ptr(out_col, g);
+                double* ov = shfl_ptr(out_val, g);
                 __syncwarp();
                 const uint32_t n = finish_wide_row<I>(sm.keys + g * Sm::kRow, sm.list + g * Sm::kRow, sm.vals + g * Sm::kRow,
-                                                      Pg, Jg->c_col + o, Jg->c_val + o, Jg->holes != 0, lane);
+                                                      Pg, oc, ov, (slot_rows >> g & 1u) != 0, lane);
                 if (lane == g) {
                     kept = n;
                     P = 0;
@@ -252,6 +269,7 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
         for (int g = 0; g < G; ++g) warp_sort(reinterpret_cast<uint32_t(&)[I]>(k[g * I]), lane);
         __syncwarp();
 
+        uint32_t same;  // see 3.
         // 3. runs of equal columns (fold_runs over all rows): bit g * I + i of `same`
         //    is position lane * I + i of row g
         {
@@ -260,7 +278,7 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
                 for (int g = 0; g < G; ++g) m |= 1u << (g * I);
                 return m;
             }();
-            uint32_t same = 0;
+            same = 0;
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 const uint32_t before = __shfl_up_sync(0xffffffffu, k[g * I + I - 1], 1);
@@ -294,7 +312,7 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
                         const uint32_t other = sm.keys[q];
                         if ((other ^ key) >> S) break;
                         acc = __dadd_rn(acc, vals[other & kSeq]);
-                        sm.keys[q] = kDeadKey;
+                        if constexpr (I > 1) sm.keys[q] = kDeadKey;
                     }
                     vals[key & kSeq] = acc;
                 }
@@ -307,17 +325,18 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
         for (int g = 0; g < G; ++g) {
             const int Pg = __shfl_sync(0xffffffffu, P, g);
             if (Pg == 0) continue;
-            const Job* Jg = reinterpret_cast<const Job*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(J), g));
-            const int64_t o = __shfl_sync(0xffffffffu, out0, g);
             const uint32_t lo = __shfl_sync(0xffffffffu, cmin, g);
-            int32_t* __restrict__ oc = Jg->c_col + o;
-            double* __restrict__ ov = Jg->c_val + o;
-            const bool holes = Jg->holes != 0;
+            int32_t* __restrict__ oc = shfl_ptr(out_col, g);
+            double* __restrict__ ov = shfl_ptr(out_val, g);
+            const bool holes = (slot_rows >> g & 1u) != 0;
             int n = 0;
 #pragma unroll
             for (int i = 0; i < I; ++i) {
                 const int p = i * 32 + lane;
-                const uint32_t key = p < Pg ? sm.keys[g * Sm::kRow + p] : kDeadKey;
+                // (one word a lane: position lane, whose word the lane holds)
+                const uint32_t key = I == 1   ? (same >> g & 1u ? kDeadKey : k[g])
+                                     : p < Pg ? sm.keys[g * Sm::kRow + p]
+                                              : kDeadKey;
                 const double v = key != kDeadKey ? sm.vals[g * Sm::kRow + (key & kSeq)] : 0.0;
                 const bool keep = nonzero(v);
                 const unsigned m = __ballot_sync(0xffffffffu, keep);
