@@ -633,6 +633,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
                         products <= (transient ? kDirectTransient : kDirectProducts);
     int32_t* k5_col = nullptr;
     double* k5_val = nullptr;
+    int64_t* h_starts = nullptr;
     if (direct) {
         k5_col = ar.alloc<int32_t>(static_cast<size_t>(products), "C col (compact)");
         k5_val = ar.alloc<double>(static_cast<size_t>(products), "C val (compact)");
@@ -642,11 +643,16 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
         check_cuda(cudaGetLastError(), "K5 launch");
         cudaEventRecord(h->ev[5], st);
+    } else if (njobs > 1) {
+        launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
+        h_starts = static_cast<int64_t*>(host_staging(h, sizeof(int64_t) * njobs));
+        launch_starts(nz, d_row_base, h_starts, njobs, st, readback_of(d_ctrl, hc, offsetof(Ctrl, cursor)));
+        launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
     } else {
         launch_readback(d_ctrl, hc, sizeof(Ctrl), st);
         ++launches;
     }
-    sync(h);  // stored count and errors
+    sync(h);  // stored count, errors and every product's first offset
     if (hc->err.code) {
         std::string msg;
         const spg_status s = map_err(hc->err, msg);
@@ -690,18 +696,6 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         // directly (row r of product j at its offset minus the product's first
         // offset): the entries of C are moved once, not compacted and then
         // copied out of one flat array.
-        launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
-        std::vector<int64_t> idx(njobs);
-        for (int j = 0; j < njobs; ++j) idx[j] = row_base[j] + j;
-        int64_t* d_idx = ar.alloc<int64_t>(static_cast<size_t>(njobs), "start index");
-        int64_t* d_starts = ar.alloc<int64_t>(static_cast<size_t>(njobs), "starts");
-        check_cuda(cudaMemcpyAsync(d_idx, idx.data(), sizeof(int64_t) * njobs, cudaMemcpyHostToDevice, st),
-                   "H2D start index");
-        launch_gather(nz, d_idx, d_starts, njobs, st);
-        int64_t* h_starts = static_cast<int64_t*>(host_staging(h, sizeof(int64_t) * njobs));
-        launch_readback(d_starts, h_starts, sizeof(int64_t) * njobs, st);
-        launches += scan_launches(static_cast<int64_t>(slots) - 1) + 2;
-        sync(h);  // every product's first offset: the sizes of its arrays
         std::vector<int64_t> starts(h_starts, h_starts + njobs);
         starts.push_back(nz_total);
         std::vector<RebaseItem> rb(njobs);
@@ -740,7 +734,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
             ar.release(r.ci);
             ar.release(r.v);
         }
-        sync(h);  // jobs, idx and rb must outlive their copies
+        sync(h);  // rb must outlive its copy
     }
     for (int j = 0; j < njobs; ++j) out[j].products = job_products[j];
     if (!direct) sync(h);
@@ -1669,12 +1663,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     p->col = plan_alloc<int32_t>(p, static_cast<size_t>(products), "plan C col");
     p->val = plan_alloc<double>(p, static_cast<size_t>(products), "plan C val");
     p->rp = plan_alloc<int64_t>(p, slots, "plan C row_ptr");
-    std::vector<int64_t> idx(n);
-    for (int j = 0; j < n; ++j) idx[j] = p->row_base[j] + j;
-    int64_t* d_idx = plan_alloc<int64_t>(p, static_cast<size_t>(n), "plan start index");
-    int64_t* d_starts = plan_alloc<int64_t>(p, static_cast<size_t>(n), "plan starts");
-    check_cuda(cudaMemcpyAsync(d_idx, idx.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, st), "H2D");
-    sync(h);  // idx, jobs copied
+    sync(h);  // jobs copied
     int64_t max_rows = 0;
     for (int32_t r : p->rows) max_rows = std::max<int64_t>(max_rows, r);
 
@@ -1688,11 +1677,10 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     // (the bins' fork and join are part of the graph)
     launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, true, false);
     launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
-    launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, items, bin_off, p->col, p->val, st);
-    launch_gather(nz, d_idx, d_starts, n, st);
+    launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, items, bin_off, p->col, p->val, st,
+                         readback_of(d_ctrl, p->hc, offsetof(Ctrl, cursor)));
+    launch_starts(nz, d_row_base, p->h_starts, n, st);
     launch_rebase_jobs(nz, p->rp, d_row_base, n, max_rows, st);
-    launch_readback(d_starts, p->h_starts, sizeof(int64_t) * n, st);
-    launch_readback(d_ctrl, p->hc, sizeof(Ctrl), st);
     const cudaError_t le = cudaGetLastError();
     const cudaError_t ce = cudaStreamEndCapture(st, &p->graph);
     h->blocks->set_capturing(false);

@@ -486,9 +486,11 @@ compact_holes_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __r
     }
 }
 
-__global__ void gather_kernel(const int64_t* __restrict__ src, const int64_t* __restrict__ idx,
-                              int64_t* __restrict__ dst, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[idx[i]];
+__global__ void starts_kernel(const int64_t* __restrict__ scanned, const int64_t* __restrict__ job_row_base, int64_t* dst,
+                              int njobs, const Readback read) {
+    read_back(read);
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < njobs; j += gridDim.x * blockDim.x)
+        dst[j] = scanned[job_row_base[j] + j];
 }
 
 // Small device->host reads by a kernel storing into mapped page-locked memory:
@@ -601,7 +603,10 @@ void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row
                           int64_t slots, const int64_t* items, const int64_t* bin_off, int32_t* out_col,
                           double* out_val, cudaStream_t stream, const Readback& read, const Stats* full,
                           const ErrWord* err) {
-    if (total_rows <= 0) return;
+    if (total_rows <= 0) {
+        if (read.words) launch_readback(read.src, read.dst, static_cast<size_t>(read.words) * 8, stream);
+        return;
+    }
     const int64_t n_long = bin_off[kNumBins] - bin_off[kLongBin];
     const int long_ctas = static_cast<int>(std::min<int64_t>(n_long, 152 * 8));
     // Rows per warp: about two steps of 256 slots.
@@ -612,9 +617,10 @@ void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row
         out_val, read, full, slots, err);
 }
 
-void launch_gather(const int64_t* d_src, const int64_t* d_idx, int64_t* d_dst, int n, cudaStream_t stream) {
-    if (n <= 0) return;
-    gather_kernel<<<grid_for(n, 256, 1024), 256, 0, stream>>>(d_src, d_idx, d_dst, n);
+void launch_starts(const int64_t* d_scanned, const int64_t* d_job_row_base, int64_t* dst, int njobs,
+                   cudaStream_t stream, const Readback& read) {
+    if (njobs <= 0) return;
+    starts_kernel<<<grid_for(njobs, 256, 1024), 256, 0, stream>>>(d_scanned, d_job_row_base, dst, njobs, read);
 }
 
 void launch_job_products(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t* d_out,

@@ -299,15 +299,16 @@ void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row
                           int64_t slots, const int64_t* items, const int64_t* bin_off, int32_t* out_col,
                           double* out_val, cudaStream_t stream, const Readback& read = {},
                           const Stats* full = nullptr, const ErrWord* err = nullptr);
-// Batched results: dst[i] = src[idx[i]], and the offsets of every product from
-// those of the whole batch.
+// Batched results: every product's first offset (dst may be page-locked host
+// memory), and the offsets of every product from those of the whole batch.
 struct RebaseItem {
     int64_t* rp;         // rows + 1 offsets of one product
     const int64_t* src;  // the same in the batch
     int64_t start;       // subtracted from every offset
     int64_t rows;
 };
-void launch_gather(const int64_t* d_src, const int64_t* d_idx, int64_t* d_dst, int n, cudaStream_t stream);
+void launch_starts(const int64_t* d_scanned, const int64_t* d_job_row_base, int64_t* dst, int njobs,
+                   cudaStream_t stream, const Readback& read = {});
 void launch_rebase(const RebaseItem* d_items, int n, int64_t max_rows, cudaStream_t stream);
 // GPU validator (k_validate.cu).
 size_t validate_cell_bytes();
