@@ -166,6 +166,19 @@ num_rows_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
             const uint32_t incl = warp_incl_scan(static_cast<uint32_t>(len) | (len > 0 ? 0x10000u : 0u), lane);
             const int total = static_cast<int>(__shfl_sync(0xffffffffu, incl, 31) & 0xffffu);
             const uint32_t s = (incl & 0xffffu) - static_cast<uint32_t>(len);
+            // B's rows hold one entry (an aggregation's prolongation): every lane has
+            // its product, without the table (262,144 rows of 32 products: 0.189 ->
+            // 0.156 ms)
+            if (__all_sync(0xffffffffu, len <= 1)) {
+                if (len > 0) {
+                    const int at = static_cast<int>(s) + delta_g + done;
+                    sm.keys[at] = static_cast<uint32_t>(__ldg(cp));
+                    sm.vals[at] = __dmul_rn(sc, __ldg(vp));
+                }
+                done += total;
+                __syncwarp();
+                continue;
+            }
             if (len > 0) {
                 const uint32_t r = (incl >> 16) - 1u;
                 sm.colb[r] = reinterpret_cast<uint64_t>(cp) - 4u * static_cast<uint64_t>(s);
