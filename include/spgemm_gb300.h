@@ -12,7 +12,9 @@
  * bit-identical to the reference's serialSpgemm and spgemm().
  *
  * Threading: a handle owns one CUDA stream and its workspace; calls on one
- * handle must not overlap.  Use one handle per host thread.
+ * handle must not overlap.  Use one handle per host thread.  A handle keeps the
+ * device memory its calls free for its next calls (the handles of a device at most
+ * 1/16 of its memory between them); spg_destroy gives it back.
  *
  * Errors: every call returns an spg_status; spg_last_error(handle) gives the
  * message of the last failure on that handle.  include/spgemm_gb300.hpp maps
@@ -75,14 +77,18 @@ typedef struct {
  * its scalar-product count and compacts once (12 bytes of scratch per product,
  * one pass over the products); EXACT first counts every row's distinct columns
  * (a second pass over the products, no scratch); AUTO picks UPPER_BOUND unless
- * its scratch would exceed the budget or half of the free device memory. */
+ * its scratch would exceed the budget or half of the free device memory (looked
+ * at above 2 GiB; below, EXACT follows if an allocation fails).  C's device arrays
+ * may be larger than C, up to 12 bytes per scalar product for calls of at most
+ * 2^22 of them. */
 typedef enum { SPG_MODE_AUTO = 0, SPG_MODE_EXACT = 1, SPG_MODE_UPPER_BOUND = 2 } spg_mode;
 
 typedef struct {
     int32_t device;             /* CUDA device ordinal */
     int32_t mode;               /* spg_mode */
     uint64_t hbm_budget_bytes;  /* largest device footprint a request may reserve; 0 = no limit */
-    int32_t bin_streams;        /* streams the numeric bins of one call spread over: 1, or 3 (0 = 3) */
+    int32_t bin_streams;        /* 1: the numeric bins of a call run one after the other on its
+                                 * stream; 3 or 0: spread over several */
     int32_t reserved;
 } spg_config;
 
@@ -94,8 +100,8 @@ typedef struct {
                                     768, 1024, 1536, 2048, 3072, 4096, 6144, 8192, 12288, 16384, heavier */
     int64_t launches;            /* kernels this library launched for the call */
     float ms_numeric_bin[20];    /* per bin (same order as bin_rows): time from the start of the numeric
-                                    phase to the end of the bin's launch (bins run on three streams at
-                                    once); spg_tune runs them one after the other and times each */
+                                    phase to the end of the bin's launch (bins run on several streams
+                                    at once); spg_tune runs them one after the other and times each */
 } spg_timings;
 
 typedef struct spg_handle spg_handle;

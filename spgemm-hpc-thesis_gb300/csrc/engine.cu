@@ -1,10 +1,11 @@
 // Host side of the GB300 SpGEMM engine and its C ABI (include/spgemm_gb300.h).
 //
-// One call runs the phases on the handle's stream:
-//   stage operands -> K1 row work + bins -> [sync: bin sizes, errors]
-//   -> K2 symbolic per bin -> K3 scan -> [sync: C size] -> allocate C
-//   -> K4 numeric per bin -> [sync: stored count, errors]
-//   -> (K5 compaction only if some sum was an exact zero) -> result.
+// One call runs the phases on the handle's stream (K2 and K4 on several, BinStreams):
+//   upper-bound layout: stage operands -> K1 row work + bins, K3 scan -> [wait: bin
+//   sizes, errors] -> allocate C_tmp -> K4 numeric per bin -> [wait: stored count,
+//   errors; not for small calls] -> K5 compaction if some slot holds no entry -> result;
+//   exact layout: K1 -> [wait] -> K2 symbolic per bin -> K3 -> [wait: C's size] ->
+//   allocate C -> K4 -> [wait] -> (K5 only if some sum was an exact zero) -> result.
 // All rows of all products of a call are flattened into one set of bin lists,
 // so a batch of products costs the same number of launches as one product.
 // Device memory comes from the handle's kept blocks (blocks.h) and the device's

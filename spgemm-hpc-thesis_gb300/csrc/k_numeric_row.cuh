@@ -23,9 +23,10 @@
 // CTA with the keys in shared memory and the values in shared memory or a
 // per-CTA global slab (num_block_kernel).  Heavier rows are split by column
 // range into pieces that run on the same pipeline (num_piece_kernel) in the
-// upper-bound layout; in the exact layout rows of <= 16384 run one per CTA with
-// a value slab and heavier ones with the whole sort in a global slab
-// (num_heavy_kernel, k_numeric.cu).
+// upper-bound layout, and in the exact layout where memory allows (else rows of
+// <= 16384 run one per CTA with a value slab and heavier ones with the whole sort in
+// a global slab, num_heavy_kernel, k_numeric.cu).  Many rows of <= 64 products run
+// several per warp (num_rows_kernel, k_numeric_warp.cu).
 #pragma once
 
 #include <atomic>
