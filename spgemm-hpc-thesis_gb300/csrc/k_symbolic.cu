@@ -9,6 +9,13 @@
 //   * rows of <= 512 products: one warp per row, table in shared memory;
 //   * rows of <= 16384 products: one CTA per row, table in shared memory;
 //   * heavier rows: one CTA per row, table in a global-memory slab per CTA.
+// Where a bit per column of B takes at most twice the words of the bin's table, the
+// table is a bitmap: one atomic per product instead of a hash, a compare-and-swap and
+// its retries.  Column c is bit c / words of word c % words, so that neighbouring
+// columns lie in neighbouring banks.  A heavier row's bitmap is in shared memory up to
+// 2^20 columns.  K2 of power-law squares of 65,536, 131,071 and 262,144 rows: 304 ->
+// 187, 541 -> 395 and 1,076 -> 870 us; with the line at the table's size 200, 417 and
+// 918, at four times it 187, 444 and 946 (fewer CTAs per SM, more words to clear).
 // Every launch reserves the tables of its bin's largest row only (a power of
 // two >= twice the bin capacity), so that the bins of short rows keep many
 // CTAs per SM.  It also rejects B columns outside [0, B.cols).
@@ -52,10 +59,41 @@ __device__ inline int hash_insert(int32_t* tab, uint32_t mask, int log2t, int32_
     }
 }
 
+// log2 of the words of a bitmap of `cols` columns.
+__host__ __device__ inline int bitmap_log2(int64_t cols) {
+    const int l = ceil_log2(cols) - 5;
+    return l > 0 ? l : 0;
+}
+
+// Sets column col's bit in a bitmap of 2^log2w words; returns 1 if it was not set.
+__device__ inline int bitmap_insert(uint32_t* map, int log2w, int32_t col) {
+    const uint32_t bit = 1u << (static_cast<uint32_t>(col) >> log2w);
+    return (atomicOr(&map[static_cast<uint32_t>(col) & ((1u << log2w) - 1u)], bit) & bit) == 0u;
+}
+
+constexpr int kMaxBitmapLog2 = 15;  // 128 KiB of shared memory
+
+// log2 of the words reserved per row of a bin: the table's, or a bitmap's of up to
+// twice as many.
+int reserved_log2(int bin, int64_t max_cols) {
+    const int slots = sym_table_slots(bin), map = bitmap_log2(max_cols);
+    return map <= kMaxBitmapLog2 && (1 << map) <= 2 * slots ? std::max(map, ceil_log2(slots)) : ceil_log2(slots);
+}
+
+template <int NT>
+__device__ inline void clear_words(int32_t* tab, uint32_t n, int tid, int32_t value) {
+    if (n >= 4 * NT) {
+        for (uint32_t s = 4 * tid; s < n; s += 4 * NT) *reinterpret_cast<int4*>(tab + s) = make_int4(value, value, value, value);
+    } else {
+        for (uint32_t s = tid; s < n; s += NT) tab[s] = value;
+    }
+}
+
 __global__ void __launch_bounds__(kSymWarpThreads)
 sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count, int tiny,
-                int wtab, ErrWord* __restrict__ err) {
-    extern __shared__ int32_t s_dyn[];  // kSymWarpThreads / 32 tables of wtab slots
+                int wtab_log2, ErrWord* __restrict__ err) {
+    extern __shared__ __align__(16) int32_t s_dyn[];  // kSymWarpThreads / 32 tables of wtab slots
+    const int wtab = 1 << wtab_log2;
     __shared__ RowSegs<32, 512> s_seg[kSymWarpThreads / 32];  // rows of at most 512 products
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (kSymWarpThreads / 32);
@@ -83,11 +121,14 @@ sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
             const int log2t = max(6, ceil_log2(2 * ub));
             const uint32_t tsize = 1u << log2t, mask = tsize - 1;
             int32_t* tab = s_dyn + w * wtab;
-            for (uint32_t s = lane; s < tsize; s += 32) tab[s] = -1;
+            const int log2w = bitmap_log2(J.B.cols);
+            const bool bits = log2w <= wtab_log2;
+            clear_words<32>(tab, bits ? 1u << log2w : tsize, lane, bits ? 0 : -1);
             __syncwarp();
             int mine = 0;
             team_row_products<32, 512, 4, false>(J, row, s_seg[w], nullptr, lane, [&](int32_t, int32_t c, double, double) {
-                if (col_ok(c, J.B.cols, err)) mine += hash_insert(tab, mask, log2t, c);
+                if (!col_ok(c, J.B.cols, err)) return;
+                mine += bits ? bitmap_insert(reinterpret_cast<uint32_t*>(tab), log2w, c) : hash_insert(tab, mask, log2t, c);
             });
             found = warp_sum(mine);
             __syncwarp();
@@ -99,8 +140,8 @@ sym_warp_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items,
 template <int NT, int CAP>
 __global__ void __launch_bounds__(NT)
 sym_block_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count,
-                 ErrWord* __restrict__ err) {
-    extern __shared__ int32_t s_tab[];  // the bin's table slots
+                 int tab_log2, ErrWord* __restrict__ err) {
+    extern __shared__ __align__(16) int32_t s_tab[];  // 2^tab_log2 words
     __shared__ RowSegs<NT, CAP> s_seg;
     __shared__ int64_t s_warp[NT / 32 + 1];
     __shared__ int s_found;
@@ -110,12 +151,15 @@ sym_block_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items
         const int row = item_row(it);
         const int log2t = max(6, ceil_log2(2 * J.ub[row]));
         const uint32_t tsize = 1u << log2t, mask = tsize - 1;
-        for (uint32_t s = threadIdx.x; s < tsize; s += NT) s_tab[s] = -1;
+        const int log2w = bitmap_log2(J.B.cols);
+        const bool bits = log2w <= tab_log2;
+        clear_words<NT>(s_tab, bits ? 1u << log2w : tsize, threadIdx.x, bits ? 0 : -1);
         if (threadIdx.x == 0) s_found = 0;
         __syncthreads();
         int mine = 0;
         team_row_products<NT, CAP, 4, false>(J, row, s_seg, s_warp, threadIdx.x, [&](int32_t, int32_t c, double, double) {
-            if (col_ok(c, J.B.cols, err)) mine += hash_insert(s_tab, mask, log2t, c);
+            if (!col_ok(c, J.B.cols, err)) return;
+            mine += bits ? bitmap_insert(reinterpret_cast<uint32_t*>(s_tab), log2w, c) : hash_insert(s_tab, mask, log2t, c);
         });
         mine = warp_sum(mine);
         if ((threadIdx.x & 31) == 0) atomicAdd(&s_found, mine);
@@ -127,7 +171,8 @@ sym_block_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items
 
 __global__ void __launch_bounds__(kSymHeavyThreads)
 sym_heavy_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count,
-                 int32_t* __restrict__ slabs, int64_t slab_slots, ErrWord* __restrict__ err) {
+                 int32_t* __restrict__ slabs, int64_t slab_slots, int map_log2, ErrWord* __restrict__ err) {
+    extern __shared__ __align__(16) int32_t s_map[];  // 2^map_log2 words
     __shared__ SegTab<kSymHeavyThreads> s_seg;
     __shared__ int64_t s_warp[kSymHeavyThreads / 32 + 1];
     __shared__ unsigned long long s_found;
@@ -138,13 +183,16 @@ sym_heavy_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items
         const int row = item_row(it);
         const int log2t = ceil_log2(2 * J.ub[row]);
         const uint32_t tsize = 1u << log2t, mask = tsize - 1;
-        for (uint32_t s = threadIdx.x; s < tsize; s += kSymHeavyThreads) tab[s] = -1;
+        const int log2w = bitmap_log2(J.B.cols);
+        const bool bits = log2w <= map_log2;
+        clear_words<kSymHeavyThreads>(bits ? s_map : tab, bits ? 1u << log2w : tsize, threadIdx.x, bits ? 0 : -1);
         if (threadIdx.x == 0) s_found = 0;
         __syncthreads();
         int mine = 0;
         team_products<kSymHeavyThreads, false>(J, row, s_seg, s_warp, threadIdx.x,
                                                [&](int64_t, int32_t c, double, double) {
-            if (col_ok(c, J.B.cols, err)) mine += hash_insert(tab, mask, log2t, c);
+            if (!col_ok(c, J.B.cols, err)) return;
+            mine += bits ? bitmap_insert(reinterpret_cast<uint32_t*>(s_map), log2w, c) : hash_insert(tab, mask, log2t, c);
         });
         mine = warp_sum(mine);
         if ((threadIdx.x & 31) == 0) atomicAdd(&s_found, static_cast<unsigned long long>(mine));
@@ -170,30 +218,41 @@ size_t symbolic_scratch_bytes(const int64_t* bin_count, int64_t max_ub, int num_
 }
 
 void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
-                     void* d_scratch, size_t, Stats*, ErrWord* d_err, cudaStream_t stream, int num_sms) {
+                     int64_t max_cols, void* d_scratch, size_t, Stats*, ErrWord* d_err, cudaStream_t stream, int num_sms) {
     if (count <= 0) return;
     if (bin <= kLastWarpBin) {
-        const int wtab = sym_table_slots(bin);
-        const int smem = (kSymWarpThreads / 32) * wtab * static_cast<int>(sizeof(int32_t));
-        cudaFuncSetAttribute(sym_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const int wtab_log2 = reserved_log2(bin, max_cols);
+        const int smem = (kSymWarpThreads / 32) * (4 << wtab_log2);
+        allow_smem<sym_warp_kernel>((kSymWarpThreads / 32) * 4 * 2 * sym_table_slots(kLastWarpBin));
         const int grid = capped_grid(count, kSymWarpThreads / 32, num_sms * 32);
-        sym_warp_kernel<<<grid, kSymWarpThreads, smem, stream>>>(d_jobs, d_items, count, bin == 1, wtab, d_err);
+        sym_warp_kernel<<<grid, kSymWarpThreads, smem, stream>>>(d_jobs, d_items, count, bin == 1, wtab_log2, d_err);
     } else if (bin <= kLastSymSmemBin) {
-        const int smem = sym_table_slots(bin) * static_cast<int>(sizeof(int32_t));
+        const int tab_log2 = reserved_log2(bin, max_cols);
+        const int smem = 4 << tab_log2;
         auto run = [&](auto kernel, int nt) {
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            kernel<<<capped_grid(count, 1, num_sms * (2048 / nt)), nt, smem, stream>>>(d_jobs, d_items, count, d_err);
+            kernel<<<capped_grid(count, 1, num_sms * (2048 / nt)), nt, smem, stream>>>(d_jobs, d_items, count, tab_log2, d_err);
         };
         // CTA size by row size: 6-12 products per thread on the bins below 4096 products
+        allow_smem<sym_block_kernel<64, 1024>>(4 << kMaxBitmapLog2);
+        allow_smem<sym_block_kernel<128, 2048>>(4 << kMaxBitmapLog2);
         if (bin <= kSymB64) run(sym_block_kernel<64, 1024>, 64);
         else if (bin <= kSymB128) run(sym_block_kernel<128, 2048>, 128);
-        else if (bin <= kLastSmemBin) run(sym_block_kernel<256, 8192>, 256);
-        else run(sym_block_kernel<512, 16384>, 512);
+        else if (bin <= kLastSmemBin) {
+            allow_smem<sym_block_kernel<256, 8192>>(4 << kMaxBitmapLog2);
+            run(sym_block_kernel<256, 8192>, 256);
+        } else {
+            allow_smem<sym_block_kernel<512, 16384>>(4 << kMaxBitmapLog2);
+            run(sym_block_kernel<512, 16384>, 512);
+        }
     } else {
         const int grid = heavy_ctas(count, num_sms);
         const int64_t slots = int64_t{1} << ceil_log2(2 * max_ub);
-        sym_heavy_kernel<<<grid, kSymHeavyThreads, 0, stream>>>(d_jobs, d_items, count,
-                                                               static_cast<int32_t*>(d_scratch), slots, d_err);
+        // the shared bitmaps of the products that have few enough columns
+        const int map_log2 = std::min(bitmap_log2(max_cols), kMaxBitmapLog2);
+        const int smem = 4 << map_log2;
+        allow_smem<sym_heavy_kernel>(4 << kMaxBitmapLog2);
+        sym_heavy_kernel<<<grid, kSymHeavyThreads, smem, stream>>>(d_jobs, d_items, count,
+                                                                  static_cast<int32_t*>(d_scratch), slots, map_log2, d_err);
     }
 }
 

@@ -227,7 +227,7 @@ inline void bin_lists(const Stats& stats, int64_t* count, int64_t* off) {
 }
 // K2: distinct columns per row into job.cnt[row] for the items of one bin.
 void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
-                     void* d_scratch, size_t scratch_bytes, Stats* d_stats, ErrWord* d_err,
+                     int64_t max_cols, void* d_scratch, size_t scratch_bytes, Stats* d_stats, ErrWord* d_err,
                      cudaStream_t stream, int num_sms);
 // Global scratch of the symbolic phase (hash slabs of rows above 8192 products).
 size_t symbolic_scratch_bytes(const int64_t* bin_count, int64_t max_ub, int num_sms);
