@@ -383,7 +383,8 @@ int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, con
 // products: 188 -> 171 us a call with the readbacks and memset below taken into other
 // launches; accumulation of four products 894 -> 805).  C's arrays
 // then have the upper bound's size: at most 48 MiB where the caller keeps them, 384
-// where they only live until they have been copied or added to.
+// where they only live until they have been copied or added to.  (Not for a batch's
+// device results: the serving loop charges them by their entries.)
 constexpr int64_t kDirectProducts = int64_t{1} << 22;
 constexpr int64_t kDirectTransient = int64_t{1} << 25;
 
@@ -427,10 +428,10 @@ struct CallSetup {
 static_assert(alignof(Job) <= 8 && alignof(Ctrl) <= 8, "both follow 8-byte row bases");
 
 // The phase pipeline for one or more products.  Results stay on the device.
-// products_out (optional) receives the scalar products of every product.  transient:
-// the results do not outlive the call, or the next one's.
+// products_out (optional) receives the scalar products of every product.  direct_most:
+// scalar products up to which C's arrays may have the upper bound's size.
 void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                       int64_t* products_out, bool transient) {
+                       int64_t* products_out, int64_t direct_most) {
     cudaStream_t st = h->stream;
     Arena ar(h);
     const int njobs = static_cast<int>(in.size());
@@ -633,7 +634,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     // count, into arrays of the upper bound's size; it moves nothing if there is
     // nothing to close up.
     const bool direct = !exact && njobs == 1 && total_rows > 0 && !h->cfg.hbm_budget_bytes &&
-                        products <= (transient ? kDirectTransient : kDirectProducts);
+                        products <= direct_most;
     int32_t* k5_col = nullptr;
     double* k5_val = nullptr;
     int64_t* h_starts = nullptr;
@@ -765,7 +766,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
 }
 
 void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                  int64_t* products_out, bool transient = false) {
+                  int64_t* products_out, int64_t direct_most = 0) {
     h->force_exact = false;
     h->assumed_fit = false;
     const auto drain = [&] {  // nothing of the failed attempt still reads what it freed or what it uploads from
@@ -775,13 +776,13 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         out.clear();
     };
     try {
-        run_products_once(h, in, out, count_only, products_out, transient);
+        run_products_once(h, in, out, count_only, products_out, direct_most);
     } catch (const Failure& f) {
         drain();
         if (f.status != SPG_OUT_OF_MEMORY || !h->assumed_fit) throw;
         h->force_exact = true;
         try {
-            run_products_once(h, in, out, count_only, products_out, transient);
+            run_products_once(h, in, out, count_only, products_out, direct_most);
         } catch (...) {
             h->force_exact = false;
             drain();
@@ -968,7 +969,7 @@ spg_status spg_multiply(spg_handle* h, const spg_csr_view* A, const spg_csr_view
         require(out_location == SPG_HOST || out_location == SPG_DEVICE, SPG_INVALID_ARGUMENT, "bad out_location");
         std::vector<JobIn> in{{A, B, CsrView{}}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr, out_location == SPG_HOST);
+        run_products(h, in, out, false, nullptr, out_location == SPG_HOST ? kDirectTransient : kDirectProducts);
         deliver(h, out[0], out_location, C);
     });
 }
@@ -1071,7 +1072,7 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
                 blk.row_ptr = dv[0].row_ptr + r0;  // absolute offsets into A's column/value arrays
                 std::vector<JobIn> in{{&blk, &dv[1], CsrView{}}};
                 std::vector<DevResult> out;
-                run_products(h, in, out, false, nullptr, true);
+                run_products(h, in, out, false, nullptr, kDirectTransient);
                 DevResult& r = out[0];
                 held.push_back(r);  // freed by release_held, on success or failure
                 if (off + r.nnz > c_capacity) {
@@ -1471,7 +1472,7 @@ spg_status spg_accum_add(spg_handle* h, const spg_csr_view* A, const spg_csr_vie
         }
         std::vector<JobIn> in{{A, B, S}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr, true);
+        run_products(h, in, out, false, nullptr, kDirectTransient);
         if (h->acc_has) free_result_arrays(h, &h->acc);
         deliver(h, out[0], SPG_DEVICE, &h->acc);
         h->acc_has = true;
@@ -1524,7 +1525,7 @@ spg_status spg_multiply_batch(spg_handle* h, int32_t n, const spg_csr_view* A, c
         std::vector<JobIn> in(n);
         for (int i = 0; i < n; ++i) in[i] = {&A[i], &B[i], CsrView{}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr);
+        run_products(h, in, out, false, nullptr, out_location == SPG_HOST ? kDirectTransient : 0);
         for (int i = 0; i < n; ++i) deliver(h, out[i], out_location, &C[i]);
     });
 }
