@@ -240,18 +240,24 @@ int pass_count(int32_t cols) { return std::max(1, (column_bits(cols) + 7) / 8); 
 size_t up256(size_t x) { return (x + 255) & ~size_t{255}; }
 
 // Scratch: counts (256 tiles + 1), scan partials of the counts and of the
-// columns, then the entries between passes (one set of two passes, two of more).
+// columns, then the entries between passes: values, columns and rows of one set,
+// and with more than two passes the columns of a second one, whose rows and values
+// lie in the result's arrays (20 bytes an entry).
 struct TransposeLayout {
-    size_t counts = 0, partials = 0, col_partials = 0, sets = 0, set_bytes = 0, bytes = 0;
+    size_t counts = 0, partials = 0, col_partials = 0, val = 0, col = 0, row = 0, col2 = 0, bytes = 0;
 };
 TransposeLayout transpose_layout(int64_t nnz, int32_t cols) {
     TransposeLayout L;
     const int64_t tiles = (nnz + kTTile - 1) / kTTile;
     L.partials = up256(static_cast<size_t>(256 * tiles + 1) * 8);
     L.col_partials = L.partials + up256(scan_partials_count(256 * tiles + 1) * 8);
-    L.sets = L.col_partials + up256(scan_partials_count(static_cast<int64_t>(cols) + 1) * 8);
-    L.set_bytes = up256(static_cast<size_t>(nnz) * 8) + 2 * up256(static_cast<size_t>(nnz) * 4);
-    L.bytes = L.sets + static_cast<size_t>(std::min(pass_count(cols) - 1, 2)) * L.set_bytes;
+    const int between = std::min(pass_count(cols) - 1, 2);
+    const size_t n = static_cast<size_t>(nnz);
+    L.val = L.col_partials + up256(scan_partials_count(static_cast<int64_t>(cols) + 1) * 8);
+    L.col = L.val + (between > 0 ? up256(n * 8) : 0);
+    L.row = L.col + (between > 0 ? up256(n * 4) : 0);
+    L.col2 = L.row + (between > 0 ? up256(n * 4) : 0);
+    L.bytes = L.col2 + (between > 1 ? up256(n * 4) : 0);
     return L;
 }
 
@@ -276,14 +282,10 @@ void launch_transpose(const int64_t* rp, const int32_t* col, const double* val, 
     if (nnz == 0) return;
     const int bits = column_bits(cols), passes = pass_count(cols);
     const int smem = static_cast<int>(sizeof(PassSmem));
-    auto set = [&](int i) {
-        unsigned char* p = s + L.sets + static_cast<size_t>(i) * L.set_bytes;
-        Entries e;
-        e.val = reinterpret_cast<double*>(p);
-        e.col = reinterpret_cast<int32_t*>(p + up256(static_cast<size_t>(nnz) * 8));
-        e.row = reinterpret_cast<int32_t*>(p + up256(static_cast<size_t>(nnz) * 8) + up256(static_cast<size_t>(nnz) * 4));
-        return e;
-    };
+    // the last pass reads the scratch's set, the one before it the other, and so on
+    const Entries own{reinterpret_cast<int32_t*>(s + L.col), reinterpret_cast<int32_t*>(s + L.row),
+                      reinterpret_cast<double*>(s + L.val)};
+    const Entries shared{reinterpret_cast<int32_t*>(s + L.col2), out_col, out_val};
     Entries in;
     in.col = const_cast<int32_t*>(col);
     in.val = const_cast<double*>(val);
@@ -292,7 +294,7 @@ void launch_transpose(const int64_t* rp, const int32_t* col, const double* val, 
         const int width = (bits - shift + passes - p - 1) / (passes - p);
         const uint32_t mask = (1u << width) - 1u;
         const bool first = p == 0, last = p == passes - 1;
-        Entries out = last ? Entries{nullptr, out_col, out_val} : set(p % 2);
+        Entries out = last ? Entries{nullptr, out_col, out_val} : (passes - p) % 2 == 0 ? own : shared;
         tile_hist_kernel<<<static_cast<unsigned>(tiles), kTThreads, 0, st>>>(in.col, nnz, shift, mask, tiles, counts);
         launch_scan(counts, (static_cast<int64_t>(mask) + 1) * tiles, partials, st);
         auto kern = first ? (last ? tile_scatter_kernel<true, true> : tile_scatter_kernel<true, false>)
