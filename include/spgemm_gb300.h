@@ -12,9 +12,11 @@
  * bit-identical to the reference's serialSpgemm and spgemm().
  *
  * Threading: a handle owns one CUDA stream and its workspace; calls on one
- * handle must not overlap.  Use one handle per host thread.  A handle keeps the
- * device memory its calls free for its next calls (the handles of a device at most
- * 1/16 of its memory between them); spg_destroy gives it back.
+ * handle must not overlap.  Use one handle per host thread.  A handle keeps small
+ * temporary arrays for its next calls (128 MiB at most, and within its budget where
+ * it has one); spg_destroy gives them back.  Larger ones and results go back to
+ * stream-ordered pools, whose unused memory the driver gives to other allocations
+ * of the process when they need it.
  *
  * Errors: every call returns an spg_status; spg_last_error(handle) gives the
  * message of the last failure on that handle.  include/spgemm_gb300.hpp maps

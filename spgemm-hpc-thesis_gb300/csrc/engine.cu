@@ -8,9 +8,8 @@
 //   allocate C -> K4 -> [wait] -> (K5 only if some sum was an exact zero) -> result.
 // All rows of all products of a call are flattened into one set of bin lists,
 // so a batch of products costs the same number of launches as one product.
-// Device memory comes from the handle's kept blocks (blocks.h) and the device's
-// stream-ordered pool (cudaMallocAsync), whose release threshold is raised so
-// that repeated calls reuse memory.
+// Device memory comes from stream-ordered pools, one for results and one for
+// temporaries, and from small blocks that the handle keeps (device_memory.h).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,17 +22,28 @@
 #include <vector>
 
 #include "../../include/spgemm_gb300.h"
-#include "blocks.h"
+#include "device_memory.h"
 #include "spg_common.cuh"
 
 
 using namespace spg;
 
+// A product on the device: memory of a result, or temporaries of the handle where
+// the product does not leave it (bytes of each array, device_memory.h).
+struct DevResult {
+    int32_t rows = 0, cols = 0;
+    int64_t nnz = 0, products = 0;
+    int64_t* rp = nullptr;
+    int32_t* ci = nullptr;
+    double* v = nullptr;
+    size_t rp_bytes = 0, ci_bytes = 0, v_bytes = 0;
+};
+
 struct spg_handle {
     int device = 0;
     int num_sms = 152;
     cudaStream_t stream = nullptr;
-    std::unique_ptr<BlockCache> blocks;  // device memory of the handle's calls
+    std::unique_ptr<DeviceMemory> mem;  // device memory of the handle's calls
     spg_config cfg{};
     std::string err;
     cudaEvent_t ev[6] = {};
@@ -47,10 +57,10 @@ struct spg_handle {
     bool one_bin_stream = false;  // spg_config.bin_streams == 1
     bool force_exact = false, assumed_fit = false;  // use_exact_mode of the call in progress
     spg_timings last{};
-    // accumulate mode: the running sum S (device result) and its shape
+    // accumulate mode: the running sum S and its shape
     bool acc_active = false;
     int32_t acc_rows = 0, acc_cols = 0;
-    spg_csr_result acc{};
+    DevResult acc;
     bool acc_has = false;
     // pinned control block for small device->host reads
     void* ctrl = nullptr;
@@ -89,37 +99,69 @@ void check_cuda(cudaError_t e, const char* what) {
 // Device allocations of one call; freed unless released to a result.
 class Arena {
 public:
-    explicit Arena(spg_handle* h) : h_(h) {}
+    // leaves: the call's results leave the handle
+    explicit Arena(spg_handle* h, bool leaves = true) : h_(h), leaves_(leaves) {}
+    Arena(const Arena&) = delete;
     ~Arena() {
-        for (void* p : live_)
-            if (p) h_->blocks->free(p);
+        for (const Block& b : live_) h_->mem->free(b);
     }
     template <typename T>
     T* alloc(size_t count, const char* what) {
-        void* p = nullptr;
-        check_cuda(h_->blocks->alloc(&p, std::max<size_t>(count * sizeof(T), 16)), what);
-        live_.push_back(p);
-        bytes_ += count * sizeof(T);
-        return static_cast<T*>(p);
+        return static_cast<T*>(take(count * sizeof(T), false, what));
     }
-    void release(void* p) {
-        for (auto& q : live_)
-            if (q == p) q = nullptr;
+    // For an array that (usually) becomes part of a result.
+    template <typename T>
+    T* alloc_result(size_t count, const char* what) {
+        return static_cast<T*>(take(count * sizeof(T), leaves_, what));
+    }
+    // The array is the result's; returns what DevResult has to know of it.
+    size_t release(void* p) {
+        for (Block& b : live_)
+            if (b.p == p) {
+                const Block out = leaves_ ? h_->mem->let_go(b) : b;
+                b = Block{};
+                return out.bytes;
+            }
+        return 0;
+    }
+    void release(DevResult& r) {
+        r.rp_bytes = release(r.rp);
+        r.ci_bytes = release(r.ci);
+        r.v_bytes = release(r.v);
     }
     void free_now(void* p) {
-        for (auto& q : live_)
-            if (q == p) {
-                h_->blocks->free(q);
-                q = nullptr;
+        for (Block& b : live_)
+            if (b.p == p) {
+                h_->mem->free(b);
+                b = Block{};
             }
     }
     size_t bytes() const { return bytes_; }
 
 private:
+    void* take(size_t bytes, bool result, const char* what) {
+        live_.emplace_back();  // (before the allocation: it may throw)
+        const size_t want = std::max<size_t>(bytes, 16);
+        Block b;
+        const cudaError_t e = result ? h_->mem->result(&b, want) : h_->mem->temporary(&b, want);
+        check_cuda(e, what);
+        live_.back() = b;
+        bytes_ += bytes;
+        return b.p;
+    }
+
     spg_handle* h_;
-    std::vector<void*> live_;
+    bool leaves_;
+    std::vector<Block> live_;
     size_t bytes_ = 0;
 };
+
+void free_arrays(spg_handle* h, DevResult& r) {
+    h->mem->free(Block{r.rp, r.rp_bytes});
+    h->mem->free(Block{r.ci, r.ci_bytes});
+    h->mem->free(Block{r.v, r.v_bytes});
+    r = DevResult{};
+}
 
 void sync(spg_handle* h) { check_cuda(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize"); }
 
@@ -188,14 +230,6 @@ struct JobIn {
     const spg_csr_view* A;
     const spg_csr_view* B;
     CsrView S;  // S.rp == nullptr: none
-};
-
-struct DevResult {
-    int32_t rows = 0, cols = 0;
-    int64_t nnz = 0, products = 0;
-    int64_t* rp = nullptr;
-    int32_t* ci = nullptr;
-    double* v = nullptr;
 };
 
 struct Ctrl {  // layout of the pinned control block and its device twin
@@ -428,12 +462,17 @@ struct CallSetup {
 static_assert(alignof(Job) <= 8 && alignof(Ctrl) <= 8, "both follow 8-byte row bases");
 
 // The phase pipeline for one or more products.  Results stay on the device.
-// products_out (optional) receives the scalar products of every product.  direct_most:
-// scalar products up to which C's arrays may have the upper bound's size.
+// products_out (optional) receives the scalar products of every product.  use: what
+// the caller does with the results.
+struct ResultUse {
+    bool leaves = true;       // they leave the handle (else: copied to the host or added to)
+    int64_t direct_most = 0;  // scalar products up to which C's arrays may have the upper bound's size
+};
+
 void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                       int64_t* products_out, int64_t direct_most) {
+                       int64_t* products_out, const ResultUse& use) {
     cudaStream_t st = h->stream;
-    Arena ar(h);
+    Arena ar(h, use.leaves);
     const int njobs = static_cast<int>(in.size());
     std::vector<Job> jobs(njobs);
     std::vector<int64_t> row_base(njobs + 1, 0);
@@ -461,7 +500,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     const size_t slots = static_cast<size_t>(total_rows + njobs);
     int64_t* ub = ar.alloc<int64_t>(static_cast<size_t>(total_rows), "ub");
     int64_t* cnt = ar.alloc<int64_t>(slots, "cnt");
-    int64_t* nz = ar.alloc<int64_t>(slots, "nz");
+    int64_t* nz = njobs == 1 ? ar.alloc_result<int64_t>(slots, "nz") : ar.alloc<int64_t>(slots, "nz");
     int64_t* items = ar.alloc<int64_t>(static_cast<size_t>(total_rows), "items");
     bool empty_job = false;
     for (int j = 0; j < njobs; ++j) {
@@ -587,8 +626,11 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     }
     if (h->cfg.hbm_budget_bytes && ar.bytes() + static_cast<size_t>(tmp_total) * 12 > h->cfg.hbm_budget_bytes)
         throw Failure{SPG_BUDGET_EXCEEDED, "product footprint exceeds the handle's HBM budget"};
-    int32_t* c_col = ar.alloc<int32_t>(static_cast<size_t>(tmp_total), "C col");
-    double* c_val = ar.alloc<double>(static_cast<size_t>(tmp_total), "C val");
+    const bool final_size = exact && njobs == 1;  // (unless a sum is an exact zero)
+    int32_t* c_col = final_size ? ar.alloc_result<int32_t>(static_cast<size_t>(tmp_total), "C col")
+                                : ar.alloc<int32_t>(static_cast<size_t>(tmp_total), "C col");
+    double* c_val = final_size ? ar.alloc_result<double>(static_cast<size_t>(tmp_total), "C val")
+                               : ar.alloc<double>(static_cast<size_t>(tmp_total), "C val");
     for (int j = 0; j < njobs; ++j) {
         jobs[j].c_col = c_col;
         jobs[j].c_val = c_val;
@@ -634,13 +676,13 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     // count, into arrays of the upper bound's size; it moves nothing if there is
     // nothing to close up.
     const bool direct = !exact && njobs == 1 && total_rows > 0 && !h->cfg.hbm_budget_bytes &&
-                        products <= direct_most;
+                        products <= use.direct_most;
     int32_t* k5_col = nullptr;
     double* k5_val = nullptr;
     int64_t* h_starts = nullptr;
     if (direct) {
-        k5_col = ar.alloc<int32_t>(static_cast<size_t>(products), "C col (compact)");
-        k5_val = ar.alloc<double>(static_cast<size_t>(products), "C val (compact)");
+        k5_col = ar.alloc_result<int32_t>(static_cast<size_t>(products), "C col (compact)");
+        k5_val = ar.alloc_result<double>(static_cast<size_t>(products), "C val (compact)");
         launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
         launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, k5_col, k5_val, st,
                              readback_of(d_ctrl, hc, offsetof(Ctrl, cursor)), &d_ctrl->stats, &d_ctrl->err);
@@ -674,8 +716,8 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
             if (!direct) {
                 launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
                 launches += scan_launches(static_cast<int64_t>(slots) - 1) + 1;
-                final_col = ar.alloc<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
-                final_val = ar.alloc<double>(static_cast<size_t>(nz_total), "C val (compact)");
+                final_col = ar.alloc_result<int32_t>(static_cast<size_t>(nz_total), "C col (compact)");
+                final_val = ar.alloc_result<double>(static_cast<size_t>(nz_total), "C val (compact)");
                 if (exact) launch_compact(d_jobs, in[0].A->rows, final_col, final_val, st);
                 else launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, final_col, final_val, st);
                 check_cuda(cudaGetLastError(), "K5 launch");
@@ -692,9 +734,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         r.rp = final_rp;
         r.ci = final_col;
         r.v = final_val;
-        ar.release(final_rp);
-        ar.release(final_col);
-        ar.release(final_val);
+        ar.release(r);
     } else {
         // Every product gets arrays of its own, which the compaction fills
         // directly (row r of product j at its offset minus the product's first
@@ -709,9 +749,9 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
             r.rows = in[j].A->rows;
             r.cols = in[j].B->cols;
             r.nnz = starts[j + 1] - starts[j];
-            r.rp = ar.alloc<int64_t>(static_cast<size_t>(r.rows) + 1, "result row_ptr");
-            r.ci = ar.alloc<int32_t>(static_cast<size_t>(r.nnz), "result col");
-            r.v = ar.alloc<double>(static_cast<size_t>(r.nnz), "result val");
+            r.rp = ar.alloc_result<int64_t>(static_cast<size_t>(r.rows) + 1, "result row_ptr");
+            r.ci = ar.alloc_result<int32_t>(static_cast<size_t>(r.nnz), "result col");
+            r.v = ar.alloc_result<double>(static_cast<size_t>(r.nnz), "result val");
             jobs[j].out_col = r.ci;
             jobs[j].out_val = r.v;
             rb[j] = RebaseItem{r.rp, nz + row_base[j] + j, starts[j], r.rows};
@@ -733,11 +773,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         launch_rebase(d_rb, njobs, max_rows, st);
         check_cuda(cudaGetLastError(), "rebase launch");
         launches += 2 + (exact ? njobs : 1);
-        for (auto& r : out) {
-            ar.release(r.rp);
-            ar.release(r.ci);
-            ar.release(r.v);
-        }
+        for (auto& r : out) ar.release(r);
         sync(h);  // rb must outlive its copy
     }
     for (int j = 0; j < njobs; ++j) out[j].products = job_products[j];
@@ -766,7 +802,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
 }
 
 void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevResult>& out, bool count_only,
-                  int64_t* products_out, int64_t direct_most = 0) {
+                  int64_t* products_out, const ResultUse& use = {}) {
     h->force_exact = false;
     h->assumed_fit = false;
     const auto drain = [&] {  // nothing of the failed attempt still reads what it freed or what it uploads from
@@ -776,13 +812,13 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
         out.clear();
     };
     try {
-        run_products_once(h, in, out, count_only, products_out, direct_most);
+        run_products_once(h, in, out, count_only, products_out, use);
     } catch (const Failure& f) {
         drain();
         if (f.status != SPG_OUT_OF_MEMORY || !h->assumed_fit) throw;
         h->force_exact = true;
         try {
-            run_products_once(h, in, out, count_only, products_out, direct_most);
+            run_products_once(h, in, out, count_only, products_out, use);
         } catch (...) {
             h->force_exact = false;
             drain();
@@ -798,9 +834,9 @@ void run_products(spg_handle* h, const std::vector<JobIn>& in, std::vector<DevRe
 void free_result_arrays(spg_handle* h, spg_csr_result* c) {
     if (!c) return;
     if (c->location == SPG_DEVICE) {
-        h->blocks->free(c->row_ptr);
-        h->blocks->free(c->col);
-        h->blocks->free(c->val);
+        h->mem->free(Block{c->row_ptr, 0});
+        h->mem->free(Block{c->col, 0});
+        h->mem->free(Block{c->val, 0});
     } else {
         std::free(c->row_ptr);
         std::free(c->col);
@@ -840,9 +876,7 @@ void deliver(spg_handle* h, DevResult& r, int32_t loc, spg_csr_result* C) {
     if (e == cudaSuccess && r.nnz)
         e = cudaMemcpyAsync(C->val, r.v, sizeof(double) * r.nnz, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    h->blocks->free(r.rp);
-    h->blocks->free(r.ci);
-    h->blocks->free(r.v);
+    free_arrays(h, r);
     if (e != cudaSuccess) {
         free_result_arrays(h, C);
         check_cuda(e, "D2H result");
@@ -911,7 +945,12 @@ spg_status spg_create(const spg_config* config, spg_handle** out) {
         uint64_t threshold = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
     }
-    h->blocks = std::make_unique<BlockCache>(h->device, h->stream);
+    try {
+        h->mem = std::make_unique<DeviceMemory>(h->device, h->stream, cfg.hbm_budget_bytes);
+    } catch (const std::exception&) {
+        spg_destroy(h);
+        return SPG_OUT_OF_MEMORY;
+    }
     *out = h;
     return SPG_OK;
 }
@@ -919,7 +958,7 @@ spg_status spg_create(const spg_config* config, spg_handle** out) {
 void spg_destroy(spg_handle* h) {
     if (!h) return;
     cudaSetDevice(h->device);
-    if (h->acc_has) free_result_arrays(h, &h->acc);
+    if (h->acc_has) free_arrays(h, h->acc);
     cudaStreamSynchronize(h->stream);
     if (h->copy_stream) {
         cudaStreamSynchronize(h->copy_stream);
@@ -935,7 +974,7 @@ void spg_destroy(spg_handle* h) {
     }
     if (h->fork) cudaEventDestroy(h->fork);
     for (auto e : h->join) cudaEventDestroy(e);
-    h->blocks.reset();
+    h->mem.reset();
     cudaStreamDestroy(h->stream);
     cudaFreeHost(h->ctrl);
     delete h;
@@ -969,7 +1008,8 @@ spg_status spg_multiply(spg_handle* h, const spg_csr_view* A, const spg_csr_view
         require(out_location == SPG_HOST || out_location == SPG_DEVICE, SPG_INVALID_ARGUMENT, "bad out_location");
         std::vector<JobIn> in{{A, B, CsrView{}}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr, out_location == SPG_HOST ? kDirectTransient : kDirectProducts);
+        const bool leaves = out_location == SPG_DEVICE;
+        run_products(h, in, out, false, nullptr, {leaves, leaves ? kDirectProducts : kDirectTransient});
         deliver(h, out[0], out_location, C);
     });
 }
@@ -1045,11 +1085,7 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
         // compute wait for the copies (the pool orders reuse after the free).
         std::vector<DevResult> held;
         auto release_held = [&] {
-            for (auto& q : held) {
-                h->blocks->free(q.rp);
-                h->blocks->free(q.ci);
-                h->blocks->free(q.v);
-            }
+            for (auto& q : held) free_arrays(h, q);
             held.clear();
         };
         // On any failure after the first block (a capacity shortfall, an input
@@ -1072,7 +1108,7 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
                 blk.row_ptr = dv[0].row_ptr + r0;  // absolute offsets into A's column/value arrays
                 std::vector<JobIn> in{{&blk, &dv[1], CsrView{}}};
                 std::vector<DevResult> out;
-                run_products(h, in, out, false, nullptr, kDirectTransient);
+                run_products(h, in, out, false, nullptr, {false, kDirectTransient});
                 DevResult& r = out[0];
                 held.push_back(r);  // freed by release_held, on success or failure
                 if (off + r.nnz > c_capacity) {
@@ -1229,12 +1265,8 @@ spg_status spg_tune(spg_handle* h, const spg_csr_view* A, const spg_csr_view* B,
             std::vector<JobIn> in{{A, B, CsrView{}}};
             auto one_call = [&] {
                 std::vector<DevResult> out;
-                run_products(h, in, out, false, nullptr);
-                for (auto& o : out) {
-                    h->blocks->free(o.rp);
-                    h->blocks->free(o.ci);
-                    h->blocks->free(o.v);
-                }
+                run_products(h, in, out, false, nullptr, {false, 0});
+                for (auto& o : out) free_arrays(h, o);
             };
             for (int v = 0; v < kNumVariants; ++v) {
                 std::memset(h->bin_variant, v, sizeof h->bin_variant);
@@ -1393,7 +1425,7 @@ spg_status spg_transpose(spg_handle* h, const spg_csr_view* A, int32_t out_locat
         require(out_location == SPG_HOST || out_location == SPG_DEVICE, SPG_INVALID_ARGUMENT, "bad out_location");
         check_view(A, "A");
         cudaStream_t st = h->stream;
-        Arena ar(h);
+        Arena ar(h, out_location == SPG_DEVICE);
         const CsrView a = stage(h, ar, A);
         int* d_flag = ar.alloc<int>(1, "flag");
         check_cuda(cudaMemsetAsync(d_flag, 0, sizeof(int), st), "memset");
@@ -1406,9 +1438,9 @@ spg_status spg_transpose(spg_handle* h, const spg_csr_view* A, int32_t out_locat
         r.rows = A->cols;
         r.cols = A->rows;
         r.nnz = A->nnz;
-        r.rp = ar.alloc<int64_t>(static_cast<size_t>(A->cols) + 1, "transpose row_ptr");
-        r.ci = ar.alloc<int32_t>(static_cast<size_t>(A->nnz), "transpose col");
-        r.v = ar.alloc<double>(static_cast<size_t>(A->nnz), "transpose val");
+        r.rp = ar.alloc_result<int64_t>(static_cast<size_t>(A->cols) + 1, "transpose row_ptr");
+        r.ci = ar.alloc_result<int32_t>(static_cast<size_t>(A->nnz), "transpose col");
+        r.v = ar.alloc_result<double>(static_cast<size_t>(A->nnz), "transpose val");
         void* scratch = ar.alloc<unsigned char>(transpose_scratch_bytes(A->nnz, A->cols), "transpose scratch");
         check_cuda(cudaEventRecord(h->fork, st), "event");
         check_cuda(cudaStreamWaitEvent(h->aux[0], h->fork, 0), "stream wait");
@@ -1417,9 +1449,7 @@ spg_status spg_transpose(spg_handle* h, const spg_csr_view* A, int32_t out_locat
         cudaEventRecord(h->join[0], h->aux[0]);
         cudaStreamWaitEvent(st, h->join[0], 0);
         check_cuda(launched, "transpose launch");
-        ar.release(r.rp);
-        ar.release(r.ci);
-        ar.release(r.v);
+        ar.release(r);
         deliver(h, r, out_location, C);
     });
 }
@@ -1447,7 +1477,7 @@ spg_status spg_last_timings(const spg_handle* h, spg_timings* t) {
 spg_status spg_accum_begin(spg_handle* h, int32_t rows, int32_t cols) {
     return guarded(h, [&] {
         require(rows >= 0 && cols >= 0, SPG_INVALID_ARGUMENT, "negative accumulator shape");
-        if (h->acc_has) free_result_arrays(h, &h->acc);
+        if (h->acc_has) free_arrays(h, h->acc);
         h->acc_has = false;
         h->acc_active = true;
         h->acc_rows = rows;
@@ -1466,15 +1496,15 @@ spg_status spg_accum_add(spg_handle* h, const spg_csr_view* A, const spg_csr_vie
             S.rows = h->acc.rows;
             S.cols = h->acc.cols;
             S.nnz = h->acc.nnz;
-            S.rp = h->acc.row_ptr;
-            S.ci = h->acc.col;
-            S.v = h->acc.val;
+            S.rp = h->acc.rp;
+            S.ci = h->acc.ci;
+            S.v = h->acc.v;
         }
         std::vector<JobIn> in{{A, B, S}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr, kDirectTransient);
-        if (h->acc_has) free_result_arrays(h, &h->acc);
-        deliver(h, out[0], SPG_DEVICE, &h->acc);
+        run_products(h, in, out, false, nullptr, {false, kDirectTransient});
+        if (h->acc_has) free_arrays(h, h->acc);
+        h->acc = out[0];
         h->acc_has = true;
     });
 }
@@ -1486,31 +1516,33 @@ spg_status spg_accum_finish(spg_handle* h, int32_t out_location, spg_csr_result*
         require(h->acc_active, SPG_INVALID_ARGUMENT, "no accumulation in progress");
         require(C != nullptr, SPG_INVALID_ARGUMENT, "C is NULL");
         require(out_location == SPG_HOST || out_location == SPG_DEVICE, SPG_INVALID_ARGUMENT, "bad out_location");
+        Arena ar(h, out_location == SPG_DEVICE);
         DevResult r;
         r.rows = h->acc_rows;
         r.cols = h->acc_cols;
         r.nnz = h->acc_has ? h->acc.nnz : 0;
         r.products = h->acc_has ? h->acc.products : 0;
         const size_t rp_bytes = sizeof(int64_t) * (static_cast<size_t>(r.rows) + 1);
-        check_cuda(h->blocks->alloc(reinterpret_cast<void**>(&r.rp), rp_bytes), "alloc row_ptr");
-        check_cuda(h->blocks->alloc(reinterpret_cast<void**>(&r.ci), std::max<size_t>(16, 4 * r.nnz)), "alloc col");
-        check_cuda(h->blocks->alloc(reinterpret_cast<void**>(&r.v), std::max<size_t>(16, 8 * r.nnz)), "alloc val");
+        r.rp = ar.alloc_result<int64_t>(static_cast<size_t>(r.rows) + 1, "alloc row_ptr");
+        r.ci = ar.alloc_result<int32_t>(static_cast<size_t>(r.nnz), "alloc col");
+        r.v = ar.alloc_result<double>(static_cast<size_t>(r.nnz), "alloc val");
         if (h->acc_has) {
-            check_cuda(cudaMemcpyAsync(r.rp, h->acc.row_ptr, rp_bytes, cudaMemcpyDeviceToDevice, h->stream), "D2D");
+            check_cuda(cudaMemcpyAsync(r.rp, h->acc.rp, rp_bytes, cudaMemcpyDeviceToDevice, h->stream), "D2D");
             if (r.nnz) {
-                check_cuda(cudaMemcpyAsync(r.ci, h->acc.col, 4 * r.nnz, cudaMemcpyDeviceToDevice, h->stream), "D2D");
-                check_cuda(cudaMemcpyAsync(r.v, h->acc.val, 8 * r.nnz, cudaMemcpyDeviceToDevice, h->stream), "D2D");
+                check_cuda(cudaMemcpyAsync(r.ci, h->acc.ci, 4 * r.nnz, cudaMemcpyDeviceToDevice, h->stream), "D2D");
+                check_cuda(cudaMemcpyAsync(r.v, h->acc.v, 8 * r.nnz, cudaMemcpyDeviceToDevice, h->stream), "D2D");
             }
         } else {  // no stage added yet: an all-empty result
             check_cuda(cudaMemsetAsync(r.rp, 0, rp_bytes, h->stream), "memset");
         }
+        ar.release(r);
         deliver(h, r, out_location, C);
     });
 }
 
 spg_status spg_accum_end(spg_handle* h) {
     return guarded(h, [&] {
-        if (h->acc_has) free_result_arrays(h, &h->acc);
+        if (h->acc_has) free_arrays(h, h->acc);
         h->acc_has = false;
         h->acc_active = false;
     });
@@ -1525,7 +1557,8 @@ spg_status spg_multiply_batch(spg_handle* h, int32_t n, const spg_csr_view* A, c
         std::vector<JobIn> in(n);
         for (int i = 0; i < n; ++i) in[i] = {&A[i], &B[i], CsrView{}};
         std::vector<DevResult> out;
-        run_products(h, in, out, false, nullptr, out_location == SPG_HOST ? kDirectTransient : 0);
+        const bool leaves = out_location == SPG_DEVICE;
+        run_products(h, in, out, false, nullptr, {leaves, leaves ? 0 : kDirectTransient});
         for (int i = 0; i < n; ++i) deliver(h, out[i], out_location, &C[i]);
     });
 }
@@ -1560,7 +1593,15 @@ namespace {
 template <typename T>
 T* plan_alloc(spg_plan* p, size_t count, const char* what) {
     void* q = nullptr;
-    check_cuda(device_malloc(&q, std::max<size_t>(count * sizeof(T), 16)), what);
+    const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
+    cudaError_t e = cudaMalloc(&q, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // tried again without the handle's kept blocks
+        cudaGetLastError();
+        p->h->mem->give_back();
+        sync(p->h);
+        e = cudaMalloc(&q, bytes);
+    }
+    check_cuda(e, what);
     p->bufs.push_back(q);
     return static_cast<T*>(q);
 }
@@ -1672,10 +1713,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     for (int32_t r : p->rows) max_rows = std::max<int64_t>(max_rows, r);
 
     // values: the replayed part
-    h->blocks->set_capturing(true);
-    const cudaError_t be = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
-    if (be != cudaSuccess) h->blocks->set_capturing(false);
-    check_cuda(be, "begin capture");
+    check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed), "begin capture");
     cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st);
     cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st);
     // (the bins' fork and join are part of the graph)
@@ -1687,7 +1725,6 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     launch_rebase_jobs(nz, p->rp, d_row_base, n, max_rows, st);
     const cudaError_t le = cudaGetLastError();
     const cudaError_t ce = cudaStreamEndCapture(st, &p->graph);
-    h->blocks->set_capturing(false);
     check_cuda(le, "plan capture launches");
     check_cuda(ce, "end capture");
     check_cuda(cudaGraphInstantiate(&p->exec, p->graph, 0), "graph instantiate");

@@ -23,7 +23,6 @@
 #include <vector>
 
 #include "../../include/spgemm_gb300.h"
-#include "blocks.h"
 
 namespace {
 
@@ -262,9 +261,9 @@ extern "C" spg_status spg_read_matrix_market(const char* path, int32_t out_locat
         }
         return SPG_OK;
     }
-    cudaError_t e = spg::device_malloc(reinterpret_cast<void**>(&C->row_ptr), brp);
-    if (e == cudaSuccess) e = spg::device_malloc(reinterpret_cast<void**>(&C->col), bci);
-    if (e == cudaSuccess) e = spg::device_malloc(reinterpret_cast<void**>(&C->val), bva);
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&C->row_ptr), brp);
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&C->col), bci);
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&C->val), bva);
     if (e == cudaSuccess) e = cudaMemcpy(C->row_ptr, rp.data(), brp, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nnz) e = cudaMemcpy(C->col, ci.data(), sizeof(int32_t) * nnz, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nnz) e = cudaMemcpy(C->val, va.data(), sizeof(double) * nnz, cudaMemcpyHostToDevice);
@@ -282,9 +281,9 @@ extern "C" spg_status spg_read_matrix_market(const char* path, int32_t out_locat
 extern "C" void spg_csr_release(spg_csr_result* C) {
     if (!C) return;
     if (C->location == SPG_DEVICE) {
-        spg::block_release(C->row_ptr);
-        spg::block_release(C->col);
-        spg::block_release(C->val);
+        cudaFree(C->row_ptr);
+        cudaFree(C->col);
+        cudaFree(C->val);
     } else {
         std::free(C->row_ptr);
         std::free(C->col);

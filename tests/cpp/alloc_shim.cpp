@@ -5,13 +5,17 @@
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 
+#include <atomic>
+#include <chrono>
 #include <mutex>
+#include <thread>
 #include <unordered_map>
 
 namespace {
 
 std::mutex lock;
 std::unordered_map<void*, size_t> live;
+std::atomic<long long> slow_bytes{-1}, slow_ms{0};  // allocations of at least that many bytes take that long
 long long calls, bytes, peak, failed, fail_from, fail_count, total;
 
 template <typename F>
@@ -29,6 +33,8 @@ cudaError_t counted(void** p, size_t n, Alloc&& alloc) {
             return cudaErrorMemoryAllocation;
         }
     }
+    const long long slow = slow_bytes;
+    if (slow >= 0 && static_cast<long long>(n) >= slow) std::this_thread::sleep_for(std::chrono::milliseconds(slow_ms));
     const cudaError_t e = alloc();
     if (e == cudaSuccess) {
         std::lock_guard<std::mutex> g(lock);
@@ -83,6 +89,10 @@ void shim_start(long long from, long long count) {
     peak = bytes;
     fail_from = from;
     fail_count = count;
+}
+void shim_slow(long long from_bytes, long long ms) {
+    slow_ms = ms;
+    slow_bytes = from_bytes;
 }
 // calls, failed ones, bytes held now, their peak, all bytes ever asked for
 void shim_stats(long long* out) {
