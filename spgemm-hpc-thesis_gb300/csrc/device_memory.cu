@@ -35,6 +35,15 @@ cudaMemPool_t temporaries_pool(int device) {
     return pool;
 }
 
+// Small blocks come in steps of an eighth where there is no budget, so that calls of
+// about the same size share them; the pools' own granularity is 512 bytes.
+size_t block_size(size_t bytes, bool exact) {
+    size_t step = 512;
+    if (!exact && bytes <= DeviceMemory::kKeptBlock)
+        for (size_t p = 4096; p * 2 <= bytes; p *= 2) step = p / 4;
+    return std::max(step, (bytes + step - 1) / step * step);
+}
+
 }  // namespace
 
 DeviceMemory::DeviceMemory(int device, cudaStream_t stream, size_t budget)
@@ -44,21 +53,13 @@ DeviceMemory::DeviceMemory(int device, cudaStream_t stream, size_t budget)
 
 DeviceMemory::~DeviceMemory() { give_back(); }
 
-// Without a budget small blocks come in steps of an eighth, so that calls of about
-// the same size share them; the pools' own granularity is 512 bytes.
-size_t DeviceMemory::block_size(size_t bytes) const noexcept {
-    size_t step = 512;
-    if (!budget_ && bytes <= kKeptBlock)
-        for (size_t p = 4096; p * 2 <= bytes; p *= 2) step = p / 4;
-    return std::max(step, (bytes + step - 1) / step * step);
-}
-
-cudaError_t DeviceMemory::temporary(Block* b, size_t bytes) noexcept {
-    const size_t want = block_size(bytes);
+cudaError_t DeviceMemory::temporary(Block* b, size_t bytes, bool may_leave) noexcept {
+    const size_t want = block_size(bytes, budget_ != 0);
+    const size_t most = budget_ || may_leave ? want : want + want / 4;
     if (budget_ && live_ + kept_bytes_ + want > budget_) give_back();
-    size_t best = kept_.size();  // the smallest kept block that is not more than a quarter too large
+    size_t best = kept_.size();  // the smallest kept block that is not much too large
     for (size_t i = 0; i < kept_.size(); ++i)
-        if (kept_[i].bytes >= want && kept_[i].bytes <= (budget_ ? want : want + want / 4) &&
+        if (kept_[i].bytes >= want && kept_[i].bytes <= most &&
             (best == kept_.size() || kept_[i].bytes < kept_[best].bytes))
             best = i;
     if (best < kept_.size()) {

@@ -46,8 +46,9 @@ public:
     DeviceMemory(const DeviceMemory&) = delete;
     DeviceMemory& operator=(const DeviceMemory&) = delete;
 
-    // At least `bytes` for work on the handle's stream.
-    cudaError_t temporary(Block* b, size_t bytes) noexcept;
+    // At least `bytes` for work on the handle's stream; where the block may become
+    // memory of a result, at most an eighth more, and no more above kKeptBlock.
+    cudaError_t temporary(Block* b, size_t bytes, bool may_leave) noexcept;
     // Exactly `bytes` for a result that the caller keeps.
     cudaError_t result(Block* b, size_t bytes) noexcept;
     // Frees a block after the work queued on the handle's stream; memory of results
@@ -59,8 +60,6 @@ public:
     void give_back() noexcept;
 
 private:
-    size_t block_size(size_t bytes) const noexcept;
-
     const cudaStream_t stream_;
     const size_t budget_;
     const cudaMemPool_t pool_;  // of temporaries; nullptr: the default pool

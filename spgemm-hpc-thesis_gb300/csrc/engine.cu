@@ -107,12 +107,17 @@ public:
     }
     template <typename T>
     T* alloc(size_t count, const char* what) {
-        return static_cast<T*>(take(count * sizeof(T), false, what));
+        return static_cast<T*>(take(count * sizeof(T), false, false, what));
     }
     // For an array that (usually) becomes part of a result.
     template <typename T>
     T* alloc_result(size_t count, const char* what) {
-        return static_cast<T*>(take(count * sizeof(T), leaves_, what));
+        return static_cast<T*>(take(count * sizeof(T), leaves_, false, what));
+    }
+    // For an array that now and then does.
+    template <typename T>
+    T* alloc_maybe_result(size_t count, const char* what) {
+        return static_cast<T*>(take(count * sizeof(T), false, leaves_, what));
     }
     // The array is the result's; returns what DevResult has to know of it.
     size_t release(void* p) {
@@ -139,11 +144,11 @@ public:
     size_t bytes() const { return bytes_; }
 
 private:
-    void* take(size_t bytes, bool result, const char* what) {
+    void* take(size_t bytes, bool result, bool may_leave, const char* what) {
         live_.emplace_back();  // (before the allocation: it may throw)
         const size_t want = std::max<size_t>(bytes, 16);
         Block b;
-        const cudaError_t e = result ? h_->mem->result(&b, want) : h_->mem->temporary(&b, want);
+        const cudaError_t e = result ? h_->mem->result(&b, want) : h_->mem->temporary(&b, want, may_leave);
         check_cuda(e, what);
         live_.back() = b;
         bytes_ += bytes;
@@ -499,7 +504,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     // per-row workspace: ub (rows), cnt and nz (rows + 1 per job)
     const size_t slots = static_cast<size_t>(total_rows + njobs);
     int64_t* ub = ar.alloc<int64_t>(static_cast<size_t>(total_rows), "ub");
-    int64_t* cnt = ar.alloc<int64_t>(slots, "cnt");
+    int64_t* cnt = ar.alloc_maybe_result<int64_t>(slots, "cnt");
     int64_t* nz = njobs == 1 ? ar.alloc_result<int64_t>(slots, "nz") : ar.alloc<int64_t>(slots, "nz");
     int64_t* items = ar.alloc<int64_t>(static_cast<size_t>(total_rows), "items");
     bool empty_job = false;
@@ -628,9 +633,9 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         throw Failure{SPG_BUDGET_EXCEEDED, "product footprint exceeds the handle's HBM budget"};
     const bool final_size = exact && njobs == 1;  // (unless a sum is an exact zero)
     int32_t* c_col = final_size ? ar.alloc_result<int32_t>(static_cast<size_t>(tmp_total), "C col")
-                                : ar.alloc<int32_t>(static_cast<size_t>(tmp_total), "C col");
+                                : ar.alloc_maybe_result<int32_t>(static_cast<size_t>(tmp_total), "C col");
     double* c_val = final_size ? ar.alloc_result<double>(static_cast<size_t>(tmp_total), "C val")
-                               : ar.alloc<double>(static_cast<size_t>(tmp_total), "C val");
+                               : ar.alloc_maybe_result<double>(static_cast<size_t>(tmp_total), "C val");
     for (int j = 0; j < njobs; ++j) {
         jobs[j].c_col = c_col;
         jobs[j].c_val = c_val;

@@ -61,6 +61,27 @@ def test_budget_bounds_what_is_kept(tmp_path):
         assert sizes == want
 
 
+def handed_over(shim):
+    """Sizes of the arrays of results that need no compaction."""
+    import numpy as np
+    out = []
+    with sg.Engine(0) as eng:
+        for n in (5000, 4900, 100_000, 70_000):
+            d = sg.Csr.from_arrays(n, n, np.arange(n + 1), np.arange(n), np.ones(n))
+            b = sg.synth_uniform(n, n, 3, 9, seed=n)
+            for _ in range(2):
+                r = eng.multiply(d, b, out="device")
+                out.append([[shim.size(p) for p in r.pointers], [8 * (n + 1), 4 * r.nnz, 8 * r.nnz], r.nnz == r.products])
+                r.free()
+    return out
+
+
+def test_arrays_handed_over_have_their_size(tmp_path):
+    for sizes, want, full in alloc_shim.run(tmp_path, ME, "handed_over"):
+        assert full
+        assert all(w <= s <= w + max(w // 8, 512) for s, w in zip(sizes, want)), (sizes, want)
+
+
 def beside_a_slow_one(shim):
     """Longest call of a handle with small products while another handle's large
     allocations take 400 ms each."""
