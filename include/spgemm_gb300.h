@@ -81,8 +81,8 @@ typedef struct {
  * (a second pass over the products, no scratch); AUTO picks UPPER_BOUND unless
  * its scratch would exceed the budget or half of the free device memory (looked
  * at above 2 GiB; below, EXACT follows if an allocation fails).  C's device arrays
- * may be larger than C, up to 12 bytes per scalar product for calls of at most
- * 2^22 of them. */
+ * may be larger than C for calls of at most 2^22 scalar products: by 1 MiB, or
+ * twice as large. */
 typedef enum { SPG_MODE_AUTO = 0, SPG_MODE_EXACT = 1, SPG_MODE_UPPER_BOUND = 2 } spg_mode;
 
 typedef struct {
