@@ -180,8 +180,9 @@ void spg_server::run_batch(int lane, std::vector<Request*>& batch) {
         std::fill(each.begin(), each.end(), SPG_OK);
     } else if (n > 1 && (s == SPG_INVALID_ARGUMENT || s == SPG_OUT_OF_RANGE_COLUMN || s == SPG_OVERFLOW)) {
         // an input error of some request: run them one by one so that only it fails
+        // (batches of one, whose results have the size that they are charged with)
         for (int i = 0; i < n; ++i) {
-            each[i] = spg_multiply(h, &A[i], &B[i], cfg.out_location, &C[i]);
+            each[i] = spg_multiply_batch(h, 1, &A[i], &B[i], cfg.out_location, &C[i]);
             if (each[i] != SPG_OK) msg[i] = spg_last_error(h);
             spg_last_timings(h, &t);
             launches += t.launches;
