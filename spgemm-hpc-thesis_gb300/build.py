@@ -22,7 +22,7 @@ OBJ = HERE / "_build" / platform.machine()  # host objects differ per architectu
 LIB = HERE / "libspgemm_gb300.so"
 SOURCES = ["engine.cu", "device_memory.cu", "k_rowwork.cu", "k_symbolic.cu", "k_numeric.cu", "k_numeric_warp.cu", "k_numeric_alt.cu",
            "k_validate.cu", "k_transpose.cu", "mtx.cu", "noalloc.cu", "server.cu"]
-HEADERS = ["device_memory.h", "spg_common.cuh", "spg_enum.cuh", "spg_warp_sort.cuh", "k_numeric_row.cuh"]
+HEADERS = ["device_memory.h", "dispatch.h", "spg_common.cuh", "spg_enum.cuh", "spg_warp_sort.cuh", "k_numeric_row.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC,-O3",
               "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]

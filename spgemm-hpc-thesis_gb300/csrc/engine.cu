@@ -603,14 +603,17 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         if (scanned) check_cuda(cudaMemsetAsync(cnt, 0, slots * sizeof(int64_t), st), "memset cnt");
         // K2's bins share no scratch: a stream each (0.86 -> 0.71 ms for 74 M products
         // in 19 bins)
-        int64_t max_cols = 0;
-        for (const JobIn& j : in) max_cols = std::max<int64_t>(max_cols, j.B->cols);
+        int64_t max_cols = 0, map_cols = 0;
+        for (const JobIn& j : in) {
+            max_cols = std::max<int64_t>(max_cols, j.B->cols);
+            map_cols = std::max(map_cols, heavy_map_cols(j.B->cols));
+        }
         BinStreams k2(h, 0);
         k2.begin(bin_count);
         k2.for_each_bin([&](int b) {
             if (!bin_count[b]) return;
-            launch_symbolic(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, max_cols, scratch, scratch_bytes,
-                            &d_ctrl->stats, &d_ctrl->err, k2.of(b), h->num_sms);
+            launch_symbolic(b, d_jobs, items + bin_off[b], bin_count[b], max_ub, max_cols, map_cols, scratch,
+                            scratch_bytes, &d_ctrl->stats, &d_ctrl->err, k2.of(b), h->num_sms);
             ++launches;
         });
         k2.end();

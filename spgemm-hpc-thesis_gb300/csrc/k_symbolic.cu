@@ -59,19 +59,11 @@ __device__ inline int hash_insert(int32_t* tab, uint32_t mask, int log2t, int32_
     }
 }
 
-// log2 of the words of a bitmap of `cols` columns.
-__host__ __device__ inline int bitmap_log2(int64_t cols) {
-    const int l = ceil_log2(cols) - 5;
-    return l > 0 ? l : 0;
-}
-
 // Sets column col's bit in a bitmap of 2^log2w words; returns 1 if it was not set.
 __device__ inline int bitmap_insert(uint32_t* map, int log2w, int32_t col) {
     const uint32_t bit = 1u << (static_cast<uint32_t>(col) >> log2w);
     return (atomicOr(&map[static_cast<uint32_t>(col) & ((1u << log2w) - 1u)], bit) & bit) == 0u;
 }
-
-constexpr int kMaxBitmapLog2 = 15;  // 128 KiB of shared memory
 
 // log2 of the words reserved per row of a bin: the table's, or a bitmap's of up to
 // twice as many.
@@ -172,7 +164,7 @@ sym_block_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items
 __global__ void __launch_bounds__(kSymHeavyThreads)
 sym_heavy_kernel(const Job* __restrict__ jobs, const int64_t* __restrict__ items, int64_t count,
                  int32_t* __restrict__ slabs, int64_t slab_slots, int map_log2, ErrWord* __restrict__ err) {
-    extern __shared__ __align__(16) int32_t s_map[];  // 2^map_log2 words
+    extern __shared__ __align__(16) int32_t s_map[];  // 2^map_log2 words; none if map_log2 < 0
     __shared__ SegTab<kSymHeavyThreads> s_seg;
     __shared__ int64_t s_warp[kSymHeavyThreads / 32 + 1];
     __shared__ unsigned long long s_found;
@@ -218,7 +210,8 @@ size_t symbolic_scratch_bytes(const int64_t* bin_count, int64_t max_ub, int num_
 }
 
 void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
-                     int64_t max_cols, void* d_scratch, size_t, Stats*, ErrWord* d_err, cudaStream_t stream, int num_sms) {
+                     int64_t max_cols, int64_t map_cols, void* d_scratch, size_t, Stats*, ErrWord* d_err,
+                     cudaStream_t stream, int num_sms) {
     if (count <= 0) return;
     if (bin <= kLastWarpBin) {
         const int wtab_log2 = reserved_log2(bin, max_cols);
@@ -248,8 +241,8 @@ void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t
         const int grid = heavy_ctas(count, num_sms);
         const int64_t slots = int64_t{1} << ceil_log2(2 * max_ub);
         // the shared bitmaps of the products that have few enough columns
-        const int map_log2 = std::min(bitmap_log2(max_cols), kMaxBitmapLog2);
-        const int smem = 4 << map_log2;
+        const int map_log2 = heavy_map_log2(map_cols);
+        const int smem = map_log2 < 0 ? 0 : 4 << map_log2;
         allow_smem<sym_heavy_kernel>(4 << kMaxBitmapLog2);
         sym_heavy_kernel<<<grid, kSymHeavyThreads, smem, stream>>>(d_jobs, d_items, count,
                                                                   static_cast<int32_t*>(d_scratch), slots, map_log2, d_err);

@@ -186,8 +186,8 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         return ret(SPG_BUDGET_EXCEEDED, "heavy rows need more than the 32 MiB allocation-free scratch", err, err_len);
 
     for (int b = 1; b < kNumBins; ++b)
-        launch_symbolic(b, d_job, items + bin_off[b], bin_count[b], max_ub, B->cols, d_slab,
-                        slab, &d_ctrl->stats, &d_ctrl->err, st, num_sms);
+        launch_symbolic(b, d_job, items + bin_off[b], bin_count[b], max_ub, B->cols,
+                        heavy_map_cols(B->cols), d_slab, slab, &d_ctrl->stats, &d_ctrl->err, st, num_sms);
     launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "symbolic launch", err, err_len);
     int64_t total = 0;

@@ -14,6 +14,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "dispatch.h"
+
 namespace spg {
 
 constexpr int kWarp = 32;
@@ -225,10 +227,11 @@ inline void bin_lists(const Stats& stats, int64_t* count, int64_t* off) {
     }
     off[kNumBins] = at;
 }
-// K2: distinct columns per row into job.cnt[row] for the items of one bin.
+// K2: distinct columns per row into job.cnt[row] for the items of one bin.  max_cols:
+// most columns of a B; map_cols: the most that heavy_map_cols counts.
 void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
-                     int64_t max_cols, void* d_scratch, size_t scratch_bytes, Stats* d_stats, ErrWord* d_err,
-                     cudaStream_t stream, int num_sms);
+                     int64_t max_cols, int64_t map_cols, void* d_scratch, size_t scratch_bytes, Stats* d_stats,
+                     ErrWord* d_err, cudaStream_t stream, int num_sms);
 // Global scratch of the symbolic phase (hash slabs of rows above 8192 products).
 size_t symbolic_scratch_bytes(const int64_t* bin_count, int64_t max_ub, int num_sms);
 // K3: exclusive scan of n+1 int64 counts (16-byte aligned) in place (last entry

@@ -321,10 +321,4 @@ __device__ inline uint32_t hash_slot(int32_t col, int log2t) {
     return (static_cast<uint32_t>(col) * 0x9E3779B1u) >> (32 - log2t);
 }
 
-__host__ __device__ inline int ceil_log2(int64_t x) {
-    int l = 0;
-    while ((int64_t{1} << l) < x) ++l;
-    return l;
-}
-
 }  // namespace spg
