@@ -1,7 +1,9 @@
 // Rules of the dispatch that depend on sizes alone, free of device code.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -29,5 +31,56 @@ inline int64_t heavy_map_cols(int64_t cols) { return bitmap_log2(cols) <= kMaxBi
 // memory for one (128 KiB that no row can use halve the CTAs per SM: 2,000 rows of
 // 40,000 products, 2^20 + 1 columns, 4.7 ms with them and 3.4 without).
 inline int heavy_map_log2(int64_t map_cols) { return map_cols > 0 ? bitmap_log2(map_cols) : -1; }
+
+// K1's lanes per row, by the entries of A in the rows of a launch.  Measured with 4 / 8
+// lanes (2 and 32 were slower everywhere; one warp per row with 64-bit shared atomics
+// before): 65,536 rows of 16 entries 13.3 / 15.8 us (21), power-law rows of 24 on
+// average 244 / 255 us (323), uneven rows of 34 38 / 35 us (34), R and R*A of the
+// 128^3 Galerkin chain (8 and 32 entries) 110 / 86 us (143).
+inline int rowwork_lanes(int64_t entries, int64_t rows) { return entries / rows <= 24 ? 4 : 8; }
+
+// The row blocks of a product that is copied to the host while it is computed.
+struct RowBlock {
+    int32_t first, end;  // rows
+    int64_t entries;     // of A in them
+};
+
+// Operands with at least this many entries in A are multiplied in row blocks.
+constexpr int64_t kBlockedEntries = int64_t{1} << 22;
+
+// Row blocks by A's entries: 1/32, 1/32, 1/16, then 1/8 each, so that the first
+// copy starts after a small block and the later blocks keep the copy engine
+// busy while the next one computes.  Small operands run as one block.  The
+// cuts come from A's row offsets on the host, or from equal row counts
+// when A lives on the device (row_ptr is nullptr).
+inline std::vector<RowBlock> row_blocks(int32_t rows, int64_t nnz, const int64_t* row_ptr) {
+    std::vector<int32_t> cut{0};
+    if (nnz >= kBlockedEntries && rows > 1) {
+        const double fr[] = {1.0 / 32, 1.0 / 32, 1.0 / 16, 1.0 / 8, 1.0 / 8, 1.0 / 8, 1.0 / 8, 1.0 / 8, 1.0 / 8, 1.0 / 8};
+        double acc = 0.0;
+        for (double f : fr) {
+            acc += f;
+            int32_t r;
+            if (acc >= 1.0 - 1e-12) {
+                r = rows;
+            } else if (row_ptr) {
+                const int64_t target = static_cast<int64_t>(acc * static_cast<double>(nnz));
+                r = static_cast<int32_t>(std::lower_bound(row_ptr, row_ptr + rows + 1, target) - row_ptr);
+            } else {
+                r = static_cast<int32_t>(acc * rows);
+            }
+            r = std::min(std::max(r, cut.back()), rows);
+            if (r > cut.back()) cut.push_back(r);
+        }
+    }
+    if (cut.back() != rows) cut.push_back(rows);
+    std::vector<RowBlock> blocks;
+    for (size_t k = 0; k + 1 < cut.size(); ++k) {
+        const int32_t r0 = cut[k], r1 = cut[k + 1];
+        blocks.push_back({r0, r1, row_ptr ? row_ptr[r1] - row_ptr[r0]
+                                          : static_cast<int64_t>(static_cast<double>(nnz) * (r1 - r0) / rows)});
+    }
+    return blocks;
+}
 
 }  // namespace spg

@@ -235,6 +235,7 @@ struct JobIn {
     const spg_csr_view* A;
     const spg_csr_view* B;
     CsrView S;  // S.rp == nullptr: none
+    int64_t entries = -1;  // of A in its rows, where that is not A->nnz (a row block of a larger matrix)
 };
 
 struct Ctrl {  // layout of the pinned control block and its device twin
@@ -493,7 +494,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
         check_view(in[j].B, "B");
         require(in[j].A->cols == in[j].B->rows, SPG_INVALID_ARGUMENT, "SpGEMM requires A.cols == B.rows");
         row_base[j + 1] = row_base[j] + in[j].A->rows;
-        entries += in[j].A->nnz;
+        entries += in[j].entries >= 0 ? in[j].entries : in[j].A->nnz;
     }
     const int64_t total_rows = row_base[njobs];
     for (int j = 0; j < njobs; ++j) {
@@ -1039,9 +1040,6 @@ spg_status spg_multiply(spg_handle* h, const spg_csr_view* A, const spg_csr_view
     });
 }
 
-// Operands with at least this many entries in A are multiplied in row blocks.
-constexpr int64_t kBlockedEntries = int64_t{1} << 22;
-
 spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_csr_view* B, int64_t* c_row_ptr,
                                 int32_t* c_col, double* c_val, int64_t c_capacity, int64_t* c_nnz) {
     return guarded(h, [&] {
@@ -1073,34 +1071,8 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
                 }
             }
         }
-        // Row blocks by A's entries: 1/32, 1/32, 1/16, then 1/8 each, so that the first
-        // copy starts after a small block and the later blocks keep the copy engine
-        // busy while the next one computes.  Small operands run as one block.  The
-        // cuts come from A's row offsets on the host, or from equal row counts
-        // when A lives on the device.
         const int32_t m = A->rows;
-        std::vector<int32_t> cut{0};
-        if (A->nnz >= kBlockedEntries && m > 1) {
-            const double fr[] = {1.0 / 32, 1.0 / 32, 1.0 / 16, 1.0 / 8, 1.0 / 8, 1.0 / 8, 1.0 / 8,
-                                 1.0 / 8, 1.0 / 8, 1.0 / 8};
-            double acc = 0.0;
-            for (double f : fr) {
-                acc += f;
-                int32_t r;
-                if (acc >= 1.0 - 1e-12) {
-                    r = m;
-                } else if (A->location == SPG_HOST) {
-                    const int64_t target = static_cast<int64_t>(acc * static_cast<double>(A->nnz));
-                    r = static_cast<int32_t>(std::lower_bound(A->row_ptr, A->row_ptr + m + 1, target) - A->row_ptr);
-                } else {
-                    r = static_cast<int32_t>(acc * m);
-                }
-                r = std::min(std::max(r, cut.back()), m);
-                if (r > cut.back()) cut.push_back(r);
-            }
-        }
-        if (cut.back() != m) cut.push_back(m);
-        const int nchunks = static_cast<int>(cut.size()) - 1;
+        const std::vector<RowBlock> blocks = row_blocks(m, A->nnz, A->location == SPG_HOST ? A->row_ptr : nullptr);
         int64_t products = 0;
         spg_timings sum{};
         int64_t off = 0;
@@ -1126,12 +1098,12 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
         };
         c_row_ptr[0] = 0;
         try {
-            for (int k = 0; k < nchunks; ++k) {
-                const int32_t r0 = cut[k], r1 = cut[k + 1];
+            for (const RowBlock& block : blocks) {
+                const int32_t r0 = block.first, r1 = block.end;
                 spg_csr_view blk = dv[0];
                 blk.rows = r1 - r0;
                 blk.row_ptr = dv[0].row_ptr + r0;  // absolute offsets into A's column/value arrays
-                std::vector<JobIn> in{{&blk, &dv[1], CsrView{}}};
+                std::vector<JobIn> in{{&blk, &dv[1], CsrView{}, block.entries}};
                 std::vector<DevResult> out;
                 run_products(h, in, out, false, nullptr, {false, kDirectTransient});
                 DevResult& r = out[0];

@@ -60,7 +60,7 @@ __device__ __forceinline__ int64_t entry_products(const Job& J, int64_t p0, int6
 // entries gives the rest to the whole warp, so that a long row among short ones
 // does not keep T lanes busy alone.  Bound by the gathers of B's offsets (and, at
 // one warp per row, by the lanes that a short row leaves idle): see
-// launch_rowwork for the choice of T.  The counters are kept per lane and per
+// rowwork_lanes for the choice of T.  The counters are kept per lane and per
 // CTA: a 64-bit atomic in shared memory is a compare-and-swap loop, and four of
 // them per row took as long as the row.
 template <int T>
@@ -556,17 +556,12 @@ int grid_for(int64_t work, int per_block, int cap) {
 void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows, int64_t entries,
                     Stats* d_stats, ErrWord* d_err, cudaStream_t stream) {
     if (total_rows <= 0) return;
-    // Lanes per row.  Measured with 4 / 8 lanes (2 and 32 were slower everywhere;
-    // one warp per row with 64-bit shared atomics before): 65,536 rows of 16
-    // entries 13.3 / 15.8 us (21), power-law rows of 24 on average 244 / 255 us
-    // (323), uneven rows of 34 38 / 35 us (34), R and R*A of the 128^3 Galerkin
-    // chain (8 and 32 entries) 110 / 86 us (143).
     auto run = [&](auto t) {
         constexpr int T = decltype(t)::value;
         rowwork_kernel<T><<<grid_for(total_rows, kRowworkThreads / T, 152 * 8), kRowworkThreads, 0, stream>>>(
             d_jobs, njobs, d_job_row_base, total_rows, d_stats, d_err);
     };
-    if (entries / total_rows <= 24) run(std::integral_constant<int, 4>{});
+    if (rowwork_lanes(entries, total_rows) == 4) run(std::integral_constant<int, 4>{});
     else run(std::integral_constant<int, 8>{});
 }
 

@@ -209,7 +209,7 @@ struct Readback {
 };
 // K1: products per row (ub), bin histogram, product total and input checks.
 // Rows of all jobs are flattened: job j owns rows [row_base_j, row_base_j + A_j.rows).
-// entries: stored entries of all A (sets the lanes per row only).
+// entries: stored entries of A in these rows (sets the lanes per row only).
 void launch_rowwork(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows, int64_t entries,
                     Stats* d_stats, ErrWord* d_err, cudaStream_t stream);
 // K1b: scatter work items into per-bin lists, which follow one another in bin

@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <initializer_list>
+#include <vector>
 
 #include "dispatch.h"
 
@@ -32,5 +33,33 @@ int main() {
     CHECK(map_log2({1 << 30}) == -1);
     CHECK(map_log2({0}) == -1);
     CHECK(map_log2({1 << 21, 5000, 40}) == spg::bitmap_log2(5000));
+
+    // Row blocks cover the rows in order, and each knows its own entries: K1's lanes
+    // follow the mean of the block, not the matrix's entries over the block's rows
+    for (int32_t rows : {2, 33, 262144, 1 << 20})
+        for (int64_t mean : {8, 24, 25, 40, 1 << 22}) {
+            std::vector<int64_t> rp(static_cast<size_t>(rows) + 1, 0);
+            for (int32_t r = 0; r < rows; ++r) rp[r + 1] = rp[r] + mean + (r % 3 - 1) * (r + 1 < rows - rows % 3);
+            const int64_t nnz = rp[rows];
+            for (const int64_t* row_ptr : {static_cast<const int64_t*>(rp.data()), static_cast<const int64_t*>(nullptr)}) {
+                const std::vector<spg::RowBlock> blocks = spg::row_blocks(rows, nnz, row_ptr);
+                CHECK((blocks.size() > 1) == (nnz >= spg::kBlockedEntries));
+                int32_t at = 0;
+                int64_t entries = 0;
+                for (const spg::RowBlock& b : blocks) {
+                    CHECK(b.first == at && b.end > at);
+                    at = b.end;
+                    entries += b.entries;
+                    const int64_t own = rp[b.end] - rp[b.first];
+                    CHECK(b.entries == own || (!row_ptr && b.entries >= own - 2 && b.entries <= own + 2));
+                    if (mean != 24 && mean != 25)
+                        CHECK(spg::rowwork_lanes(b.entries, b.end - b.first) == spg::rowwork_lanes(nnz, rows));
+                }
+                CHECK(at == rows);
+                CHECK(entries <= nnz && entries >= nnz - 10);
+            }
+        }
+    CHECK(spg::row_blocks(0, 0, nullptr).empty());
+    CHECK(spg::rowwork_lanes(24 * 1000 + 999, 1000) == 4 && spg::rowwork_lanes(25 * 1000, 1000) == 8);
     return failures ? 1 : 0;
 }
