@@ -1073,7 +1073,7 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
         }
         const int32_t m = A->rows;
         const std::vector<RowBlock> blocks = row_blocks(m, A->nnz, A->location == SPG_HOST ? A->row_ptr : nullptr);
-        int64_t products = 0;
+        int64_t products = 0, direct_left = kDirectTransient;  // for all blocks, which are held together
         spg_timings sum{};
         int64_t off = 0;
         std::vector<cudaEvent_t> done;
@@ -1105,9 +1105,10 @@ spg_status spg_multiply_to_host(spg_handle* h, const spg_csr_view* A, const spg_
                 blk.row_ptr = dv[0].row_ptr + r0;  // absolute offsets into A's column/value arrays
                 std::vector<JobIn> in{{&blk, &dv[1], CsrView{}, block.entries}};
                 std::vector<DevResult> out;
-                run_products(h, in, out, false, nullptr, {false, kDirectTransient});
+                run_products(h, in, out, false, nullptr, {false, direct_left});
                 DevResult& r = out[0];
                 held.push_back(r);  // freed by release_held, on success or failure
+                if (r.products <= direct_left) direct_left -= r.products;
                 if (off + r.nnz > c_capacity) {
                     *c_nnz = off + r.nnz;  // at least this many entries are needed
                     throw Failure{SPG_BUDGET_EXCEEDED, "nnz(C) exceeds c_capacity"};
