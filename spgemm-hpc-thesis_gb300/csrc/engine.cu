@@ -690,14 +690,23 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
     // Up to kDirectProducts the compaction follows without a wait for the stored
     // count, into arrays of the upper bound's size; it moves nothing if there is
     // nothing to close up.
-    const bool direct = !exact && njobs == 1 && total_rows > 0 && !h->cfg.hbm_budget_bytes &&
-                        products <= use.direct_most;
+    bool direct = !exact && njobs == 1 && total_rows > 0 && !h->cfg.hbm_budget_bytes && products <= use.direct_most;
     int32_t* k5_col = nullptr;
     double* k5_val = nullptr;
     int64_t* h_starts = nullptr;
     if (direct) {
-        k5_col = ar.alloc_result<int32_t>(static_cast<size_t>(products), "C col (compact)");
-        k5_val = ar.alloc_result<double>(static_cast<size_t>(products), "C val (compact)");
+        try {
+            k5_col = ar.alloc_result<int32_t>(static_cast<size_t>(products), "C col (compact)");
+            k5_val = ar.alloc_result<double>(static_cast<size_t>(products), "C val (compact)");
+        } catch (const Failure& f) {  // arrays of C's size may fit
+            if (f.status != SPG_OUT_OF_MEMORY) throw;
+            cudaGetLastError();
+            if (k5_col) ar.free_now(k5_col);
+            k5_col = nullptr;
+            direct = false;
+        }
+    }
+    if (direct) {
         launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
         launch_compact_holes(d_jobs, 1, d_row_base, total_rows, products, items, bin_off, k5_col, k5_val, st,
                              readback_of(d_ctrl, hc, offsetof(Ctrl, cursor)), &d_ctrl->stats, &d_ctrl->err);

@@ -27,6 +27,9 @@ class Shim:
     def start(self, fail_from: int = 0, fail_count: int = 0) -> None:
         self.lib.shim_start(fail_from, fail_count)
 
+    def limit(self, more: int = -1) -> None:
+        self.lib.shim_limit(self._c.c_longlong(more))
+
     def slow(self, from_bytes: int, ms: int) -> None:
         self.lib.shim_slow(self._c.c_longlong(from_bytes), self._c.c_longlong(ms))
 

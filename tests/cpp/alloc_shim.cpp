@@ -16,6 +16,7 @@ namespace {
 std::mutex lock;
 std::unordered_map<void*, size_t> live;
 std::atomic<long long> slow_bytes{-1}, slow_ms{0};  // allocations of at least that many bytes take that long
+long long limit = -1;  // most bytes held at once
 long long calls, bytes, peak, failed, fail_from, fail_count, total;
 
 template <typename F>
@@ -28,7 +29,8 @@ cudaError_t counted(void** p, size_t n, Alloc&& alloc) {
     {
         std::lock_guard<std::mutex> g(lock);
         const long long i = calls++;
-        if (fail_count && i >= fail_from && i - fail_from < fail_count) {
+        if ((fail_count && i >= fail_from && i - fail_from < fail_count) ||
+            (limit >= 0 && bytes + static_cast<long long>(n) > limit)) {
             ++failed;
             return cudaErrorMemoryAllocation;
         }
@@ -89,6 +91,11 @@ void shim_start(long long from, long long count) {
     peak = bytes;
     fail_from = from;
     fail_count = count;
+}
+// A device of that many bytes more than are held now (< 0: without a limit).
+void shim_limit(long long more) {
+    std::lock_guard<std::mutex> g(lock);
+    limit = more < 0 ? -1 : bytes + more;
 }
 void shim_slow(long long from_bytes, long long ms) {
     slow_ms = ms;
