@@ -148,7 +148,11 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
     int64_t* cnt = cv.take<int64_t>(slots);
     int64_t* nz = cv.take<int64_t>(slots);
     int64_t* items = cv.take<int64_t>(static_cast<size_t>(m));
-    int64_t* partials = cv.take<int64_t>(scan_partials_count(static_cast<int64_t>(slots)));
+    // The scans' tile sums need no scratch of their own: those of cnt lie in nz, which
+    // the numeric phase finds cleared again, those of nz in the bin lists, done with.
+    const size_t sums = scan_partials_count(m);
+    int64_t* const cnt_sums = nz;
+    int64_t* const nz_sums = items;
     if (!cv.fits())
         return ret(SPG_BUDGET_EXCEEDED, "A has too many rows for the 32 MiB allocation-free scratch", err, err_len);
 
@@ -188,7 +192,8 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
     for (int b = 1; b < kNumBins; ++b)
         launch_symbolic(b, d_job, items + bin_off[b], bin_count[b], max_ub, B->cols,
                         heavy_map_cols(B->cols), d_slab, slab, &d_ctrl->stats, &d_ctrl->err, st, num_sms);
-    launch_scan(cnt, static_cast<int64_t>(slots) - 1, partials, st);
+    launch_scan(cnt, m, cnt_sums, st);
+    if (scan_launches(m) > 1) cudaMemsetAsync(nz, 0, sizeof(int64_t) * std::min(sums, slots), st);
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "symbolic launch", err, err_len);
     int64_t total = 0;
     if ((ce = cudaMemcpyAsync(&total, cnt + m, sizeof total, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
@@ -214,7 +219,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
     *c_nnz = nnz;
     if (nnz > c_capacity) return ret(SPG_BUDGET_EXCEEDED, "output capacity is smaller than nnz(C) (see c_nnz)", err, err_len);
     // Rows into the caller's arrays: nz scanned gives the final offsets.
-    launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
+    launch_scan(nz, m, nz_sums, st);
     launch_compact(d_job, static_cast<int>(m), c_col, c_val, st);
     if ((ce = cudaMemcpyAsync(c_row_ptr, nz, slots * sizeof(int64_t), cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
         (ce = cudaGetLastError()) != cudaSuccess || (ce = cudaStreamSynchronize(st)) != cudaSuccess)
