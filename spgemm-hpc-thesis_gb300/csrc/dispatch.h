@@ -39,6 +39,24 @@ inline int heavy_map_log2(int64_t map_cols) { return map_cols > 0 ? bitmap_log2(
 // 128^3 Galerkin chain (8 and 32 entries) 110 / 86 us (143).
 inline int rowwork_lanes(int64_t entries, int64_t rows) { return entries / rows <= 24 ? 4 : 8; }
 
+// K4's rows of bins 1 and 2 (<= 32 and <= 64 products) eight and four to a warp, or one:
+// `entries` of A in the `count` rows of the bin.  Several rows to a warp leave fewer
+// warps than the GPU holds below 64 rows per SM (accumulated stages with 4-500 such
+// rows: 9.5 us a launch against 7).  They also walk their entries one row after the
+// other, which entries whose B row is empty make long.  Several / one, in us:
+//   bin 1, rows of 14 products: 10,000 rows of 16 entries 17.8 / 18.3, of 32 21.7 / 19.2,
+//     of 1,024 265 / 134; 20,000 of 32 24 / 27, of 64 35 / 33, of 1,024 306 / 226; 50,000 of
+//     96 77 / 79, of 192 143 / 130; 200,000 of 16 81 / 142, of 512 1,012 / 1,044;
+//   bin 2, rows of 44 products: 20,000 rows of 32 32 / 28, of 128 56 / 46, of 1,024 246 /
+//     185; 200,000 of 32 157 / 151, of 64 202 / 202, of 128 328 / 306, of 512 936 / 817;
+//     rows of 56 products without empty B rows: 50,000 of 8 40 / 48, of 36 54 / 66, of 56
+//     68 / 79, 200,000 of 8 122 / 162, of 28 174 / 184, of 56 226 / 276.
+inline bool several_rows_per_warp(int bin, int64_t count, int64_t entries, int num_sms) {
+    if (count < static_cast<int64_t>(num_sms) * 64) return false;
+    if (bin == 1) return 8 * (entries / count) <= 3 * (count / num_sms);
+    return bin == 2 && entries / count <= 64;
+}
+
 // The row blocks of a product that is copied to the host while it is computed.
 struct RowBlock {
     int32_t first, end;  // rows

@@ -377,7 +377,7 @@ struct ExactSplit {
 // 17-19 are split in one launch (apart for the tuner, which times each bin).
 // Returns the kernels launched.
 int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, const int64_t* bin_count,
-                    const int64_t* bin_off, int64_t max_ub, const SplitTotals& split, void* scratch,
+                    const int64_t* bin_off, const Stats& stats, int64_t max_ub, const SplitTotals& split, void* scratch,
                     const NumericScratch& ns, Ctrl* d_ctrl, bool holes, bool timed, const ExactSplit* exact_split = nullptr) {
     spg_handle* h = bs.h;
     int64_t launches = 0;
@@ -409,7 +409,7 @@ int64_t launch_bins(BinStreams& bs, const Job* d_jobs, const int64_t* items, con
             }
         launch_numeric(b, d_jobs, items + bin_off[first], count, max_ub, split, scratch,
                        static_cast<unsigned char*>(scratch) + ns.slab[b], &d_ctrl->stats, &d_ctrl->err, st, h->num_sms,
-                       holes, h->bin_variant[b]);
+                       holes, bin_entries(stats, b), h->bin_variant[b]);
         launches += split_rows ? 3 : 1;  // planner, pieces, global-slab rows
         if (timed)
             for (int i = first; i <= b; ++i) cudaEventRecord(h->bin_ev[i], st);
@@ -683,7 +683,7 @@ void run_products_once(spg_handle* h, const std::vector<JobIn>& in, std::vector<
             }
         }
     }
-    launches += launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, !exact, true,
+    launches += launch_bins(streams, d_jobs, items, bin_count, bin_off, hc->stats, max_ub, split, scratch, ns, d_ctrl, !exact, true,
                             exact_split.d_jobs ? &exact_split : nullptr);
     check_cuda(cudaGetLastError(), "K4 launch");
     cudaEventRecord(h->ev[4], st);
@@ -1724,7 +1724,7 @@ void plan_build(spg_plan* p, int32_t n, const spg_csr_view* A, const spg_csr_vie
     cudaMemsetAsync(nz, 0, slots * sizeof(int64_t), st);
     cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), st);
     // (the bins' fork and join are part of the graph)
-    launch_bins(streams, d_jobs, items, bin_count, bin_off, max_ub, split, scratch, ns, d_ctrl, true, false);
+    launch_bins(streams, d_jobs, items, bin_count, bin_off, p->hc->stats, max_ub, split, scratch, ns, d_ctrl, true, false);
     launch_scan(nz, static_cast<int64_t>(slots) - 1, partials, st);
     launch_compact_holes(d_jobs, n, d_row_base, total_rows, products, items, bin_off, p->col, p->val, st,
                          readback_of(d_ctrl, p->hc, offsetof(Ctrl, cursor)));

@@ -626,11 +626,11 @@ void launch_split_exact(const Job* d_jobs, const Job* d_split_jobs, const int64_
 
 void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
                     const SplitTotals& split, void* d_scratch, void* d_slab, Stats* d_stats, ErrWord* d_err,
-                    cudaStream_t st, int num_sms, bool holes, int variant) {
+                    cudaStream_t st, int num_sms, bool holes, int64_t entries, int variant) {
     if (count <= 0) return;
     if (variant == 1 && launch_numeric_alt(bin, d_jobs, d_items, count, d_stats, d_err, st, num_sms)) return;
     if (bin <= kLastWarpBin) {
-        launch_numeric_warp(bin, d_jobs, d_items, count, d_stats, d_err, st, num_sms);
+        launch_numeric_warp(bin, d_jobs, d_items, count, entries, d_stats, d_err, st, num_sms);
         return;
     }
     // Rows above 8,192 products are split into column-range pieces in the

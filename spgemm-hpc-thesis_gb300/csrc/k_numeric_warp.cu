@@ -383,24 +383,21 @@ void run_rows(const Job* jobs, const int64_t* items, int64_t count, Stats* stats
 
 }  // namespace
 
-void launch_numeric_warp(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, Stats* d_stats,
-                         ErrWord* d_err, cudaStream_t st, int num_sms) {
+void launch_numeric_warp(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t entries,
+                         Stats* d_stats, ErrWord* d_err, cudaStream_t st, int num_sms) {
     // Several short rows per warp: 0.160 -> 0.072 ms for 262,144 rows of 56 products
     // in 8 segments, 0.28 -> 0.21 ms for 262,144 rows of 32 products in 32
     // segments (bound there by the L1 lines that its gathers touch), against one
-    // row per warp.  Only where that still leaves every resident warp
-    // (32 per SM) a row or two; below, one row per warp ends sooner (accumulated
-    // stages with 4-500 such rows: 7 us a launch against 9.5).  Rows of 65-128
-    // products measure the same either way (two to a warp: 0.110 and 0.113 ms on
-    // the power-law product, one: 0.102 and 0.094).
-    const bool full = count >= static_cast<int64_t>(num_sms) * 64;
+    // row per warp.  Rows of 65-128 products measure the same either way (two to a
+    // warp: 0.110 and 0.113 ms on the power-law product, one: 0.102 and 0.094).
+    const bool several = several_rows_per_warp(bin, count, entries, num_sms);
     switch (bin) {
         case 1:
-            if (full) run_rows<1, 8>(d_jobs, d_items, count, d_stats, d_err, st, num_sms);
+            if (several) run_rows<1, 8>(d_jobs, d_items, count, d_stats, d_err, st, num_sms);
             else run_warp<1>(d_jobs, d_items, count, d_stats, d_err, st, num_sms);
             break;
         case 2:
-            if (full) run_rows<2, 4>(d_jobs, d_items, count, d_stats, d_err, st, num_sms);
+            if (several) run_rows<2, 4>(d_jobs, d_items, count, d_stats, d_err, st, num_sms);
             else run_warp<2>(d_jobs, d_items, count, d_stats, d_err, st, num_sms);
             break;
         case 3: run_warp<3>(d_jobs, d_items, count, d_stats, d_err, st, num_sms); break;

@@ -69,17 +69,18 @@ rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restric
                int64_t total_rows, Stats* __restrict__ stats, ErrWord* __restrict__ err) {
     constexpr int U = 4, kRows = 32 / T;
     __shared__ unsigned int s_bins[kNumBins];
-    __shared__ unsigned long long s_products, s_max, s_split;
+    __shared__ unsigned long long s_products, s_max, s_split, s_short[2];
     const int lane = threadIdx.x & 31, tl = lane % T;
     if (threadIdx.x < kNumBins) s_bins[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         s_products = 0;
         s_max = 0;
         s_split = 0;
+        s_short[0] = s_short[1] = 0;
     }
     __syncthreads();
 
-    int64_t products = 0, most = 0, split = 0;
+    int64_t products = 0, most = 0, split = 0, short1 = 0, short2 = 0;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * (kRowworkThreads / 32) * kRows;
     for (int64_t g0 = (static_cast<int64_t>(blockIdx.x) * (kRowworkThreads / 32) + (threadIdx.x >> 5)) * kRows;
          g0 < total_rows; g0 += stride) {
@@ -125,12 +126,18 @@ rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restric
             products += len;
             most = len > most ? len : most;
             if (len > kSplitThreshold) split += len;
+            if (len > 0 && len <= bin_capacity(1)) short1 += a1 - a0;
+            else if (len > 0 && len <= bin_capacity(2)) short2 += a1 - a0;
         }
     }
     products = warp_sum(products);
     most = warp_max(most);
     split = warp_sum(split);
+    short1 = warp_sum(short1);
+    short2 = warp_sum(short2);
     if (lane == 0 && products) {
+        if (short1) atomicAdd(&s_short[0], static_cast<unsigned long long>(short1));
+        if (short2) atomicAdd(&s_short[1], static_cast<unsigned long long>(short2));
         atomicAdd(&s_products, static_cast<unsigned long long>(products));
         atomicMax(&s_max, static_cast<unsigned long long>(most));
         if (split) atomicAdd(&s_split, static_cast<unsigned long long>(split));
@@ -142,6 +149,8 @@ rowwork_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restric
         atomicAdd(&stats->products, s_products);
         atomicMax(&stats->max_ub, s_max);
         if (s_split) atomicAdd(&stats->split_products, s_split);
+        if (s_short[0]) atomicAdd(&stats->short_entries[0], s_short[0]);
+        if (s_short[1]) atomicAdd(&stats->short_entries[1], s_short[1]);
     }
 }
 

@@ -183,6 +183,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         return ret(SPG_OVERFLOW, "an output row has more than 2^30 scalar products", err, err_len);
     int64_t bin_count[kNumBins], bin_off[kNumBins + 1];
     bin_lists(hc.stats, bin_count, bin_off);
+    const Stats row_stats = hc.stats;
     const NumericScratch ns = numeric_scratch(bin_count, max_ub, SplitTotals{}, num_sms, false, BinOrder::kSerial);
     const size_t slab = std::max(symbolic_scratch_bytes(bin_count, max_ub, num_sms), ns.bytes);
     unsigned char* d_slab = slab ? cv.take<unsigned char>(slab) : nullptr;
@@ -209,7 +210,7 @@ extern "C" spg_status spg_multiply_noalloc(const spg_csr_view* A, const spg_csr_
         return from_cuda(ce, "job update", err, err_len);
     for (int b = 1; b < kNumBins; ++b)
         launch_numeric(b, d_job, items + bin_off[b], bin_count[b], max_ub, SplitTotals{}, d_slab,
-                       d_slab + ns.slab[b], &d_ctrl->stats, &d_ctrl->err, st, num_sms, false);
+                       d_slab + ns.slab[b], &d_ctrl->stats, &d_ctrl->err, st, num_sms, false, bin_entries(row_stats, b));
     if ((ce = cudaGetLastError()) != cudaSuccess) return from_cuda(ce, "numeric launch", err, err_len);
     if ((ce = cudaMemcpyAsync(&hc, d_ctrl, sizeof hc, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (ce = cudaStreamSynchronize(st)) != cudaSuccess)

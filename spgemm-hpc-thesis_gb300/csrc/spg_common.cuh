@@ -115,6 +115,7 @@ struct Stats {
     unsigned long long sym_total;     // sum of cnt
     unsigned long long nz_total;      // sum of nz
     unsigned long long split_products;  // sum of ub over rows of more than kSplitThreshold products
+    unsigned long long short_entries[2];  // entries of A in the rows of bins 1 and 2
     // the row queue of each bin's numeric launch: rows (or, for the split rows
     // of bins 17-19, pieces) handed out past the launch's first wave
     unsigned long long ticket[kNumBins];
@@ -246,10 +247,14 @@ int scan_launches(int64_t n);  // kernels of launch_scan
 // (they size the staging of split rows; one launch may take the rows of all of
 // bins 17-19).  d_scratch and d_slab: the call's numeric scratch and the bin's
 // slab in it (numeric_scratch).  variant: 0 the default team shape of the bin,
-// 1 its alternative (where the bin has one; see launch_numeric_alt).
+// 1 its alternative (where the bin has one; see launch_numeric_alt).  entries: of A in
+// the rows of bin 1 or 2 (bin_entries).
 void launch_numeric(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
                     const SplitTotals& split, void* d_scratch, void* d_slab, Stats* d_stats, ErrWord* d_err,
-                    cudaStream_t stream, int num_sms, bool holes, int variant = 0);
+                    cudaStream_t stream, int num_sms, bool holes, int64_t entries, int variant = 0);
+inline int64_t bin_entries(const Stats& stats, int bin) {
+    return bin == 1 || bin == 2 ? static_cast<int64_t>(stats.short_entries[bin - 1]) : 0;
+}
 // The rows of bins 17-19 in the exact layout by way of the split: d_split_jobs
 // are the jobs with holes set, C_tmp arrays of split.products slots and cnt
 // arrays of their own; the kept entries then move to d_jobs' places.  Scratch:
@@ -264,8 +269,8 @@ bool launch_numeric_alt(int bin, const Job* d_jobs, const int64_t* d_items, int6
                         ErrWord* d_err, cudaStream_t stream, int num_sms);
 constexpr int kNumVariants = 2;
 // K4 for the warp-per-row bins (1..kLastWarpBin), compiled separately.
-void launch_numeric_warp(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, Stats* d_stats,
-                         ErrWord* d_err, cudaStream_t stream, int num_sms);
+void launch_numeric_warp(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t entries,
+                         Stats* d_stats, ErrWord* d_err, cudaStream_t stream, int num_sms);
 // How the bins of one call run beside one another, which is what their scratch
 // may share: one after the other; the bins above 8192 products beside the
 // others; every bin beside every other (bins 17-19 excepted).

@@ -60,6 +60,18 @@ int main() {
             }
         }
     CHECK(spg::row_blocks(0, 0, nullptr).empty());
+
+    // Short rows several to a warp: many rows of few entries, not rows whose entries
+    // mostly meet empty rows of B (measured on both sides, see the rule)
+    constexpr int kSms = 152;
+    auto several = [](int bin, int64_t rows, int64_t each) {
+        return spg::several_rows_per_warp(bin, rows, rows * each, kSms);
+    };
+    CHECK(several(1, 10000, 16) && several(1, 20000, 32) && several(1, 50000, 96) && several(1, 262144, 32));
+    CHECK(!several(1, 10000, 64) && !several(1, 20000, 128) && !several(1, 50000, 192) && !several(1, 20000, 2000));
+    CHECK(several(2, 262144, 8) && several(2, 50000, 56) && !several(2, 20000, 128) && !several(2, 200000, 512));
+    for (int bin : {1, 2}) CHECK(!several(bin, 64 * kSms - 1, 2) && several(bin, 64 * kSms, 2));
+    CHECK(!several(3, 262144, 8));
     CHECK(spg::rowwork_lanes(24 * 1000 + 999, 1000) == 4 && spg::rowwork_lanes(25 * 1000, 1000) == 8);
     return failures ? 1 : 0;
 }
