@@ -685,6 +685,24 @@ __device__ __noinline__ int32_t write_share(const uint32_t* keys, const double* 
     return all;
 }
 
+// The sum of the products at positions [q, hi) of column c, after acc, in order, for
+// rows that keep columns and sequence numbers apart; the columns ascend.  A run's adds
+// follow one another, its loads need not: four at a time, rows of 2,500 products in
+// one column take 2.70 -> TODO ms (5,000 rows), of 10,000 in three columns 14.4 -> TODO.
+__device__ __forceinline__ double sum_run(const uint32_t* keys, const uint16_t* seqs, const double* vals, int q, int hi,
+                                          uint32_t c, double acc) {
+    constexpr int U = 4;
+    for (; q + U <= hi && keys[q + U - 1] == c; q += U) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = vals[seqs[q + u]];
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc = __dadd_rn(acc, v[u]);
+    }
+    for (; q < hi && keys[q] == c; ++q) acc = __dadd_rn(acc, vals[seqs[q]]);
+    return acc;
+}
+
 // write_slots for the rows that keep columns and sequence numbers apart: slots
 // [x0, x1) of a row whose runs may start or end anywhere in [lo, hi).  Returns
 // the warp's kept sums.
@@ -695,8 +713,7 @@ __device__ __noinline__ uint32_t write_slots_plain(const uint32_t* keys, const u
         const uint32_t c = keys[p];
         double acc = 0.0;
         if (p == lo || keys[p - 1] != c) {
-            acc = vals[seqs[p]];
-            for (int q = p + 1; q < hi && keys[q] == c; ++q) acc = __dadd_rn(acc, vals[seqs[q]]);
+            acc = sum_run(keys, seqs, vals, p + 1, hi, c, vals[seqs[p]]);
         }
         const bool keep = nonzero(acc);
         oc[p] = keep ? static_cast<int32_t>(c) : -1;
@@ -722,8 +739,7 @@ __device__ __forceinline__ uint32_t write_kept_plain(RowSmem<W, ITEMS, SV>& sm, 
             const uint32_t c = sm.keys[pos];
             if (pos == 0 || sm.keys[pos - 1] != c) {
                 const uint32_t s0 = sm.seqs[pos];
-                double acc = vals[s0];
-                for (int q = pos + 1; q < P && sm.keys[q] == c; ++q) acc = __dadd_rn(acc, vals[sm.seqs[q]]);
+                const double acc = sum_run(sm.keys, sm.seqs, vals, pos + 1, P, c, vals[s0]);
                 vals[s0] = acc;
                 keep = nonzero(acc);
             }
