@@ -688,7 +688,8 @@ __device__ __noinline__ int32_t write_share(const uint32_t* keys, const double* 
 // The sum of the products at positions [q, hi) of column c, after acc, in order, for
 // rows that keep columns and sequence numbers apart; the columns ascend.  A run's adds
 // follow one another, its loads need not: four at a time, rows of 2,500 products in
-// one column take 2.70 -> TODO ms (5,000 rows), of 10,000 in three columns 14.4 -> TODO.
+// one column take 1.42 ms (5,000 rows), of 10,000 in three columns 8.0; one at a time
+// 2.70 and 14.4 (with the loop inlined in the row's code 2.50 and 13.2).
 __device__ __forceinline__ double sum_run(const uint32_t* keys, const uint16_t* seqs, const double* vals, int q, int hi,
                                           uint32_t c, double acc) {
     constexpr int U = 4;
