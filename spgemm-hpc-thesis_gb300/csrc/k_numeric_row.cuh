@@ -80,15 +80,8 @@ constexpr int kBucketWords = W == 1 ? 4 : 2 * kCoarse<W> + W * 32 * ITEMS + 4;
 template <int ITEMS>
 constexpr int kShareItems = ITEMS + 2;
 constexpr uint32_t kMaxFine = 32;
-// Which rows take the bucket sort: CTA rows.  A warp row sorts its packed keys
-// in registers (spg_warp_sort.cuh).  Against the radix sort of rows of <= 192
-// products and the bucket sort of 193-512 (power-law product, one bin at a
-// time): <= 512 products 0.95 -> 0.49 ms, <= 384 0.79 -> 0.50, <= 256 0.35 ->
-// 0.23, <= 192 0.37 -> 0.25, <= 128 0.145 -> 0.094; 65,536 rows of 256: 0.190 ->
-// 0.147 ms.  Issue slots bound these kernels, and the network takes about half
-// the instructions of either sort (about 90 a key), none of them waiting on
-// shared memory.
-// SV: product values in shared memory (else in a per-CTA global slab).
+
+// A team's shared memory.  SV: product values in shared memory (else in a per-CTA global slab).
 template <int W, int ITEMS, bool SV = true>
 struct RowSmem {
     static constexpr int kCap = W * 32 * ITEMS;
@@ -217,7 +210,6 @@ struct RowOut {
     int64_t out0;       // first slot of the row in C_tmp
     int64_t* nz;        // the row's stored-entry count
     int32_t holes;      // upper-bound mode: slot-per-position output with holes
-    int32_t nz_add;     // a piece of a split row: add to *nz instead of storing it
 };
 
 // The sum of `all` over the warps before this one, and the team-wide maximum of m
@@ -777,8 +769,11 @@ __device__ __forceinline__ uint32_t write_kept_plain(RowSmem<W, ITEMS, SV>& sm, 
 }
 
 // The radix sort of the CTA rows with a large bucket (a column repeated more
-// than kMaxFine times): out of line, so that it takes no registers from the
-// rows that do not need it.
+// than kMaxFine times).  Out of line: inlined, the kernels of 64 registers spill more
+// (4x12 378 / 286 bytes of stores / loads against 192 / 180, 8x12 338 / 266 against
+// 192 / 180).  They still spill: what the row keeps across the calls of paths that it
+// seldom takes lies in local memory (1.8 M loads and 2.3 M stores in 183 M warp
+// instructions of the 4x12 kernel; 0.36 and 0.43 M in the kernel before it).
 template <int W, int ITEMS, bool SV>
 __device__ __noinline__ void radix_sort_cta(RowSmem<W, ITEMS, SV>& sm, int P, uint32_t cmin, int nbits, int lane, int warp,
                                             int tid) {
@@ -801,7 +796,13 @@ __device__ __forceinline__ uint32_t finish_row(const RowOut& out, RowSmem<W, ITE
     // 2. sort by column: warp rows in registers (the padding words above P sort
     //    last: a real word is all ones only when P is the row's capacity), CTA
     //    rows by bucket and then, inside the buckets, in registers, and by the
-    //    radix sort where a bucket is large
+    //    radix sort where a bucket is large.  Warp rows, against the radix sort of
+    //    rows of <= 192 products and the bucket sort of 193-512 (power-law product,
+    //    one bin at a time): <= 512 products 0.95 -> 0.49 ms, <= 384 0.79 -> 0.50,
+    //    <= 256 0.35 -> 0.23, <= 192 0.37 -> 0.25, <= 128 0.145 -> 0.094; 65,536 rows
+    //    of 256: 0.190 -> 0.147 ms.  Issue slots bound these kernels, and the network
+    //    takes about half the instructions of either sort (about 90 a key), none of
+    //    them waiting on shared memory.
     uint32_t kept = 0;
     if constexpr (W == 1 && PACKED) {
         uint32_t k[ITEMS];
@@ -951,7 +952,7 @@ __device__ uint32_t numeric_row(const Job& J, int row, RowSmem<W, ITEMS, SV>& sm
     const int P = static_cast<int>(PIECE ? pc->count : J.ub[row]);
     if constexpr (W > 1) {
         // an upper-bound row's warps add their kept counts to its count after the
-        // barriers below (a piece's row count was zeroed by the planner)
+        // barriers below (a piece's row count was zeroed by the row work, or in a plan's replay)
         if (!PIECE && J.holes && tid == 0) J.nz[row] = 0;
     }
 
@@ -1003,7 +1004,7 @@ __device__ uint32_t numeric_row(const Job& J, int row, RowSmem<W, ITEMS, SV>& sm
     const uint32_t cmin = static_cast<uint32_t>(lo);
     const uint32_t range = P ? static_cast<uint32_t>(hi - lo) : 0u;
     const int nbits = range ? 32 - __clz(range) : 0;
-    const RowOut out{J.c_col, J.c_val, J.cnt[row] + (PIECE ? pc->slot_off : 0), J.nz + row, J.holes, PIECE ? 1 : 0};
+    const RowOut out{J.c_col, J.c_val, J.cnt[row] + (PIECE ? pc->slot_off : 0), J.nz + row, J.holes};
     if constexpr (W == 1)
         if (range < (0xffffffffu >> kSeqBits)) return finish_row<W, ITEMS, SV, true>(out, sm, vals, P, cmin, range, nbits, lane, warp, tid);
     return finish_row<W, ITEMS, SV, false>(out, sm, vals, P, cmin, range, nbits, lane, warp, tid);

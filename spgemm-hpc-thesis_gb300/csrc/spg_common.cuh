@@ -233,7 +233,7 @@ inline void bin_lists(const Stats& stats, int64_t* count, int64_t* off) {
 void launch_symbolic(int bin, const Job* d_jobs, const int64_t* d_items, int64_t count, int64_t max_ub,
                      int64_t max_cols, int64_t map_cols, void* d_scratch, size_t scratch_bytes, Stats* d_stats,
                      ErrWord* d_err, cudaStream_t stream, int num_sms);
-// Global scratch of the symbolic phase (hash slabs of rows above 8192 products).
+// Global scratch of the symbolic phase (hash slabs of rows above 16384 products).
 size_t symbolic_scratch_bytes(const int64_t* bin_count, int64_t max_ub, int num_sms);
 // K3: exclusive scan of n+1 int64 counts (16-byte aligned) in place (last entry
 // becomes the total).
