@@ -417,7 +417,7 @@ __device__ void compact_long_rows(const Job* __restrict__ jobs, const int64_t* _
 // A step of a warp waits about 1 us for memory, so one row of 100,000 slots alone
 // took a warp as long as the GPU needs for 100 M slots: rows of kLongBin and above
 // are left to the first `long_ctas` CTAs.  Power-law squares of 65,539, 100,003 and
-// 1 M rows (36, 56 and 595 M slots): 165, 244 and 2,205 us (339, 422 and 2,360
+// 1 M rows (36, 56 and 595 M slots): 165, 244 and 2,204 us (339, 422 and 2,360
 // before); the last is 6.3 TB/s, 94% of the measured copy bandwidth.
 __global__ void __launch_bounds__(256)
 compact_holes_kernel(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ job_row_base,

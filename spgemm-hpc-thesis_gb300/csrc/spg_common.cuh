@@ -298,9 +298,10 @@ void launch_compact(const Job* d_job, int rows, int32_t* out_col, double* out_va
 // kernel moves nothing after an error or if every slot holds an entry
 // (full->nz_total == slots), for a caller that does not know yet.
 // Rows of kLongBin and above (more than kLongSlots slots) take a CTA each, the
-// others a warp: at 100,003 and 1 M power-law rows 236 and 2,261 us, against 255 and
-// 2,302 with the line at 8192 slots and 234 and 2,265 at 2048, where sixteen products
-// of 20,000 rows lose (323 -> 339 us: a CTA takes one row at a time).
+// others a warp: 244 and 2,204 us at 100,003 and 1 M power-law rows.  In the run that
+// set the line 236 and 2,261, against 255 and 2,302 with it at 8192 slots and 234 and
+// 2,265 at 2048, where sixteen products of 20,000 rows lose (323 -> 339 us: a CTA takes
+// one row at a time).
 constexpr int kLongBin = 15;
 constexpr int64_t kLongSlots = 4096;
 void launch_compact_holes(const Job* d_jobs, int njobs, const int64_t* d_job_row_base, int64_t total_rows,
